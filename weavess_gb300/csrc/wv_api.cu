@@ -52,6 +52,14 @@ __global__ void k_row_norms(const float *x, uint32_t n, uint32_t d, float *out) 
   }
 }
 
+// integer rows as bytes, four values per thread
+__global__ void k_pack8(const float4 *x, size_t count4, uint32_t *out) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count4; i += (size_t)gridDim.x * blockDim.x) {
+    const float4 v = x[i];
+    out[i] = (uint32_t)v.x | (uint32_t)v.y << 8 | (uint32_t)v.z << 16 | (uint32_t)v.w << 24;
+  }
+}
+
 int ensure_search_scratch(wv_ctx *c, uint32_t Lmax, SearchShape sh, int *out_blocks) {
   int blocks = route_grid(c, Lmax, sh);
   WV_CHECK(c, blocks > 0, WV_ERR_LIMIT, "search kernel cannot run with d=%u L=%u width=%u (shared memory)", c->d,
@@ -234,7 +242,7 @@ int wv_ctx_destroy(wv_ctx *c) {
   cudaStreamSynchronize(c->stream);
   for (DevBuf *b : {&c->base, &c->gids, &c->gdeg, &c->visited, &c->touched, &c->misc, &c->q_buf, &c->seed_buf,
                     &c->out_ids_buf, &c->out_dist_buf, &c->lq_buf, &c->kq_buf, &c->fg_ids, &c->fg_dist,
-                    &c->fg_deg, &c->qbase, &c->qscale})
+                    &c->fg_deg, &c->qbase, &c->qscale, &c->qnorm, &c->xnorm, &c->base8})
     b->release();
   c->release_work();
   learn_free(c);
@@ -301,8 +309,14 @@ int wv_upload_base(wv_ctx *c, const float *base, uint32_t n, uint32_t d) {
     WV_CUDA(c, c->xnorm.ensure((size_t)n * 4));
     k_row_norms<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float>(), n, d, c->xnorm.as<float>());
     WV_CUDA(c, cudaGetLastError());
+    if (d % 16 == 0 && d <= 256) {
+      WV_CUDA(c, c->base8.ensure((size_t)n * d));
+      k_pack8<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float4>(), (size_t)n * d / 4, c->base8.as<uint32_t>());
+      WV_CUDA(c, cudaGetLastError());
+    }
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
   }
+  if (!(c->base_int && d % 16 == 0 && d <= 256)) c->base8.release();
   return WV_OK;
 }
 

@@ -11,15 +11,17 @@
 //   nnew   n x (S+R), nold n x min(L+R, 2R)  join lists, lnew/lold lengths
 //
 // The plain form reproduces the single-threaded reference bit for bit:
-//  * join: every local-join pair is evaluated once (exact-order FP32) and its
-//    two offers ("insert j into i", "insert i into j") are keyed by the
-//    reference's sequential position (node n, pair position in
-//    nhood::join's loops, side).  Offers that cannot pass nhood::insert's
-//    first test (dist > pool max at that time; the max only falls during a
-//    join) are dropped at the source.  The rest are grouped per target, sorted
-//    by key, and applied by one warp per target with libstdc++'s
-//    push_heap/pop_heap, so ties resolve exactly as they do sequentially.
-//    Nodes are processed in chunks in node order, so a later chunk sees the
+//  * join: every local-join pair is evaluated (exact-order FP32, or exact
+//    integers) and offered both ways ("insert j into i", "insert i into j").
+//    Offers that cannot pass nhood::insert's first test (dist > pool max at
+//    that time; the max only falls during a join) are dropped at the source;
+//    the rest are written grouped by target.  A target's pool after the join
+//    is the L least of pool and offers in whatever order they come, except
+//    where distances tie: those targets are replayed in the reference's
+//    sequential order (keys: node n, pair position in nhood::join, side) by
+//    libstdc++'s push_heap/pop_heap, so ties resolve exactly as they do
+//    sequentially.  A join whose offers do not fit the device runs in chunks
+//    of nodes in node order, all targets replayed, a later chunk seeing the
 //    pools the earlier chunks left.
 //  * update: per node std::sort (stl_order.cuh), the sampled prefix M, the
 //    new/old split and make_heap run as in the reference.  The reverse
@@ -31,8 +33,6 @@
 //    context's stream.
 //  * the first join is skipped: nhood(L, S) leaves nn_new as 2S zeros
 //    (index.h:98-103), which join pairs with nothing.
-#include <cuda_bf16.h>
-
 #include <algorithm>
 #include <cstdlib>
 #include <string>
@@ -42,7 +42,6 @@
 #include "wv_mt.cuh"
 #include "wv_nnd.h"
 #include "wv_scan.h"
-#include "wv_umma.cuh"
 
 namespace wv {
 namespace {
@@ -233,11 +232,12 @@ __global__ void __launch_bounds__(IR_WARPS * 32)
 struct Nnd {
   uint32_t n, d, S, K, L, R, capn, capo;
   const float *base;
-  const float *xnorm;  // squared row norms (integer data; the tensor-core join)
+  const float *xnorm;    // squared row norms (integer data)
+  const uint8_t *base8;  // the rows as bytes (integer data, d a multiple of 16 up to 256), or null
   Ent *pool;
   uint32_t *psz, *M;
   uint32_t *nnew, *nold, *lnew, *lold, *pnew, *pold;
-  Ent *pre;  // sorted sampled prefix of the last update (n x L)
+  Ent *pre;  // the pools sorted by the last update, flags not yet cleared (n x L; the sampled prefix is M long)
   float *maxd, *hback;
 };
 
@@ -263,6 +263,7 @@ __global__ void k_nnd_init(Nnd s, const uint32_t *ids, const float *dist, const 
       if (!skip) P[k++] = P[t];
     }
     sz = k;
+    for (uint32_t j = 0; j < sz; j++) s.pre[(size_t)i * s.L + j] = P[j];  // (the first join's sorted pools)
   }
   stl::make_heap(P, (int)sz, EntLess());
   for (uint32_t j = 0; j < sz; j++) s.pool[(size_t)i * s.L + j] = P[j];
@@ -301,7 +302,10 @@ __global__ void k_upd_sort(Nnd s) {
   if (i >= s.n) return;
   const uint32_t sz = s.psz[i];
   for (uint32_t j = 0; j < sz; j++) P[j] = s.pool[(size_t)i * s.L + j];
-  stl::sort(P, (int)sz, EntLess());
+  // a pool the last join left in ascending order (k_apply_fast) is sorted
+  bool asc = true;
+  for (uint32_t j = 1; j < sz; j++) asc &= P[j - 1].d < P[j].d;
+  if (!asc) stl::sort(P, (int)sz, EntLess());
   const uint32_t maxl = min(s.M[i] + s.S, sz);
   uint32_t c = 0, l = 0;
   while (l < maxl && c < s.S) {
@@ -310,8 +314,8 @@ __global__ void k_upd_sort(Nnd s) {
   }
   s.M[i] = l;
   uint32_t pn = 0, po = 0;
+  for (uint32_t j = 0; j < sz; j++) s.pre[(size_t)i * s.L + j] = P[j];
   for (uint32_t j = 0; j < l; j++) {
-    s.pre[(size_t)i * s.L + j] = P[j];
     uint32_t id = P[j].idf & ID_MASK;
     if (P[j].idf & FLAG) {
       s.nnew[(size_t)i * s.capn + pn++] = id;
@@ -477,296 +481,534 @@ __global__ void k_bucket_apply(Nnd s, const uint32_t *boff, const uint32_t *bcnt
 }
 
 // ---------------------------------------------------------------- join
-struct Offers {
-  uint32_t *tgt;
-  unsigned long long *key;
-  uint32_t *cand;
-  float *dist;
-  uint32_t *cursor;
-  uint32_t cap;
-  uint32_t *tcnt;
+// The local join in two launches.  k_join computes a node's pair distances
+// into a dense tile G (rows: new ++ old, columns: new), keeps the offers that
+// pass nhood::insert's first test, and writes them grouped by target: the
+// entries {distance, candidate} of target p of node n contiguous, one
+// descriptor {offset, count, n, p} in the target's own descriptor list.  The
+// space of a node's entries is taken with one atomic per node and a
+// descriptor's slot with one per (node, target); one atomic per 32 offers on
+// a single cursor and one per offer to group them had bound the join.  What
+// bounds it now: latency between a node's short phases (lists, rows, tile,
+// counts, entries) at 16 warps per SM.  Integer rows come from the byte copy
+// (128 bytes a row at d = 128): seven joins of 100k x 128 (S 10, L 40, R 100)
+// take 12.2 ms, with the FP32 rows, the tcgen05 Gram tile and the two atomics
+// 28.6 ms; six of 60k x 96 real-valued (FP32) 14.3 ms against 18.6 ms.
+struct JoinOut {
+  uint2 *ent;                  // {distance bits, candidate id}
+  uint16_t *eq;                // the candidate's position in the node's list (new ++ old): the replay's key
+  unsigned long long *cursor;  // entries asked for (past `cap`: none written, the host retries with room)
+  unsigned long long cap;
+  uint4 *desc;                 // {offset, count, n, p}, target t's from toff[t]
+  const uint32_t *toff;        // prefix sums of the targets' occurrences in the lists
+  uint32_t *tcur;              // descriptors written per target
+  const float *mx;             // pool maxima (-inf: empty pool)
+};
+struct JoinCfg {
+  uint32_t tj;     // rows per j tile
+  uint32_t gcap;   // floats of G in shared memory; larger tiles take the block's slab of gscr
+  float *gscr;
+  size_t gslab;
+  uint32_t *lscr;  // the node's lists (4 (capn + capo) words per block) when they do not fit shared memory
 };
 
 constexpr int J_THREADS = 256;
-constexpr int J_TI = 16;  // new rows per i tile
-constexpr int J_TJ = 64;  // rows per j tile (new ++ old); fewer for long rows (the tile must fit shared memory)
+constexpr int J_TI = 16;  // FP32: new rows per i tile
+constexpr int J_TJ = 64;  // FP32: rows per j tile (new ++ old); fewer for long rows (the tile must fit shared memory)
+constexpr int JI_THREADS = 128;       // integer rows
+constexpr uint32_t JI_ROWS = 128;     // integer rows staged at once (all of a node's rows, or a 64 x 64 tile)
+constexpr uint32_t J_GCAP = 4096;     // floats of G in shared memory
 
-__device__ __forceinline__ void emit(const Offers &o, bool ok, uint32_t t, unsigned long long key, uint32_t c,
-                                     float d, int lane, int *status) {
-  unsigned m = __ballot_sync(FULL, ok);
-  if (!m) return;
-  uint32_t base = 0;
-  int leader = __ffs(m) - 1;
-  if (lane == leader) base = atomicAdd(o.cursor, (uint32_t)__popc(m));
-  base = __shfl_sync(FULL, base, leader);
-  if (ok) {
-    uint32_t pos = base + __popc(m & ((1u << lane) - 1));
-    if (pos < o.cap) {
-      o.tgt[pos] = t;
-      o.key[pos] = key;
-      o.cand[pos] = c;
-      o.dist[pos] = d;
-      atomicAdd(&o.tcnt[t], 1u);
-    } else {
-      set_err(status, DEV_OVERFLOW);
-    }
+// occurrences of every id in the lists of nodes [n0, n1), a warp per node,
+// and the largest tile a node needs
+__global__ void k_occ_count(Nnd s, uint32_t n0, uint32_t n1, uint32_t *occ, unsigned long long *gmax) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t n = n0 + w; n < n1; n += nw) {
+    const uint32_t a = s.lnew[n], b = s.lold[n];
+    if (a == 0) continue;
+    const unsigned long long g = (unsigned long long)(a + b) * (a | 1u);
+    if (lane == 0 && g > J_GCAP) atomicMax(gmax, g);
+    for (uint32_t t = lane; t < a + b; t += 32)
+      atomicAdd(&occ[t < a ? s.nnew[(size_t)n * s.capn + t] : s.nold[(size_t)n * s.capo + (t - a)]], 1u);
   }
 }
 
-// local join of nodes [n0, n1): one block per node
-__global__ void __launch_bounds__(J_THREADS) k_join(Nnd s, uint32_t n0, Offers of, unsigned long long *pairs,
-                                                     int *status, uint32_t tjc) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  const uint32_t n = n0 + blockIdx.x;
-  const uint32_t a = s.lnew[n], b = s.lold[n];
-  if (a == 0) return;
-  const uint32_t tot = a + b;
-  const uint32_t stride = ((s.d + 3) & ~3u) + 4;
-  float *ri = (float *)smem;                     // J_TI rows
-  float *rj = ri + (size_t)J_TI * stride;        // J_TJ rows
-  uint32_t *ids = (uint32_t *)(rj + (size_t)tjc * stride);  // tot ids: new ++ old
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (uint32_t t = threadIdx.x; t < tot; t += J_THREADS)
-    ids[t] = t < a ? s.nnew[(size_t)n * s.capn + t] : s.nold[(size_t)n * s.capo + (t - a)];
-  __syncthreads();
-  const uint32_t d4 = s.d >> 2;
-  unsigned long long npairs = 0;
-  for (uint32_t i0 = 0; i0 < a; i0 += J_TI) {
-    const uint32_t ti = min((uint32_t)J_TI, a - i0);
-    for (uint32_t j0 = 0; j0 < tot; j0 += tjc) {
-      const uint32_t tj = min(tjc, tot - j0);
-      __syncthreads();
-      // stage rows (coalesced 16-byte copies, one row per warp step)
-      for (uint32_t r = warp; r < ti + tj; r += J_THREADS / 32) {
-        const uint32_t id = r < ti ? ids[i0 + r] : ids[j0 + (r - ti)];
-        float *dst = r < ti ? ri + (size_t)r * stride : rj + (size_t)(r - ti) * stride;
-        const float *src = s.base + (size_t)id * s.d;
-        for (uint32_t k = lane; k < d4; k += 32) cp_async16(dst + 4 * k, src + 4 * k);
-      }
-      cp_async_wait_all();
-      __syncthreads();
-      // warps take i rows, lanes take j rows
-      for (uint32_t pa = warp; pa < ti; pa += J_THREADS / 32) {
-        const uint32_t gi = i0 + pa, iid = ids[gi];
-        for (uint32_t pj0 = 0; pj0 < tj; pj0 += 32) {
-          const uint32_t pj = pj0 + lane, gj = j0 + pj;
-          bool valid = false;
-          uint32_t jid = 0;
-          if (pj < tj) {
-            jid = ids[gj];
-            valid = gj < a ? (iid < jid) : (iid != jid);
-          }
-          float dist = 0.f;
-          if (valid) {
-            const float4 *x = reinterpret_cast<const float4 *>(ri + (size_t)pa * stride);
-            const float4 *y = reinterpret_cast<const float4 *>(rj + (size_t)pj * stride);
-            for (uint32_t g = 0; g < d4; g++) dist = __fadd_rn(dist, group4(x[g], y[g]));
-            npairs++;
-          }
-          const unsigned long long kbase = ((unsigned long long)n << 32) | ((gi * tot + gj) << 1);
-          // offer 1: insert(i <- j); offer 2: insert(j <- i)
-          bool ok1 = valid && s.psz[iid] > 0 && dist <= s.pool[(size_t)iid * s.L].d;
-          emit(of, ok1, iid, kbase, jid, dist, lane, status);
-          bool ok2 = valid && s.psz[jid] > 0 && dist <= s.pool[(size_t)jid * s.L].d;
-          emit(of, ok2, jid, kbase | 1ull, iid, dist, lane, status);
-        }
-      }
-    }
-  }
-  if (pairs) {
-    for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(FULL, npairs, o);
-    if (lane == 0 && npairs) atomicAdd(pairs, npairs);
-  }
+// nhood::insert's first test is against the pool's current maximum, the
+// heap's front (an empty pool takes nothing in a join)
+__global__ void k_pool_max(Nnd s, float *mx) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < s.n) mx[i] = s.psz[i] > 0 ? s.pool[(size_t)i * s.L].d : __int_as_float(0xff800000);
 }
 
-// ---------------------------------------------------------------- join on the tensor cores
-// The same local join for integer data in [0, 255] with d a multiple of 16,
-// d <= 128 and new lists of at most 128 ids: every pair distance is the
-// norm form |x|^2 + |y|^2 - 2 x.y with the dot products of a Gram tile
-// computed by tcgen05.mma, BF16 operands (the integer values are exact in
-// BF16, their products in FP32) and FP32 accumulation in tensor memory --
-// every partial sum an integer below 2^24, so the distances are the exact
-// FP32 values the reference's sequential sum gives, and the offers (targets,
-// keys, candidates, distances) are those of k_join.
-//
-// One CTA of 8 warps per node.  The node's rows (new ++ old) are converted to
-// BF16 into the canonical no-swizzle K-major layout (8 x 8 core matrices of
-// 16-byte rows, K-adjacent core matrices 128 bytes apart, 8-row groups d * 16
-// bytes apart).  The first 128 rows (the new rows, then old ones) are the B
-// operand (N = the new rows rounded up to 16) and also the first A tile;
-// later A tiles of 128 rows take the second buffer.  Per tile one thread
-// issues d / 16 MMAs (M = 128, N, K = 16) into up to 128 columns of tensor
-// memory and commits to an mbarrier; warp w reads accumulator lanes
-// 32(w % 4).. (rows j of new ++ old) 16 columns (new rows i) at a time with
-// tcgen05.ld and emits the two offers of each valid pair (i, j) -- warps w
-// and w + 4 share lanes 32w.. and split the columns; all warps hold rows,
-// the columns run over the short new list.  The targets'
-// pool maxima are read once per node into shared memory (pools do not change
-// during a join chunk).  The wait on the MMAs is bounded: on time-out the CTA
-// reports DEV_TIMEOUT, waits (bounded) once more for its MMAs and frees its
-// tensor memory.
-constexpr int JT_THREADS = 256;  // 8 warps: warps w and w + 4 share TMEM lanes 32w.. (column halves)
-constexpr uint32_t JT_ROWS = 128;  // rows per operand buffer (M of A, the N chunk of B)
-constexpr uint32_t JT_LBO = 128;
-constexpr uint32_t JT_TMEM_COLS = 128;
+// row stride of integer rows in shared memory: an odd multiple of 16 bytes
+// (the fragments' word loads then fall into different banks)
+__host__ __device__ inline uint32_t ji_stride(uint32_t d) { return (d / 16) % 2 ? d : d + 16; }
 
-__device__ __forceinline__ uint32_t jt_pack(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t *>(&v);
+// bytes b0..b3 of an integer row as two half pairs: 0x6400 | b is 1024 + b
+__device__ __forceinline__ void ji_halves(uint32_t w, uint32_t &lo, uint32_t &hi) {
+  const uint32_t k = 0x64646464u, m = 0x64006400u;
+  const uint32_t l = __byte_perm(w, k, 0x4140), h = __byte_perm(w, k, 0x4342);
+  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(l), "r"(m));
+  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(h), "r"(m));
+}
+__device__ __forceinline__ void ji_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// rows [r0, r0 + 128) of the node's list as BF16 in the K-major core layout
-// (zeros past tot).  Item e is the 16-byte core row at byte offset 16 e of
-// the layout (8-row group e / (8 kc), core matrix (e / 8) % kc, row e % 8):
-// consecutive threads store consecutive 16 bytes (no bank conflicts) and
-// each loads 32 bytes of one row.
-__device__ void jt_stage(uint8_t *dst, const float *__restrict__ base, uint32_t d, const uint32_t *ids, uint32_t tot,
-                         uint32_t r0, int tid) {
-  const uint32_t kc = d / 8;
-  for (uint32_t e = tid; e < JT_ROWS * kc; e += JT_THREADS) {
-    const uint32_t r = (e / (8 * kc)) * 8 + (e & 7), k = ((e >> 3) % kc) * 8;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r0 + r < tot) {
-      const float4 *src = reinterpret_cast<const float4 *>(base + (size_t)ids[r0 + r] * d + k);
-      const float4 x0 = __ldg(src), x1 = __ldg(src + 1);
-      v = make_uint4(jt_pack(x0.x, x0.y), jt_pack(x0.z, x0.w), jt_pack(x1.x, x1.y), jt_pack(x1.z, x1.w));
-    }
-    reinterpret_cast<uint4 *>(dst)[e] = v;
-  }
-}
-
-size_t join_tc_smem(uint32_t d, uint32_t capn, uint32_t capo) {
-  return 2 * (size_t)JT_ROWS * d * 2 + 3 * (size_t)(capn + capo) * 4 + 16;
-}
-
-__global__ void __launch_bounds__(JT_THREADS) k_join_tc(Nnd s, uint32_t n0, Offers of, unsigned long long *pairs,
-                                                        int *status) {
-  extern __shared__ __align__(16) uint8_t smem[];  // (the no-swizzle layout needs 16-byte alignment)
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tmem_base;
-  const uint32_t n = n0 + blockIdx.x;
-  const uint32_t a = s.lnew[n], b = s.lold[n];
-  if (a == 0) return;  // (block-uniform, before any tensor memory is taken)
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t tot = a + b, d = s.d;
-  const uint32_t sbo = (d / 8) * 128;
-  uint8_t *tA = smem, *tB = smem + (size_t)JT_ROWS * d * 2;
-  uint32_t *ids = reinterpret_cast<uint32_t *>(tB + (size_t)JT_ROWS * d * 2);
-  float *nrm = reinterpret_cast<float *>(ids + s.capn + s.capo);
-  float *mx = nrm + s.capn + s.capo;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(umma::smem_u32(&tmem_base)),
-                 "r"(JT_TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  if (tid == 0) {
-    umma::mbar_init(&bar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;");
-  }
-  for (uint32_t t = tid; t < tot; t += JT_THREADS) {
-    const uint32_t id = t < a ? s.nnew[(size_t)n * s.capn + t] : s.nold[(size_t)n * s.capo + (t - a)];
-    ids[t] = id;
-    nrm[t] = s.xnorm[id];
-    // nhood::insert's first test against the pool's current maximum (an
-    // empty pool takes nothing here, as k_join's psz test)
-    mx[t] = s.psz[id] > 0 ? s.pool[(size_t)id * s.L].d : __int_as_float(0xff800000);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = tmem_base;
-  jt_stage(tA, s.base, d, ids, tot, 0, tid);
-  unsigned long long npairs = 0;
-  uint32_t phase = 0;
-  bool ok = true;
-  const uint32_t acols = (a + 15) & ~15u;  // N: the new rows, rounded up to 16
-  for (uint32_t m0 = 0; m0 < tot && ok; m0 += JT_ROWS) {
-    const uint8_t *at = m0 == 0 ? tA : tB;
-    if (m0 > 0) jt_stage(tB, s.base, d, ids, tot, m0, tid);
-    asm volatile("fence.proxy.async.shared::cta;");  // generic stores -> tensor core reads
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t a0 = umma::smem_u32(at), b0 = umma::smem_u32(tA);
-      const uint32_t idesc = umma::idesc(128, (int)acols);
-      for (uint32_t kk = 0; kk < d / 16; kk++) {
-        const uint64_t ad = umma::desc(a0 + kk * 2 * JT_LBO, JT_LBO, sbo);
-        const uint64_t bd = umma::desc(b0 + kk * 2 * JT_LBO, JT_LBO, sbo);
-        const uint32_t acc = kk > 0 ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-            "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          umma::smem_u32(&bar)));
-    }
-    ok = __syncthreads_and(umma::mbar_wait(&bar, phase)) != 0;
-    phase ^= 1;
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    if (!ok) break;
-    // warp w: TMEM lanes 32 (w % 4).. (rows of new ++ old), columns (new
-    // rows) of half w / 4
-    const uint32_t quad = warp & 3, chalf = (uint32_t)(warp >> 2) * 64;
-    if (m0 + quad * 32 < tot) {
-      const uint32_t gj = m0 + quad * 32 + lane;  // this lane's row of new ++ old
-      const bool rowok = gj < tot;
-      const uint32_t jid = rowok ? ids[gj] : 0u;
-      const float nj = rowok ? nrm[gj] : 0.f, mj = rowok ? mx[gj] : __int_as_float(0xff800000);
-      for (uint32_t c0 = chalf; c0 < a && c0 < chalf + 64; c0 += 16) {
-        uint32_t v[16];
-        const uint32_t addr = tmem + ((quad * 32) << 16) + c0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(addr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;");
+// distances of rows J (tj of them) x rows I (ti) into G (row j0 + j, column
+// i0 + i): dot products of the integer values on the tensor cores (exact in
+// FP16; FP32 sums are integers below 2^24 for d <= 256) and the norm form in
+// 32-bit integers, converted to the FP32 value the reference's sum gives.
+// Rows past ti / tj (in the staging area, whatever it holds) only reach
+// columns / rows of the tile that are dropped.
+__device__ __forceinline__ void ji_tile(const uint8_t *I, const uint8_t *J, uint32_t stride, uint32_t d, uint32_t ti, uint32_t tj,
+                        uint32_t i0, uint32_t j0, const int *nrm, float *G, uint32_t gs, int warp, int nwarps,
+                        int lane) {
+  const int g = lane >> 2, j = lane & 3;
+  for (uint32_t mt = warp; mt * 16 < tj; mt += nwarps) {
+    for (uint32_t nb = 0; nb < ti; nb += 32) {
+      float acc[4][4];
 #pragma unroll
-        for (int ii = 0; ii < 16; ii++) {
-          const uint32_t gi = c0 + ii;  // a new row (warp-uniform)
-          if (gi >= a) continue;
-          const uint32_t iid = ids[gi];
-          const bool valid = rowok && (gj < a ? (iid < jid) : (iid != jid));
-          // integers below 2^24 throughout: the exact FP32 distance
-          const float dist = (nrm[gi] + nj) - 2.f * __uint_as_float(v[ii]);
-          npairs += valid;
-          const unsigned long long kbase = ((unsigned long long)n << 32) | ((gi * tot + gj) << 1);
-          emit(of, valid && dist <= mx[gi], iid, kbase, jid, dist, lane, status);
-          emit(of, valid && dist <= mj, jid, kbase | 1ull, iid, dist, lane, status);
+      for (int t = 0; t < 4; t++) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+      const uint32_t *ja = reinterpret_cast<const uint32_t *>(J + (size_t)(mt * 16 + g) * stride) + j;
+      const uint32_t *jb = reinterpret_cast<const uint32_t *>(J + (size_t)(mt * 16 + g + 8) * stride) + j;
+      const uint32_t *ib = reinterpret_cast<const uint32_t *>(I + (size_t)(nb + g) * stride) + j;
+      for (uint32_t k = 0; k < d / 4; k += 4) {
+        uint32_t a[4];
+        ji_halves(ja[k], a[0], a[2]);
+        ji_halves(jb[k], a[1], a[3]);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          if (nb + t * 8 < ti) {
+            uint32_t b0, b1;
+            ji_halves(ib[(size_t)t * 2 * stride + k], b0, b1);
+            ji_mma(acc[t], a, b0, b1);
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const uint32_t jj = mt * 16 + g + (e >> 1) * 8, ii = nb + t * 8 + 2 * j + (e & 1);
+          if (jj < tj && ii < ti)
+            G[(size_t)(j0 + jj) * gs + i0 + ii] =
+                (float)(nrm[j0 + jj] + nrm[i0 + ii] - 2 * __float2int_rn(acc[t][e]));
         }
       }
     }
-    // the accumulator is read and the A buffer free before the next tile
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
   }
-  if (!ok) {
-    if (tid == 0) set_err(status, DEV_TIMEOUT);
-    // the MMAs of the chunk that timed out may still run: wait for them
-    // (bounded) before the tensor memory is freed
-    umma::mbar_wait(&bar, phase ^ 1);
-  }
-  if (pairs) {
-    for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(FULL, npairs, o);
-    if (lane == 0 && npairs) atomicAdd(pairs, npairs);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(JT_TMEM_COLS));
 }
 
-// targets with offers, and the largest segment
-__global__ void k_active(uint32_t n, const uint32_t *tcnt, uint32_t *act, uint32_t *nact, uint32_t *big,
-                         uint32_t *nbig, uint32_t warp_cap, uint32_t *maxseg) {
+// the local join of nodes [n0, n1), a node per block at a time.  I8: integer
+// rows in [0, 255] from the byte copy of the base (d a multiple of 16, d <=
+// 256); else FP32 rows, every distance folded in the reference's order.
+template <bool I8>
+__global__ void __launch_bounds__(I8 ? JI_THREADS : J_THREADS)
+    k_join(Nnd s, uint32_t n0, uint32_t n1, JoinOut o, JoinCfg cf, unsigned long long *pairs) {
+  constexpr int T = I8 ? JI_THREADS : J_THREADS, NW = T / 32;
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ unsigned long long ebase;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t capt = s.capn + s.capo;
+  const uint32_t stride = I8 ? ji_stride(s.d) : (((s.d + 3) & ~3u) + 4) * 4;  // bytes
+  const size_t rbytes = (size_t)(I8 ? JI_ROWS : J_TI + cf.tj) * stride;
+  float *Gs = reinterpret_cast<float *>(smem + rbytes);
+  uint32_t *ids = cf.lscr ? cf.lscr + (size_t)blockIdx.x * 4 * capt : reinterpret_cast<uint32_t *>(Gs + cf.gcap);
+  float *mx = reinterpret_cast<float *>(ids + capt);
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(mx + capt);  // entries per target, then their offsets
+  int *nrm = reinterpret_cast<int *>(cnt + capt);           // (I8 only)
+  unsigned long long npairs = 0;
+  for (uint32_t n = n0 + blockIdx.x; n < n1; n += gridDim.x) {
+    const uint32_t a = s.lnew[n], b = s.lold[n];
+    if (a == 0) continue;  // block-uniform
+    const uint32_t tot = a + b, gs = a | 1u;
+    float *G = (size_t)tot * gs <= cf.gcap ? Gs : cf.gscr + (size_t)blockIdx.x * cf.gslab;
+    __syncthreads();  // the previous node's tile and lists are done with
+    for (uint32_t t = tid; t < tot; t += T) {
+      const uint32_t id = t < a ? s.nnew[(size_t)n * s.capn + t] : s.nold[(size_t)n * s.capo + (t - a)];
+      ids[t] = id;
+      mx[t] = o.mx[id];
+      if (I8) nrm[t] = (int)s.xnorm[id];
+    }
+    __syncthreads();
+    if constexpr (I8) {
+      const uint32_t ch = s.d / 16;
+      auto stage = [&](uint8_t *dst, uint32_t r0, uint32_t cntr) {
+        for (uint32_t e = tid; e < cntr * ch; e += T) {
+          const uint32_t r = e / ch, k = e % ch;
+          cp_async16(dst + (size_t)r * stride + k * 16, s.base8 + (size_t)ids[r0 + r] * s.d + k * 16);
+        }
+      };
+      if (tot <= JI_ROWS) {
+        stage(smem, 0, tot);
+        cp_async_wait_all();
+        __syncthreads();
+        ji_tile(smem, smem, stride, s.d, a, tot, 0, 0, nrm, G, gs, warp, NW, lane);
+      } else {
+        uint8_t *J = smem + (size_t)64 * stride;
+        for (uint32_t i0 = 0; i0 < a; i0 += 64)
+          for (uint32_t j0 = 0; j0 < tot; j0 += 64) {
+            const uint32_t ti = min(64u, a - i0), tj = min(64u, tot - j0);
+            __syncthreads();
+            if (j0 == 0) stage(smem, i0, ti);
+            stage(J, j0, tj);
+            cp_async_wait_all();
+            __syncthreads();
+            ji_tile(smem, J, stride, s.d, ti, tj, i0, j0, nrm, G, gs, warp, NW, lane);
+          }
+      }
+    } else {
+      const uint32_t fs = stride / 4, d4 = s.d >> 2;
+      float *ri = reinterpret_cast<float *>(smem);
+      float *rj = ri + (size_t)J_TI * fs;
+      for (uint32_t i0 = 0; i0 < a; i0 += J_TI) {
+        const uint32_t ti = min((uint32_t)J_TI, a - i0);
+        for (uint32_t j0 = 0; j0 < tot; j0 += cf.tj) {
+          const uint32_t tj = min(cf.tj, tot - j0);
+          if (j0 + tj <= min(a, i0 + 1)) continue;  // both new: computed with the roles exchanged
+          __syncthreads();
+          // stage rows (coalesced 16-byte copies, one row per warp step)
+          for (uint32_t r = warp; r < ti + tj; r += NW) {
+            const uint32_t id = r < ti ? ids[i0 + r] : ids[j0 + (r - ti)];
+            float *dst = r < ti ? ri + (size_t)r * fs : rj + (size_t)(r - ti) * fs;
+            const float *src = s.base + (size_t)id * s.d;
+            for (uint32_t k = lane; k < d4; k += 32) cp_async16(dst + 4 * k, src + 4 * k);
+          }
+          cp_async_wait_all();
+          __syncthreads();
+          // warps take i rows, lanes take j rows; a pair of new rows is
+          // computed once (the distance is symmetric bit for bit)
+          for (uint32_t pa = warp; pa < ti; pa += NW) {
+            const uint32_t gi = i0 + pa;
+            for (uint32_t pj0 = 0; pj0 < tj; pj0 += 32) {
+              const uint32_t pj = pj0 + lane, gj = j0 + pj;
+              if (pj >= tj || gj <= (gj < a ? gi : 0u)) continue;
+              const float4 *x = reinterpret_cast<const float4 *>(ri + (size_t)pa * fs);
+              const float4 *y = reinterpret_cast<const float4 *>(rj + (size_t)pj * fs);
+              float dist = 0.f;
+              for (uint32_t k = 0; k < d4; k++) dist = __fadd_rn(dist, group4(x[k], y[k]));
+              G[(size_t)gj * gs + gi] = dist;
+              if (gj < a) G[(size_t)gi * gs + gj] = dist;
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // offers per target: pairs of different ids (a pair of new rows is
+    // evaluated in one of its two orders, whatever the positions)
+    for (uint32_t p = warp; p < tot; p += NW) {
+      const uint32_t pid = ids[p];
+      const float m = mx[p];
+      const uint32_t end = p < a ? tot : a;
+      uint32_t c = 0;
+      for (uint32_t q0 = 0; q0 < end; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        bool diff = false, ok = false;
+        if (q < end) {
+          diff = ids[q] != pid;
+          ok = diff && (q < a ? G[(size_t)p * gs + q] : G[(size_t)q * gs + p]) <= m;
+        }
+        c += __popc(__ballot_sync(FULL, ok));
+        if (p < a && pairs) npairs += diff && (q >= a || pid < ids[q]);
+      }
+      if (lane == 0) cnt[p] = c;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t run = 0;
+      for (uint32_t p0 = 0; p0 < tot; p0 += 32) {
+        const uint32_t p = p0 + lane;
+        const uint32_t c = p < tot ? cnt[p] : 0u;
+        uint32_t x = c;
+        for (int k = 1; k < 32; k <<= 1) {
+          const uint32_t y = __shfl_up_sync(FULL, x, k);
+          if (lane >= k) x += y;
+        }
+        if (p < tot) cnt[p] = run + x;  // inclusive ends
+        run += __shfl_sync(FULL, x, 31);
+      }
+      if (lane == 0) ebase = run ? atomicAdd(o.cursor, (unsigned long long)run) : 0ull;
+    }
+    __syncthreads();
+    const uint32_t total = cnt[tot - 1];
+    if (total == 0 || ebase + total > o.cap) continue;  // block-uniform
+    for (uint32_t p = tid; p < tot; p += T) {
+      const uint32_t e0 = p ? cnt[p - 1] : 0u, c = cnt[p] - e0;
+      if (c) {
+        const uint32_t t = ids[p];
+        o.desc[o.toff[t] + atomicAdd(&o.tcur[t], 1u)] = make_uint4((uint32_t)(ebase + e0), c, n, p);
+      }
+    }
+    for (uint32_t p = warp; p < tot; p += NW) {
+      const uint32_t e0 = p ? cnt[p - 1] : 0u;
+      if (cnt[p] == e0) continue;
+      const uint32_t pid = ids[p];
+      const float m = mx[p];
+      const uint32_t end = p < a ? tot : a;
+      size_t at = (size_t)ebase + e0;
+      for (uint32_t q0 = 0; q0 < end; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        float dist = 0.f;
+        bool ok = false;
+        if (q < end && ids[q] != pid) {
+          dist = q < a ? G[(size_t)p * gs + q] : G[(size_t)q * gs + p];
+          ok = dist <= m;
+        }
+        const unsigned om = __ballot_sync(FULL, ok);
+        if (ok) {
+          const size_t w = at + __popc(om & lt);
+          o.ent[w] = make_uint2(__float_as_uint(dist), ids[q]);
+          o.eq[w] = (uint16_t)q;
+        }
+        at += __popc(om);
+      }
+    }
+  }
+  if (pairs) {
+    for (int k = 16; k > 0; k >>= 1) npairs += __shfl_xor_sync(FULL, npairs, k);
+    if (lane == 0 && npairs) atomicAdd(pairs, npairs);
+  }
+}
+
+// ---------------------------------------------------------------- offers into the pools
+// A warp reads the entries of one target through up to 32 descriptors at a
+// time as one flat range: lane l of step e0 takes entry e0 + l, whose
+// descriptor it finds by a binary search over the descriptors' prefix sums.
+struct SegBatch {
+  uint32_t off, cnt, incl, n, p, total;
+  __device__ void load(const uint4 *desc, uint32_t b, uint32_t dn, int lane) {
+    const uint4 v = b + lane < dn ? desc[b + lane] : make_uint4(0u, 0u, 0u, 0u);
+    off = v.x;
+    cnt = v.y;
+    n = v.z;
+    p = v.w;
+    incl = cnt;
+    for (int k = 1; k < 32; k <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, incl, k);
+      if (lane >= k) incl += y;
+    }
+    total = __shfl_sync(FULL, incl, 31);
+  }
+  // the descriptor (lane) of flat entry e < total, and the entry's index
+  __device__ int find(uint32_t e, uint32_t &idx) const {
+    int lo = 0;
+#pragma unroll
+    for (int st = 16; st > 0; st >>= 1)
+      if (__shfl_sync(FULL, incl, lo + st - 1) <= e) lo += st;
+    lo = min(lo, 31);
+    const uint32_t ex = __shfl_sync(FULL, incl - cnt, lo);
+    idx = __shfl_sync(FULL, off, lo) + (e - ex);
+    return lo;
+  }
+};
+
+// merges up to 32 offers (one per lane, key = distance bits << 32 | id, ~0
+// for none) into the sorted pool: repeats of an offer or of a pool entry are
+// dropped (the same id has the same distance), the rest are placed by rank.
+// fmin: the least distance this lane saw fall off the pool's end.
+__device__ __forceinline__ void fast_merge(float *pd, uint32_t *pi, uint32_t &sz, uint32_t L, unsigned long long key, uint32_t *pos,
+                           float &fmin, int lane) {
+  const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+  for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      const unsigned long long y = __shfl_xor_sync(FULL, key, j);
+      const bool lower = ((lane & j) == 0) == ((lane & k) == 0);
+      key = lower ? (key < y ? key : y) : (key < y ? y : key);
+    }
+  const unsigned long long prev = __shfl_up_sync(FULL, key, 1);
+  bool keep = key != ~0ull && !(lane > 0 && prev == key);
+  const float dist = __uint_as_float((uint32_t)(key >> 32));
+  const uint32_t id = (uint32_t)key;
+  uint32_t lo = 0, hi = keep ? sz : 0u;
+  while (lo < hi) {
+    const uint32_t m = (lo + hi) >> 1;
+    const unsigned long long pk = ((unsigned long long)__float_as_uint(pd[m]) << 32) | (pi[m] & ID_MASK);
+    if (pk < key) lo = m + 1;
+    else hi = m;
+  }
+  if (keep && lo < sz && (pi[lo] & ID_MASK) == id && pd[lo] == dist) keep = false;
+  const unsigned km = __ballot_sync(FULL, keep);
+  if (!km) return;
+  const int nk = __popc(km), r = __popc(km & lt);
+  if (keep) pos[r] = lo;
+  __syncwarp();
+  const int first = (int)pos[0];
+  for (int jt = (int)sz; jt > first; jt -= 32) {
+    const int j = jt - 32 + lane;
+    const bool act = j >= first;
+    float v = 0.f;
+    uint32_t x = 0;
+    int np = 0;
+    if (act) {
+      v = pd[j];
+      x = pi[j];
+      int l2 = 0, h2 = nk;  // offers placed at or before entry j
+      while (l2 < h2) {
+        const int m = (l2 + h2) >> 1;
+        if ((int)pos[m] <= j) l2 = m + 1;
+        else h2 = m;
+      }
+      np = j + l2;
+    }
+    __syncwarp();
+    if (act) {
+      if (np < (int)L) {
+        pd[np] = v;
+        pi[np] = x;
+      } else {
+        fmin = fminf(fmin, v);
+      }
+    }
+    __syncwarp();
+  }
+  if (keep) {
+    const uint32_t np = lo + r;
+    if (np < L) {
+      pd[np] = dist;
+      pi[np] = id | FLAG;
+    } else {
+      fmin = fminf(fmin, dist);
+    }
+  }
+  sz = min(L, sz + (uint32_t)nk);
+  __syncwarp();
+}
+
+constexpr int AF_WARPS = 8;
+constexpr uint32_t AP_WARP_CAP = 1024;   // offers per target for the warp replay
+constexpr uint32_t AP_BIG_CAP = 8192;    // offers per target for the block replay in shared memory (power of 2)
+
+// the targets left to the replay, by their number of offers, and the sizes
+// the host needs
+struct Redo {
+  uint32_t *cnt;   // [0] warp, [1] block, [2] block with global scratch, [3] most offers of the last
+  uint32_t *list[3];
+};
+__device__ __forceinline__ void redo_push(const Redo &r, uint32_t t, uint32_t cnt) {
+  const int k = cnt <= AP_WARP_CAP ? 0 : cnt <= AP_BIG_CAP ? 1 : 2;
+  r.list[k][atomicAdd(r.cnt + k, 1u)] = t;
+  if (k == 2) atomicMax(r.cnt + 3, cnt);
+}
+
+__host__ __device__ inline size_t af_warp_words(uint32_t L) { return 2 * (((size_t)L + 3) & ~size_t(3)) + 128 + 32; }
+
+// nhood::insert (index.h:120-135) of all of a target's offers, in any order.
+// Sequentially an offer enters when it is not farther than the current
+// maximum and its id is not pooled, and the maximum leaves a full pool; the
+// maximum only falls, so the pool ends as the L least of the pool and the
+// offers (repeats once, none above the first maximum).  The heap's
+// arrangement depends on the order, but the update that follows sorts the
+// pool, so the arrangement matters only where distances tie: a target with
+// two equal distances among the kept entries, or between a kept and a dropped
+// one, is left as it was and replayed in the reference's order
+// (k_replay_*).  Bound by latency (entries from L2, merges in shared memory):
+// the seven joins of the 100k x 128 build take 2.1 ms here and 5.2 ms in the
+// replays (a tenth of its integer targets tie), against 37 ms when every
+// target sorted and replayed its offers; 5.6 + 5.6 ms against 504 ms on the
+// six joins of 60k x 96 with up to 100 reverse neighbours.  srt: the pools sorted as the last update left them, flags
+// not yet cleared; the first mclr[t] entries' flags are cleared here (null:
+// none).
+__global__ void __launch_bounds__(AF_WARPS * 32)
+    k_apply_fast(Nnd s, const Ent *srt, const uint32_t *mclr, JoinOut o, Redo redo) {
+  extern __shared__ __align__(16) uint32_t af_smem[];
+  if (*o.cursor > o.cap) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t L = s.L, Lp = (L + 3) & ~3u;
+  uint32_t *sm = af_smem + warp * af_warp_words(L);
+  float *pd = reinterpret_cast<float *>(sm);
+  uint32_t *pi = sm + Lp;
+  uint2 *buf = reinterpret_cast<uint2 *>(sm + 2 * Lp);  // 64 waiting offers
+  uint32_t *pos = sm + 2 * Lp + 128;
+  for (uint32_t t = blockIdx.x * AF_WARPS + warp; t < s.n; t += gridDim.x * AF_WARPS) {
+    const uint32_t dn = o.tcur[t];
+    if (dn == 0) continue;
+    uint32_t sz = s.psz[t];
+    const uint32_t mc = mclr ? mclr[t] : 0u;
+    for (uint32_t j = lane; j < sz; j += 32) {
+      const Ent e = srt[(size_t)t * L + j];
+      pd[j] = e.d;
+      pi[j] = j < mc ? (e.idf & ID_MASK) : e.idf;
+    }
+    __syncwarp();
+    const float mx0 = pd[sz - 1];  // (a target with offers has a pool)
+    float thr = mx0, fmin = __int_as_float(0x7f800000);
+    uint32_t nb = 0, offers = 0;
+    const uint4 *dsc = o.desc + o.toff[t];
+    bool any = false;
+    for (uint32_t b = 0; b < dn; b += 32) {
+      SegBatch sb;
+      sb.load(dsc, b, dn, lane);
+      offers += sb.total;
+      for (uint32_t e0 = 0; e0 < sb.total; e0 += 64) {
+        uint32_t i0, i1;
+        sb.find(e0 + lane, i0);
+        sb.find(e0 + 32 + lane, i1);
+        const bool h0 = e0 + lane < sb.total, h1 = e0 + 32 + lane < sb.total;
+        const uint2 v0 = h0 ? __ldg(o.ent + i0) : make_uint2(0u, 0u);
+        const uint2 v1 = h1 ? __ldg(o.ent + i1) : make_uint2(0u, 0u);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const uint2 v = h ? v1 : v0;
+          const bool ok = (h ? h1 : h0) && __uint_as_float(v.x) <= thr;
+          const unsigned m = __ballot_sync(FULL, ok);
+          if (!m) continue;
+          if (ok) buf[nb + __popc(m & lt)] = v;
+          nb += __popc(m);
+          __syncwarp();
+          if (nb >= 32) {
+            const uint2 w = buf[lane];
+            const uint2 rest = lane + 32 < (int)nb ? buf[lane + 32] : make_uint2(0u, 0u);
+            __syncwarp();
+            buf[lane] = rest;
+            nb -= 32;
+            __syncwarp();
+            fast_merge(pd, pi, sz, L, ((unsigned long long)w.x << 32) | w.y, pos, fmin, lane);
+            if (sz == L) thr = pd[L - 1];
+            any = true;
+          }
+        }
+      }
+    }
+    if (nb) {
+      const uint2 w = buf[lane];
+      fast_merge(pd, pi, sz, L, lane < (int)nb ? ((unsigned long long)w.x << 32) | w.y : ~0ull, pos, fmin, lane);
+      any = true;
+    }
+    if (any) {
+      bool tie = sz == L && fmin == pd[L - 1];
+      for (uint32_t j = lane; j + 1 < sz; j += 32) tie |= pd[j] == pd[j + 1];
+      if (__any_sync(FULL, tie)) {
+        if (lane == 0) redo_push(redo, t, offers);
+      } else {
+        for (uint32_t j = lane; j < sz; j += 32) s.pool[(size_t)t * L + j] = Ent{pd[j], pi[j]};
+        if (lane == 0) s.psz[t] = sz;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// every target with offers to the replay (joins in several chunks, whose
+// heaps must keep the reference's arrangement, and init rows whose distances
+// are not those of their ids)
+__global__ void k_redo_all(uint32_t n, JoinOut o, Redo redo) {
+  if (*o.cursor > o.cap) return;
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  uint32_t c = tcnt[t];
-  if (c == 0) return;
-  atomicMax(maxseg, c);
-  if (c <= warp_cap) act[atomicAdd(nact, 1u)] = t;
-  else big[atomicAdd(nbig, 1u)] = t;
+  const uint32_t dn = o.tcur[t];
+  if (!dn) return;
+  uint32_t cnt = 0;
+  for (uint32_t k = 0; k < dn; k++) cnt += o.desc[o.toff[t] + k].y;
+  redo_push(redo, t, cnt);
 }
 
 struct WarpSync {
@@ -782,12 +1024,29 @@ struct Grouped {
   float dist;
 };
 
-__global__ void k_group(uint32_t count, Offers of, const uint32_t *toff, uint32_t *tcur, Grouped *g) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= count) return;
-  uint32_t t = of.tgt[r];
-  uint32_t pos = toff[t] + atomicAdd(&tcur[t], 1u);
-  g[pos] = Grouped{of.key[r], of.cand[r], of.dist[r]};
+// one warp gathers target t's entries with their keys -- the reference's
+// sequential position (node n, pair position in nhood::join's loops, side) --
+// into k; batches of 32 descriptors b0, b0 + bstep, ...  `at`: where the
+// warp's entries go
+__device__ __forceinline__ void gather_offers(const Nnd &s, const JoinOut &o, uint32_t t, uint32_t dn, uint32_t b, uint32_t at,
+                              Grouped *k, int lane) {
+  SegBatch sb;
+  sb.load(o.desc + o.toff[t], b, dn, lane);
+  for (uint32_t e0 = 0; e0 < sb.total; e0 += 32) {
+    uint32_t idx;
+    const int l = sb.find(e0 + lane, idx);
+    const uint32_t n = __shfl_sync(FULL, sb.n, l), p = __shfl_sync(FULL, sb.p, l);
+    if (e0 + lane < sb.total) {
+      const uint2 v = o.ent[idx];
+      const uint32_t q = o.eq[idx], a = s.lnew[n], tot = a + s.lold[n];
+      // the pair (i, j): i new, and of two new rows the one of smaller id;
+      // side 0 offers j to i, side 1 i to j
+      const bool side0 = p < a && (q >= a || t < v.y);
+      const uint32_t gi = side0 ? p : q, gj = side0 ? q : p;
+      k[at + e0 + lane] = Grouped{((unsigned long long)n << 32) | ((gi * tot + gj) << 1) | (side0 ? 0u : 1u), v.y,
+                                  __uint_as_float(v.x)};
+    }
+  }
 }
 
 // sorts `cnt` grouped offers by key in shared memory (P = pow2 >= cnt),
@@ -846,54 +1105,102 @@ __device__ void apply_offers(Ent *P, uint32_t &sz, uint32_t L, const Grouped *of
   }
 }
 
+// the replay of the targets in redo.list[0]: a warp per target, offers sorted
+// by key in shared memory
 constexpr int AP_WARPS = 4;
-constexpr uint32_t AP_WARP_CAP = 1024;   // offers per target for the warp path
-constexpr uint32_t AP_BIG_CAP = 8192;    // offers per target for the block path (power of 2)
-
-__global__ void __launch_bounds__(AP_WARPS * 32)
-    k_apply_warp(Nnd s, const uint32_t *act, const uint32_t *nact, const uint32_t *toff, const uint32_t *tcnt,
-                 Grouped *g) {
+__global__ void __launch_bounds__(AP_WARPS * 32) k_replay_warp(Nnd s, JoinOut o, Redo redo) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t w = blockIdx.x * AP_WARPS + warp;
-  if (w >= *nact) return;
   Grouped *k = (Grouped *)smem + (size_t)warp * AP_WARP_CAP;
   Ent *P = (Ent *)((Grouped *)smem + (size_t)AP_WARPS * AP_WARP_CAP) + (size_t)warp * (s.L + 1);
-  const uint32_t t = act[w], cnt = tcnt[t], off = toff[t];
-  int Pn = 1;
-  while (Pn < (int)cnt) Pn <<= 1;
-  for (int i = lane; i < Pn; i += 32) k[i] = i < (int)cnt ? g[off + i] : Grouped{~0ull, 0u, 0.f};
-  uint32_t sz = s.psz[t];
-  for (uint32_t i = lane; i < sz; i += 32) P[i] = s.pool[(size_t)t * s.L + i];
-  __syncwarp();
-  bitonic_grouped(k, Pn, lane, 32, WarpSync());
-  apply_offers(P, sz, s.L, k, cnt, lane);
-  for (uint32_t i = lane; i < sz; i += 32) s.pool[(size_t)t * s.L + i] = P[i];
-  if (lane == 0) s.psz[t] = sz;
+  const uint32_t m = redo.cnt[0];
+  for (uint32_t w = blockIdx.x * AP_WARPS + warp; w < m; w += gridDim.x * AP_WARPS) {
+    const uint32_t t = redo.list[0][w], dn = o.tcur[t];
+    uint32_t cnt = 0;
+    for (uint32_t b = 0; b < dn; b += 32) {
+      uint32_t c = b + lane < dn ? o.desc[o.toff[t] + b + lane].y : 0u;
+      for (int x = 16; x > 0; x >>= 1) c += __shfl_xor_sync(FULL, c, x);
+      gather_offers(s, o, t, dn, b, cnt, k, lane);
+      cnt += c;
+    }
+    int Pn = 1;
+    while (Pn < (int)cnt) Pn <<= 1;
+    for (int i = (int)cnt + lane; i < Pn; i += 32) k[i] = Grouped{~0ull, 0u, 0.f};
+    uint32_t sz = s.psz[t];
+    for (uint32_t i = lane; i < sz; i += 32) P[i] = s.pool[(size_t)t * s.L + i];
+    __syncwarp();
+    bitonic_grouped(k, Pn, lane, 32, WarpSync());
+    apply_offers(P, sz, s.L, k, cnt, lane);
+    for (uint32_t i = lane; i < sz; i += 32) s.pool[(size_t)t * s.L + i] = P[i];
+    if (lane == 0) s.psz[t] = sz;
+    __syncwarp();
+  }
 }
 
-__global__ void __launch_bounds__(512)
-    k_apply_block(Nnd s, const uint32_t *big, const uint32_t *toff, const uint32_t *tcnt, Grouped *g) {
+// the same for the targets of redo.list[1] (offers in shared memory) or
+// list[2] (gk: pcap keys of global scratch per block), a block per target
+constexpr int AB_THREADS = 512;
+__global__ void __launch_bounds__(AB_THREADS) k_replay_block(Nnd s, JoinOut o, Redo redo, Grouped *gk, uint32_t pcap) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const uint32_t t = big[blockIdx.x], cnt = tcnt[t], off = toff[t];
-  Grouped *k = (Grouped *)smem;
-  Ent *P = (Ent *)(k + AP_BIG_CAP);
-  __shared__ uint32_t szs;
-  int Pn = 1;
-  while (Pn < (int)cnt) Pn <<= 1;
-  for (int i = threadIdx.x; i < Pn; i += blockDim.x) k[i] = i < (int)cnt ? g[off + i] : Grouped{~0ull, 0u, 0.f};
-  const uint32_t sz0 = s.psz[t];
-  for (uint32_t i = threadIdx.x; i < sz0; i += blockDim.x) P[i] = s.pool[(size_t)t * s.L + i];
-  __syncthreads();
-  bitonic_grouped(k, Pn, threadIdx.x, blockDim.x, BlockSync());
-  if (threadIdx.x < 32) {
-    uint32_t sz = sz0;
-    apply_offers(P, sz, s.L, k, cnt, threadIdx.x);
-    if (threadIdx.x == 0) szs = sz;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Ent *P = (Ent *)smem;
+  Grouped *k = gk ? gk + (size_t)blockIdx.x * pcap : (Grouped *)(smem + ((size_t)(s.L + 2) & ~size_t(1)) * sizeof(Ent));
+  __shared__ uint32_t szs, fill;
+  const int li = gk ? 2 : 1;
+  const uint32_t m = redo.cnt[li];
+  for (uint32_t w = blockIdx.x; w < m; w += gridDim.x) {
+    const uint32_t t = redo.list[li][w], dn = o.tcur[t];
+    if (threadIdx.x == 0) fill = 0;
+    __syncthreads();
+    for (uint32_t b = 32 * warp; b < dn; b += AB_THREADS) {
+      uint32_t c = b + lane < dn ? o.desc[o.toff[t] + b + lane].y : 0u, at = 0;
+      for (int x = 16; x > 0; x >>= 1) c += __shfl_xor_sync(FULL, c, x);
+      if (lane == 0) at = atomicAdd(&fill, c);  // (any order: the keys are sorted next)
+      at = __shfl_sync(FULL, at, 0);
+      gather_offers(s, o, t, dn, b, at, k, lane);
+    }
+    __syncthreads();
+    const uint32_t cnt = fill;
+    int Pn = 1;
+    while (Pn < (int)cnt) Pn <<= 1;
+    for (int i = (int)cnt + threadIdx.x; i < Pn; i += AB_THREADS) k[i] = Grouped{~0ull, 0u, 0.f};
+    const uint32_t sz0 = s.psz[t];
+    for (uint32_t i = threadIdx.x; i < sz0; i += AB_THREADS) P[i] = s.pool[(size_t)t * s.L + i];
+    __syncthreads();
+    bitonic_grouped(k, Pn, threadIdx.x, AB_THREADS, BlockSync());
+    if (warp == 0) {
+      uint32_t sz = sz0;
+      apply_offers(P, sz, s.L, k, cnt, lane);
+      if (lane == 0) szs = sz;
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < szs; i += AB_THREADS) s.pool[(size_t)t * s.L + i] = P[i];
+    if (threadIdx.x == 0) s.psz[t] = szs;
+    __syncthreads();
   }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < szs; i += blockDim.x) s.pool[(size_t)t * s.L + i] = P[i];
-  if (threadIdx.x == 0) s.psz[t] = szs;
+}
+
+// whether every init row's distance is the distance of its ids (the
+// reference's order, a lane per entry): *ok = 0 where one is not, and the
+// joins then replay every target
+__global__ void k_check_rows(Nnd s, const uint32_t *ids, const float *dist, const uint32_t *deg, uint32_t w, int *ok) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5, d4 = s.d >> 2;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < s.n; i += nw) {
+    const uint32_t sz = min(deg[i], s.L);
+    const float4 *x = reinterpret_cast<const float4 *>(s.base + (size_t)i * s.d);
+    for (uint32_t j = lane; j < sz; j += 32) {
+      const uint32_t id = ids[(size_t)i * w + j];
+      if (id >= s.n) {
+        *ok = 0;
+        continue;
+      }
+      const float4 *y = reinterpret_cast<const float4 *>(s.base + (size_t)id * s.d);
+      float acc = 0.f;
+      for (uint32_t k = 0; k < d4; k++) acc = __fadd_rn(acc, group4(__ldg(x + k), __ldg(y + k)));
+      if (__float_as_uint(acc) != __float_as_uint(dist[(size_t)i * w + j])) *ok = 0;
+    }
+  }
 }
 
 // RefineInner tail: sort each pool, keep the first K (PruneNaive)
@@ -904,7 +1211,9 @@ __global__ void k_nnd_final(Nnd s, uint32_t *ids, float *dist, uint32_t *deg) {
   if (i >= s.n) return;
   const uint32_t sz = s.psz[i];
   for (uint32_t j = 0; j < sz; j++) P[j] = s.pool[(size_t)i * s.L + j];
-  stl::sort(P, (int)sz, EntLess());
+  bool asc = true;
+  for (uint32_t j = 1; j < sz; j++) asc &= P[j - 1].d < P[j].d;
+  if (!asc) stl::sort(P, (int)sz, EntLess());
   const uint32_t k = min(sz, s.K);
   for (uint32_t j = 0; j < k; j++) {
     ids[(size_t)i * s.K + j] = P[j].idf & ID_MASK;
@@ -1008,6 +1317,7 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
   s.capo = std::min(p.L + p.R, 2 * p.R);
   s.base = c->base.as<float>();
   s.xnorm = c->base_int ? c->xnorm.as<float>() : nullptr;
+  s.base8 = c->base_int && c->base8.p ? c->base8.as<uint8_t>() : nullptr;
   s.pool = c->buf<Ent>("pool", (size_t)n * p.L, &e);
   s.psz = c->buf<uint32_t>("psz", n, &e);
   s.M = c->buf<uint32_t>("M", n, &e);
@@ -1037,24 +1347,47 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
   unsigned long long *pairs = (unsigned long long *)c->buf<uint64_t>("pairs", 2, &e);
   WV_CUDA(c, e);
 
-  // offer buffers: the largest chunk holds at most `cap` offers
-  size_t free_b = 0, total_b = 0;
-  WV_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
-  const size_t rec_bytes = 4 + 8 + 4 + 4 + sizeof(Grouped);
-  uint32_t cap = (uint32_t)std::min<size_t>((size_t)1 << 28, std::max<size_t>(free_b / 3 / rec_bytes, 1u << 20));
-  // WV_NND_OFFER_CAP lowers the per-chunk offer capacity (more, smaller
-  // join chunks); results do not depend on it
-  if (const char *env = getenv("WV_NND_OFFER_CAP")) cap = std::max<uint32_t>(1024u, std::min<uint32_t>(cap, (uint32_t)atol(env)));
-  Offers of{};
-  of.tgt = c->buf<uint32_t>("of_t", cap, &e);
-  of.key = c->buf<unsigned long long>("of_k", cap, &e);
-  of.cand = c->buf<uint32_t>("of_c", cap, &e);
-  of.dist = c->buf<float>("of_d", cap, &e);
-  Grouped *grp = c->buf<Grouped>("of_g", cap, &e);
+  // The entry buffers hold a whole join's offers: they start at 64 per node
+  // and grow to what a join asks for while the device has room for twice
+  // that; otherwise (or with WV_NND_OFFER_CAP, which caps them) the join runs
+  // in chunks of nodes in node order whose offers' upper bound fits.  Results
+  // do not depend on it.
+  uint64_t cap_max = ~0ull;
+  if (const char *env = getenv("WV_NND_OFFER_CAP")) cap_max = std::max<uint64_t>(1024u, (uint64_t)atol(env));
+  uint64_t cap = 0;
+  JoinOut jo{};
+  auto room = [&](uint64_t want) -> int {  // entry buffers for `want` offers (0: as many as there is memory for)
+    want = std::min<uint64_t>(want, std::min<uint64_t>(cap_max, 0xfffffff0ull));
+    if (want <= cap) return WV_OK;
+    size_t free_b = 0, total_b = 0;
+    WV_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    const uint64_t have = free_b + c->work["of_e"].bytes + c->work["of_q"].bytes;
+    want = std::min<uint64_t>(want, std::max<uint64_t>(have / 2 / 10, 1u << 20));
+    if (want <= cap) return WV_OK;
+    cudaError_t e2 = cudaSuccess;
+    jo.ent = c->buf<uint2>("of_e", want, &e2);
+    jo.eq = c->buf<uint16_t>("of_q", want, &e2);
+    WV_CUDA(c, e2);
+    cap = std::min<uint64_t>(c->work["of_e"].bytes / sizeof(uint2), c->work["of_q"].bytes / sizeof(uint16_t));
+    cap = std::min<uint64_t>(cap, std::min<uint64_t>(cap_max, 0xfffffff0ull));
+    jo.cap = cap;
+    return WV_OK;
+  };
+  {
+    const int rc = room((uint64_t)n * 64);
+    if (rc) return rc;
+  }
+  jo.cursor = reinterpret_cast<unsigned long long *>(small);
+  jo.toff = toff;
+  jo.tcur = tcur;
+  float *pmax = c->buf<float>("pmax", n, &e);
+  Redo redo{};
+  redo.cnt = small + 2;
+  redo.list[0] = act;
+  redo.list[1] = big;
+  redo.list[2] = c->buf<uint32_t>("act2", n, &e);
   WV_CUDA(c, e);
-  of.cap = cap;
-  of.tcnt = tcnt;
-  of.cursor = small + 3;
+  jo.mx = pmax;
 
   cudaEvent_t ev0, ev1;
   cudaEventCreate(&ev0);
@@ -1089,83 +1422,191 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
                                                           c->fg_deg.as<uint32_t>(), c->fg_w, p.efanna ? 1 : 0);
   WV_CUDA(c, cudaGetLastError());
 
-  // the local join's pair distances: on the tensor cores where they are exact
-  // (integer data, d a multiple of 16 up to 128, new lists of at most 128
-  // ids; WV_NND_JOIN=fp32 keeps the FP32 pair kernel), else in FP32 in the
-  // reference's order.  Both give the same offers.
+  // the local join's pair distances: from the byte rows on the tensor cores
+  // for integer data with d a multiple of 16 up to 256 (WV_NND_JOIN=fp32
+  // keeps the FP32 kernel), else in FP32 in the reference's order.  Both give
+  // the same offers.
   const char *join_env = getenv("WV_NND_JOIN");
-  const bool join_tc = c->base_int && c->d % 16 == 0 && c->d <= 128 && s.capn <= JT_ROWS &&
-                       !(join_env && std::string(join_env) == "fp32");
-  const size_t jtc_smem = join_tc_smem(c->d, s.capn, s.capo);
-  if (join_tc) WV_CUDA(c, cudaFuncSetAttribute(k_join_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jtc_smem));
-  const uint32_t stride = ((c->d + 3) & ~3u) + 4;
-  uint32_t tjc = J_TJ;
-  while (tjc > 32 && (size_t)(J_TI + tjc) * stride * 4 > 200 * 1024) tjc -= 32;
-  const size_t join_smem = (size_t)(J_TI + tjc) * stride * 4 + (size_t)(s.capn + s.capo) * 4 + 16;
-  WV_CHECK(c, join_smem <= 227 * 1024, WV_ERR_LIMIT, "dimension %u too large for the local-join tile", c->d);
-  WV_CUDA(c, cudaFuncSetAttribute(k_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)join_smem));
+  const bool join_i8 = c->base_int && s.base8 && !(join_env && std::string(join_env) == "fp32");
+  const uint32_t capt = s.capn + s.capo;
+  JoinCfg jc{};
+  jc.tj = J_TJ;
+  jc.gcap = J_GCAP;
+  // shared memory: the rows, then the tile and the node's lists as far as
+  // they fit (else they live in global memory, a slab per block)
+  const uint32_t fstride = ((c->d + 3) & ~3u) + 4;
+  if (!join_i8)
+    while (jc.tj > 32 && (size_t)(J_TI + jc.tj) * fstride * 4 > 200 * 1024) jc.tj -= 32;
+  size_t join_smem = join_i8 ? (size_t)JI_ROWS * ji_stride(c->d) : (size_t)(J_TI + jc.tj) * fstride * 4;
+  const size_t lists = (size_t)capt * 16;
+  const bool lists_smem = join_smem + lists <= 200 * 1024;
+  if (lists_smem) join_smem += lists;
+  if (join_smem + (size_t)jc.gcap * 4 <= 220 * 1024) join_smem += (size_t)jc.gcap * 4;
+  else jc.gcap = 0;
+  WV_CHECK(c, join_smem + 16 <= 227 * 1024, WV_ERR_LIMIT, "dimension %u too large for the local-join tile", c->d);
+  int jper = 0;
+  if (join_i8) {
+    WV_CUDA(c, cudaFuncSetAttribute(k_join<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)join_smem));
+    WV_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&jper, k_join<true>, JI_THREADS, join_smem));
+  } else {
+    WV_CUDA(c, cudaFuncSetAttribute(k_join<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)join_smem));
+    WV_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&jper, k_join<false>, J_THREADS, join_smem));
+  }
+  WV_CHECK(c, jper > 0, WV_ERR_LIMIT, "the local join does not fit the device (d=%u)", c->d);
+  const uint32_t jgrid = (uint32_t)(c->sms * jper);
+  if (!lists_smem) jc.lscr = c->buf<uint32_t>("join_l", (size_t)jgrid * 4 * capt, &e);
+  WV_CUDA(c, e);
+  const size_t af_smem = AF_WARPS * af_warp_words(p.L) * 4;
+  WV_CUDA(c, cudaFuncSetAttribute(k_apply_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)af_smem));
   const size_t apw_smem = (size_t)AP_WARPS * AP_WARP_CAP * sizeof(Grouped) + (size_t)AP_WARPS * (p.L + 1) * sizeof(Ent);
-  WV_CUDA(c, cudaFuncSetAttribute(k_apply_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)apw_smem));
-  const size_t apb_smem = (size_t)AP_BIG_CAP * sizeof(Grouped) + (size_t)(p.L + 1) * sizeof(Ent);
-  WV_CUDA(c, cudaFuncSetAttribute(k_apply_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)apb_smem));
+  WV_CUDA(c, cudaFuncSetAttribute(k_replay_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)apw_smem));
+  const size_t apb_pool = ((size_t)(p.L + 2) & ~size_t(1)) * sizeof(Ent);
+  const size_t apb_smem = (size_t)AP_BIG_CAP * sizeof(Grouped) + apb_pool;
+  WV_CUDA(c, cudaFuncSetAttribute(k_replay_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)apb_smem));
   WV_CUDA(c, cudaMemsetAsync(pairs, 0, 8, c->stream));
 
-  std::vector<uint32_t> h_lnew(n), h_lold(n);
+  // the init rows' distances must be those of their ids for the order-free
+  // application of the offers (k_apply_fast)
+  bool dist_ok = true;
+  {
+    int *ok = reinterpret_cast<int *>(usmall + 4);
+    WV_CUDA(c, cudaMemsetAsync(ok, 1, 4, c->stream));
+    k_check_rows<<<c->sms * 8, 256, 0, c->stream>>>(s, c->fg_ids.as<uint32_t>(), c->fg_dist.as<float>(),
+                                                    c->fg_deg.as<uint32_t>(), c->fg_w, ok);
+    WV_CUDA(c, cudaGetLastError());
+    int h = 0;
+    WV_CUDA(c, cudaMemcpyAsync(&h, ok, 4, cudaMemcpyDeviceToHost, c->stream));
+    WV_CUDA(c, cudaStreamSynchronize(c->stream));
+    dist_ok = h != 0;
+  }
+
+  // one join over nodes [n0, n1); `whole`: all nodes at once.  Returns with
+  // *need > cap (and nothing applied) when the entries did not fit.
+  struct {
+    unsigned long long cursor;
+    uint32_t redo[4];
+  } hs;
+  auto join = [&](uint32_t n0, uint32_t n1, bool whole, const uint32_t *mclr) -> int {
+    WV_CUDA(c, cudaMemsetAsync(tcnt, 0, (size_t)n * 4, c->stream));
+    const int ob = (int)std::min<uint32_t>((n1 - n0 + 7) / 8, (uint32_t)c->sms * 16);
+    unsigned long long *gmax = reinterpret_cast<unsigned long long *>(small) + 4, hg = 0;
+    WV_CUDA(c, cudaMemsetAsync(small, 0, 48, c->stream));
+    k_occ_count<<<ob, 256, 0, c->stream>>>(s, n0, n1, tcnt, gmax);
+    WV_CUDA(c, exclusive_scan_u32(tcnt, toff, n, scan_tmp, c->stream));
+    uint32_t tl[2];
+    WV_CUDA(c, cudaMemcpyAsync(&tl[0], toff + n - 1, 4, cudaMemcpyDeviceToHost, c->stream));
+    WV_CUDA(c, cudaMemcpyAsync(&tl[1], tcnt + n - 1, 4, cudaMemcpyDeviceToHost, c->stream));
+    WV_CUDA(c, cudaMemsetAsync(tcur, 0, (size_t)n * 4, c->stream));
+    WV_CUDA(c, cudaMemcpyAsync(&hg, gmax, 8, cudaMemcpyDeviceToHost, c->stream));
+    k_pool_max<<<nb, NODE_THREADS, 0, c->stream>>>(s, pmax);
+    WV_CUDA(c, cudaGetLastError());
+    WV_CUDA(c, cudaStreamSynchronize(c->stream));
+    cudaError_t e2 = cudaSuccess;  // (of the buffers sized below)
+    jo.desc = c->buf<uint4>("of_d", (size_t)tl[0] + tl[1] + 1, &e2);
+    WV_CUDA(c, e2);
+    uint32_t grid = std::min(jgrid, n1 - n0);
+    if (jc.gcap == 0) hg = std::max<unsigned long long>(hg, J_GCAP);
+    if (hg > jc.gcap) {  // some tiles live in global memory
+      size_t free_b = 0, total_b = 0;
+      WV_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+      jc.gslab = (size_t)hg;
+      grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(grid, (free_b + c->work["join_g"].bytes) / 4 / (hg * 4)));
+      jc.gscr = c->buf<float>("join_g", (size_t)grid * jc.gslab, &e2);
+      WV_CUDA(c, e2);
+    }
+    if (join_i8) k_join<true><<<grid, JI_THREADS, join_smem, c->stream>>>(s, n0, n1, jo, jc, pairs + 1);
+    else k_join<false><<<grid, J_THREADS, join_smem, c->stream>>>(s, n0, n1, jo, jc, pairs + 1);
+    WV_CUDA(c, cudaGetLastError());
+    if (whole && dist_ok)
+      k_apply_fast<<<(int)std::min<uint32_t>((n + AF_WARPS - 1) / AF_WARPS, (uint32_t)c->sms * 16), AF_WARPS * 32,
+                     af_smem, c->stream>>>(s, s.pre, mclr, jo, redo);
+    else
+      k_redo_all<<<nb, NODE_THREADS, 0, c->stream>>>(n, jo, redo);
+    k_replay_warp<<<c->sms * 3, AP_WARPS * 32, apw_smem, c->stream>>>(s, jo, redo);
+    k_replay_block<<<c->sms, AB_THREADS, apb_smem, c->stream>>>(s, jo, redo, nullptr, 0);
+    WV_CUDA(c, cudaGetLastError());
+    WV_CUDA(c, cudaMemcpyAsync(&hs, small, sizeof(hs), cudaMemcpyDeviceToHost, c->stream));
+    WV_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (hs.redo[2]) {  // targets whose offers exceed shared memory
+      uint32_t P = 1;
+      while (P < hs.redo[3]) P <<= 1;
+      const uint32_t blocks = std::min<uint32_t>(hs.redo[2], (uint32_t)c->sms);
+      Grouped *gk = c->buf<Grouped>("of_g", (size_t)blocks * P, &e2);
+      WV_CUDA(c, e2);
+      k_replay_block<<<blocks, AB_THREADS, apb_pool, c->stream>>>(s, jo, redo, gk, P);
+      WV_CUDA(c, cudaGetLastError());
+    }
+    return WV_OK;
+  };
+  // the pairs of a retried join count once
+  auto take_pairs = [&](bool keep) -> int {
+    unsigned long long h = 0;
+    if (keep) {
+      WV_CUDA(c, cudaMemcpyAsync(&h, pairs + 1, 8, cudaMemcpyDeviceToHost, c->stream));
+      WV_CUDA(c, cudaStreamSynchronize(c->stream));
+      S.pairs += h;
+    }
+    WV_CUDA(c, cudaMemsetAsync(pairs + 1, 0, 8, c->stream));
+    return WV_OK;
+  };
+  {
+    const int rc = take_pairs(false);
+    if (rc) return rc;
+  }
+  bool chunked = false;  // joins no longer fit in one piece
   for (uint32_t it = 0; it < p.ITER; it++) {
     // ------------------------------------------------------------ join
     // (NN_DESCENT's first join pairs 2S zero ids -- nothing; EFANNA's is live)
     if (it > 0 || p.efanna) {
       cudaEventRecord(ev0, c->stream);
-      WV_CUDA(c, cudaMemcpyAsync(h_lnew.data(), s.lnew, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
-      WV_CUDA(c, cudaMemcpyAsync(h_lold.data(), s.lold, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
-      WV_CUDA(c, cudaStreamSynchronize(c->stream));
-      uint32_t n0 = 0;
-      while (n0 < n) {
-        // chunk: the most nodes whose offer upper bound fits `cap`
-        uint64_t acc = 0;
-        uint32_t n1 = n0;
-        while (n1 < n) {
-          uint64_t a = h_lnew[n1], b = h_lold[n1];
-          uint64_t ub = a * (a - (a > 0)) + 2 * a * b;  // 2 offers per pair
-          if (n1 > n0 && acc + ub > cap) break;
-          acc += ub;
-          n1++;
-        }
-        WV_CHECK(c, acc <= cap, WV_ERR_LIMIT, "node %u alone may produce %llu offers (> %u)", n0,
-                 (unsigned long long)acc, cap);
-        while (true) {
-          WV_CUDA(c, cudaMemsetAsync(tcnt, 0, (size_t)n * 4, c->stream));
-          WV_CUDA(c, cudaMemsetAsync(small, 0, 16, c->stream));
-          if (join_tc)
-            k_join_tc<<<n1 - n0, JT_THREADS, jtc_smem, c->stream>>>(s, n0, of, pairs, c->d_status());
-          else
-            k_join<<<n1 - n0, J_THREADS, join_smem, c->stream>>>(s, n0, of, pairs, c->d_status(), tjc);
-          WV_CUDA(c, cudaGetLastError());
-          k_active<<<nb, NODE_THREADS, 0, c->stream>>>(n, tcnt, act, small, big, small + 1, AP_WARP_CAP, small + 2);
-          uint32_t hs[4];
-          WV_CUDA(c, cudaMemcpyAsync(hs, small, 16, cudaMemcpyDeviceToHost, c->stream));
-          WV_CUDA(c, cudaStreamSynchronize(c->stream));
-          if (hs[2] > AP_BIG_CAP && n1 - n0 > 1) {
-            n1 = n0 + (n1 - n0) / 2;  // a target gets too many offers: smaller chunk
-            continue;
-          }
-          WV_CHECK(c, hs[2] <= AP_BIG_CAP, WV_ERR_LIMIT, "one node sends %u offers to one target", hs[2]);
-          const uint32_t count = hs[3];
-          S.offers += count;
+      const uint32_t *mclr = it > 0 ? s.M : nullptr;
+      bool done = false;
+      while (!chunked && !done) {
+        int rc = join(0, n, true, mclr);
+        if (rc) return rc;
+        if (hs.cursor <= cap) {
+          done = true;
+          S.offers += hs.cursor;
           S.chunks++;
-          WV_CUDA(c, exclusive_scan_u32(tcnt, toff, n, scan_tmp, c->stream));
-          WV_CUDA(c, cudaMemsetAsync(tcur, 0, (size_t)n * 4, c->stream));
-          if (count) {
-            k_group<<<(count + 255) / 256, 256, 0, c->stream>>>(count, of, toff, tcur, grp);
-            if (hs[0])
-              k_apply_warp<<<(hs[0] + AP_WARPS - 1) / AP_WARPS, AP_WARPS * 32, apw_smem, c->stream>>>(
-                  s, act, small, toff, tcnt, grp);
-            if (hs[1]) k_apply_block<<<hs[1], 512, apb_smem, c->stream>>>(s, big, toff, tcnt, grp);
-            WV_CUDA(c, cudaGetLastError());
-          }
+          rc = take_pairs(true);
+          if (rc) return rc;
           break;
         }
-        n0 = n1;
+        rc = take_pairs(false);
+        if (rc) return rc;
+        const uint64_t old = cap;
+        rc = room(hs.cursor + hs.cursor / 8);
+        if (rc) return rc;
+        if (cap < hs.cursor || cap == old) chunked = true;
+      }
+      if (!done) {
+        std::vector<uint32_t> h_lnew(n), h_lold(n);
+        WV_CUDA(c, cudaMemcpyAsync(h_lnew.data(), s.lnew, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
+        WV_CUDA(c, cudaMemcpyAsync(h_lold.data(), s.lold, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
+        WV_CUDA(c, cudaStreamSynchronize(c->stream));
+        uint32_t n0 = 0;
+        while (n0 < n) {
+          // chunk: the most nodes whose offer upper bound fits `cap`
+          uint64_t acc = 0;
+          uint32_t n1 = n0;
+          while (n1 < n) {
+            const uint64_t a = h_lnew[n1], b = h_lold[n1];
+            const uint64_t ub = a * (a - (a > 0)) + 2 * a * b;  // 2 offers per pair
+            if (n1 > n0 && acc + ub > cap) break;
+            acc += ub;
+            n1++;
+          }
+          WV_CHECK(c, acc <= cap, WV_ERR_LIMIT, "node %u alone may produce %llu offers (> %llu)", n0,
+                   (unsigned long long)acc, (unsigned long long)cap);
+          int rc = join(n0, n1, false, nullptr);
+          if (rc) return rc;
+          WV_CHECK(c, hs.cursor <= cap, WV_ERR_STATE, "a join chunk produced more offers than its bound");
+          S.offers += hs.cursor;
+          S.chunks++;
+          rc = take_pairs(true);
+          if (rc) return rc;
+          n0 = n1;
+        }
       }
       cudaEventRecord(ev1, c->stream);
       cudaEventSynchronize(ev1);
@@ -1238,10 +1679,7 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
   k_nnd_final<<<nb, NODE_THREADS, node_smem, c->stream>>>(s, c->fg_ids.as<uint32_t>(), c->fg_dist.as<float>(),
                                                            c->fg_deg.as<uint32_t>());
   WV_CUDA(c, cudaGetLastError());
-  unsigned long long hp = 0;
-  WV_CUDA(c, cudaMemcpyAsync(&hp, pairs, 8, cudaMemcpyDeviceToHost, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
-  S.pairs = hp;
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
   c->fg_w = p.K;

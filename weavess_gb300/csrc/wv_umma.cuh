@@ -1,8 +1,7 @@
 // Helpers for kernels that drive Blackwell's 5th-generation tensor cores
 // (tcgen05) directly: shared-memory matrix and instruction descriptors for
 // BF16 operands in the canonical no-swizzle K-major layout, and bounded
-// mbarrier waits.  Used by the MLP GEMM (wv_umma.cu) and the local join's
-// Gram tiles (wv_nnd.cu).
+// mbarrier waits.  Used by the MLP GEMM (wv_umma.cu).
 #pragma once
 #include <cstdint>
 
