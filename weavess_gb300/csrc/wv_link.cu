@@ -17,12 +17,10 @@
 // Plain form, bit-exact with the single-threaded reference:
 //  * candidates: the beam kernel in build mode (seeds flagged, every visit
 //    recorded in order), seeds drawn on the host in node order;
-//  * prune: one warp per node sorts the visit pool with the warp replica of
-//    std::sort, then picks in pool order 32 candidates at a time: each lane
-//    tests its candidate against the rows picked before the batch, and a
-//    bitmask records which earlier batch members would occlude it, so the
-//    sequential pick/skip walk over the batch needs no further distances.
-//    VAMANA refills from the skipped items through libstdc++'s heap steps;
+//  * prune: a block per node sorts the visit pool by (distance, id) and walks
+//    it 128 candidates at a time; nodes where the order of equal distances
+//    could matter are redone in the order of std::sort (warp_sort.cuh).
+//    VAMANA refills from the skipped items as libstdc++'s heap pops them;
 //  * InterInsert: sequentially, node n walks its current row and inserts
 //    itself into each neighbour's row (dedup, append, or re-prune).  Node n's
 //    row at that moment is its pruned row plus the insertions from nodes < n
@@ -34,12 +32,11 @@
 //    insertions from higher ids, read from their snapshots.  Each warp keeps
 //    the vectors' pairwise distances of its row in shared memory, so an
 //    insertion costs one new distance column.
-#include <cuda_bf16.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "warp_sort.cuh"
@@ -53,7 +50,6 @@
 namespace wv {
 namespace {
 
-constexpr int PR_WARPS = 4;
 constexpr uint32_t LINK_MAX_R = 63;  // row slots (R + 1) index a 64-bit mask
 
 // exact-order squared L2 of two base rows, read from global memory by one lane
@@ -91,9 +87,9 @@ struct PruneArgs {
   const uint32_t *g_deg;
   uint32_t gw;
   int clean;            // Vamana: a short pool is sorted too (clean mode)
-  const float *xnorm;   // integer data, d % 32 == 0, d <= 128, R <= 32: the Gram-tile variant's row norms
-  int *gscr;            // per warp: 2 * vcap + 256 ints
-  HeapItem *hscr;       // per warp: vcap items (VAMANA refill)
+  const float *xnorm;   // integer rows: their squared norms
+  int *gscr;            // per block: 2 * vcap + 256 ints (EXACT, pools beyond shared memory)
+  HeapItem *hscr;       // per block: vcap items (EXACT VAMANA refill)
   uint32_t *out_ids;    // rows of width R, indexed by node
   float *out_dist;
   uint32_t *out_deg;
@@ -112,261 +108,557 @@ __device__ __forceinline__ bool ssg_occludes(float pd, float rd, float djk, floa
   return cos_ij > threshold;
 }
 
-// ---- pair distances of a prune batch as Gram tiles (integer data)
-// On integer data in [0, 255] with d a multiple of 32 up to 128, the exact
-// distance of rows x, y equals |x|^2 + |y|^2 - 2 x.y computed in FP32 (every
-// value an integer below 2^24), and x.y comes from BF16 tensor-core tiles
-// (integers up to 255 are exact in BF16).  Per warp, shared memory holds the
-// rows picked so far and the batch's 32 candidate rows as BF16 (row stride
-// an odd multiple of 64 bytes: the fragment loads are free of bank
-// conflicts), and the two tiles candidate x picked and candidate x candidate.
-constexpr uint32_t PT_ROWS = 32;  // rows picked (R <= 32) and candidates per batch
+// ---- the prune with a block per node
+// The walk over a node's sorted pool needs its order only where distances
+// differ: the pool is sorted by (distance, id), and a node where equal
+// distances could have come out in another order is left to k_prune, which
+// sorts as std::sort does -- two picks of equal distance, a candidate
+// occluded by a pick of its own distance, equal distances on both sides of
+// the examination bound, or among the entries a Vamana refill takes.  Pools
+// of more than 1,024 entries are sorted a window at a time, as far as the
+// walk gets.  A
+// candidate is tested against the picks until one occludes it: a warp takes
+// 32 candidates, drops the occluded ones after each test and, once 16 (8) are
+// left, tests them against two (four) picks at a time; the survivors of the
+// block's four warps are then picked in order, each pick tested against the
+// rest.  On integer data the rows are bytes and the distances exact integers
+// (__dp4a), else FP32 sums in the reference's order.
+//
+// What bounds it: latency of the short phases and barriers; a block's rows,
+// picks and sort keys take 34 KB (d = 128 bytes), so 6 nodes per SM are in
+// flight.  A warp per node with every pool sorted by the introsort replica in
+// global memory and all pairs of a batch as Gram tiles (29 KB per warp, 4
+// warps per SM) took 193 ms for the NSG prune of 200k x 128 nodes; this takes
+// 17 ms and the EXACT redo 2.8 ms.  Two real-valued Vamana prunes of 20k x 96
+// (pools of 1,800 and 4,400): 33 ms -> 13.3 ms.
+constexpr int PF_THREADS = 128, PF_NW = PF_THREADS / 32, PF_SIZES = 4;
+// pool sizes of the launches
+__host__ __device__ constexpr uint32_t pf_keys(int l) { return 1024u << l; }
 
-__host__ __device__ inline uint32_t pt_stride(uint32_t d) { return (d * 2) % 128 == 64 ? d * 2 : d * 2 + 64; }
-__host__ __device__ inline size_t pt_warp_bytes(uint32_t d) {
-  return 2 * (size_t)PT_ROWS * pt_stride(d) + 2 * (size_t)PT_ROWS * PT_ROWS * 4 + PT_ROWS * 4;
+struct PruneFast {
+  const uint8_t *base8;   // byte rows (I8)
+  uint32_t keys;          // longest pool this launch takes (a pf_keys value)
+  uint32_t cs;            // bytes of a row in shared memory (0: rows read where they lie)
+  const uint32_t *list, *nlist;  // the pools (null: all)
+  uint32_t *more, *nmore;  // longer pools, for the next launch (null: to redo)
+  uint32_t *redo, *nredo;  // pools for the EXACT launch
+};
+
+constexpr uint32_t PF_WINDOW = 1024;  // keys sorted at a time
+constexpr uint32_t PF_SAVED = 128;    // skipped keys of the first window kept for the Vamana refill
+__host__ __device__ inline size_t pf_smem(uint32_t keys, uint32_t cs, uint32_t R, bool exact) {
+  return (size_t)keys * 8 + (keys > PF_WINDOW && !exact ? PF_WINDOW * 8 : 0) + PF_WINDOW / 8 + PF_SAVED * 8 +
+         (size_t)cs * (32 * PF_NW + R + 1) + (exact ? (2 * (size_t)keys + 256) * 4 : 0);
 }
 
-__device__ __forceinline__ uint32_t pt_pack(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t *>(&v);
-}
-
-// row `id` of the FP32 base into slot `r` of a BF16 row area (16 lanes per row)
-__device__ __forceinline__ void pt_stage_row(uint8_t *area, uint32_t stride, uint32_t r, const float *base,
-                                             uint32_t d, uint32_t id, int sub) {
-  for (uint32_t k = (uint32_t)sub * 8; k < d; k += 16 * 8) {
-    const float4 *src = reinterpret_cast<const float4 *>(base + (size_t)id * d + k);
-    const float4 x0 = __ldg(src), x1 = __ldg(src + 1);
-    *reinterpret_cast<uint4 *>(area + (size_t)r * stride + k * 2) =
-        make_uint4(pt_pack(x0.x, x0.y), pt_pack(x0.z, x0.w), pt_pack(x1.x, x1.y), pt_pack(x1.z, x1.w));
-  }
-}
-
-__device__ __forceinline__ void pt_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                       uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// G[x][y] = X_x . Y_y for the 32 rows of X and the first ncol (a multiple of
-// 8, <= 32) rows of Y; lane (g, j) loads dimensions 32t + 8j .. +7 of its
-// rows (the dot product's terms permuted alike in A and B)
-__device__ void pt_gram(const uint8_t *X, const uint8_t *Y, uint32_t stride, uint32_t d, uint32_t ncol, float *G,
-                        int lane) {
-  const int g = lane >> 2, j = lane & 3;
-  const uint32_t T = d / 32;
-  for (int gi = 0; gi < 2; gi++) {
-    for (uint32_t nt = 0; nt * 8 < ncol; nt++) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      for (uint32_t t = 0; t < T; t++) {
-        const uint32_t off = (32 * t + 8 * j) * 2;
-        const uint4 a0 = *reinterpret_cast<const uint4 *>(X + (size_t)(16 * gi + g) * stride + off);
-        const uint4 a1 = *reinterpret_cast<const uint4 *>(X + (size_t)(16 * gi + g + 8) * stride + off);
-        const uint4 b = *reinterpret_cast<const uint4 *>(Y + (size_t)(8 * nt + g) * stride + off);
-        pt_mma(acc, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
-        pt_mma(acc, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
+template <int E>
+__device__ __noinline__ void pf_sort(unsigned long long *K) {
+  constexpr int N = PF_THREADS * E;
+  const int tid = threadIdx.x;
+  unsigned long long v[E];
+#pragma unroll
+  for (int e = 0; e < E; e++) v[e] = K[e * PF_THREADS + tid];  // (any assignment: the sort starts here)
+  auto cx = [](unsigned long long &a, unsigned long long &b, bool up) {
+    const unsigned long long lo = a < b ? a : b, hi = a < b ? b : a;
+    a = up ? lo : hi;
+    b = up ? hi : lo;
+  };
+  // element tid * E + e in v[e]; sizes up to E inside a thread
+#pragma unroll
+  for (int k = 2; k <= E; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int e = 0; e < E; e++)
+        if ((e & j) == 0) cx(v[e], v[e | j], k < E ? (e & k) == 0 : (tid & 1) == 0);
+  for (int k = 2 * E; k <= N; k <<= 1) {
+    const bool up = ((tid * E) & k) == 0;
+    for (int j = k >> 1; j >= E; j >>= 1) {
+      const int tm = j / E;
+      const bool keep_lo = ((tid & tm) == 0) == up;
+      if (tm >= 32) {
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < E; e++) K[e * PF_THREADS + tid] = v[e];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+          const unsigned long long o = K[e * PF_THREADS + (tid ^ tm)];
+          v[e] = keep_lo ? (v[e] < o ? v[e] : o) : (v[e] < o ? o : v[e]);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+          const unsigned long long o = __shfl_xor_sync(FULL, v[e], tm);
+          v[e] = keep_lo ? (v[e] < o ? v[e] : o) : (v[e] < o ? o : v[e]);
+        }
       }
-      // lane (g, j): rows 16 gi + g (c0, c1) and + 8 (c2, c3), columns 8 nt + 2j, + 1
-      float *r0 = G + (size_t)(16 * gi + g) * PT_ROWS + 8 * nt + 2 * j;
-      float *r1 = G + (size_t)(16 * gi + g + 8) * PT_ROWS + 8 * nt + 2 * j;
-      r0[0] = acc[0];
-      r0[1] = acc[1];
-      r1[0] = acc[2];
-      r1[1] = acc[3];
+    }
+#pragma unroll
+    for (int j = E >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int e = 0; e < E; e++)
+        if ((e & j) == 0) cx(v[e], v[e | j], up);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; e++) K[tid * E + e] = v[e];
+  __syncthreads();
+}
+
+// the next keys of a long pool: those above `lo` (the last window's end) up
+// to a distance that PF_WINDOW of them do not exceed, unsorted into W (padded
+// with ~0).  A linear histogram over the remaining keys' distance bits finds
+// it; keys of one distance share a bin, so no window ends between equal
+// distances.  Returns the keys taken (0: a bin alone exceeds the window) and
+// the new bound in lo.  hist: PF_WINDOW words, W itself.
+__device__ __noinline__ uint32_t pf_window(const unsigned long long *U, uint32_t m, unsigned long long *W,
+                                           uint32_t &lo, bool first) {
+  __shared__ uint32_t mn, mx, bin, taken;
+  uint32_t *hist = reinterpret_cast<uint32_t *>(W);
+  const int tid = threadIdx.x;
+  // (distances are below 2^31 as bits; bits >= lo remain)
+  if (tid == 0) {
+    mn = 0xffffffffu;
+    mx = 0;
+    taken = 0;
+    bin = 0;
+  }
+  for (uint32_t i = tid; i < PF_WINDOW; i += PF_THREADS) hist[i] = 0;
+  __syncthreads();
+  const uint32_t from = first ? 0u : lo;
+  uint32_t a = 0xffffffffu, b = 0;
+  for (uint32_t i = tid; i < m; i += PF_THREADS) {
+    const uint32_t d = (uint32_t)(U[i] >> 32);
+    if (d >= from) {
+      a = min(a, d);
+      b = max(b, d);
     }
   }
+  a = __reduce_min_sync(FULL, a);
+  b = __reduce_max_sync(FULL, b);
+  if ((tid & 31) == 0) {
+    atomicMin(&mn, a);
+    atomicMax(&mx, b);
+  }
+  __syncthreads();
+  const uint32_t base = mn;
+  if (base > mx) return 0;  // (nothing left; block-uniform)
+  uint32_t sh = 0;
+  while (((mx - base) >> sh) >= PF_WINDOW) sh++;
+  for (uint32_t i = tid; i < m; i += PF_THREADS) {
+    const uint32_t d = (uint32_t)(U[i] >> 32);
+    if (d >= from) atomicAdd(&hist[(d - base) >> sh], 1u);
+  }
+  __syncthreads();
+  if (tid < 32) {  // bins that fit, from the nearest
+    uint32_t run = 0, nb = 0;
+    for (uint32_t b0 = 0; b0 < PF_WINDOW; b0 += 32) {
+      const uint32_t c = hist[b0 + tid];
+      uint32_t x = c;
+      for (int k = 1; k < 32; k <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, x, k);
+        if (tid >= k) x += y;
+      }
+      const unsigned over = __ballot_sync(FULL, run + x > PF_WINDOW);
+      if (over) {
+        nb = b0 + __ffs(over) - 1;
+        break;
+      }
+      run += __shfl_sync(FULL, x, 31);
+      nb = b0 + 32;
+    }
+    if (tid == 0) bin = nb;
+  }
+  __syncthreads();
+  const uint32_t nb = bin;
+  if (nb == 0) return 0;
+  for (uint32_t i = tid; i < PF_WINDOW; i += PF_THREADS) W[i] = ~0ull;
+  __syncthreads();
+  for (uint32_t i = tid; i < m; i += PF_THREADS) {
+    const unsigned long long k = U[i];
+    const uint32_t d = (uint32_t)(k >> 32);
+    if (d >= from && ((d - base) >> sh) < nb) W[atomicAdd(&taken, 1u)] = k;
+  }
+  __syncthreads();
+  // the first distance of bin nb (past the last bin: above every distance)
+  const unsigned long long next = (unsigned long long)base + ((unsigned long long)nb << sh);
+  lo = next > 0xffffffffull ? 0xffffffffu : (uint32_t)next;
+  return taken;
 }
 
-// MODE: 0 Vamana, 1 NSG, 2 SSG.  TC: the pair distances from Gram tiles
-// (integer data, d a multiple of 32 up to 128, R <= 32; same values)
-template <int MODE, bool TC>
-__global__ void __launch_bounds__(PR_WARPS * 32) k_prune(PruneArgs a) {
-  constexpr bool NSG = MODE != 0;  // the NSG-style walk (SSG shares it with the angle test)
-  __shared__ uint32_t pk_id[PR_WARPS][LINK_MAX_R];
-  __shared__ float pk_d[PR_WARPS][LINK_MAX_R];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t gwarp = blockIdx.x * PR_WARPS + warp, nwarps = gridDim.x * PR_WARPS;
-  int *scr = a.gscr + (size_t)gwarp * (2 * a.vcap + 256);
-  HeapItem *heap = a.hscr + (size_t)gwarp * a.vcap;
-  uint32_t *pid = pk_id[warp];
-  float *pd = pk_d[warp];
-  // TC: per warp, the picked rows, the batch's rows, the two tiles, the
-  // picked rows' norms
-  extern __shared__ __align__(16) uint8_t pt_smem[];
-  const uint32_t pst = pt_stride(a.d);
-  uint8_t *prow = pt_smem + (TC ? (size_t)warp * pt_warp_bytes(a.d) : 0);
-  uint8_t *crow = prow + (size_t)PT_ROWS * pst;
-  float *G1 = reinterpret_cast<float *>(crow + (size_t)PT_ROWS * pst);
-  float *G2 = G1 + PT_ROWS * PT_ROWS;
-  float *pxn = G2 + PT_ROWS * PT_ROWS;
-  for (uint32_t qi = gwarp; qi < a.cnt; qi += nwarps) {
-    const uint32_t node = a.n0 + qi;
+// distance of two rows: bytes (with their squared norms), or FP32 in the
+// reference's order
+template <bool I8>
+__device__ __forceinline__ float pf_dist(const uint8_t *x, const uint8_t *y, uint32_t d, int nx, int ny) {
+  if (I8) {
+    unsigned dot = 0, dot2 = 0;
+    const uint4 *p = reinterpret_cast<const uint4 *>(x), *q = reinterpret_cast<const uint4 *>(y);
+#pragma unroll 4
+    for (uint32_t k = 0; k < d / 16; k++) {
+      const uint4 u = p[k], v = q[k];
+      dot = __dp4a(u.x, v.x, dot);
+      dot2 = __dp4a(u.y, v.y, dot2);
+      dot = __dp4a(u.z, v.z, dot);
+      dot2 = __dp4a(u.w, v.w, dot2);
+    }
+    return (float)(nx + ny - 2 * (int)(dot + dot2));
+  }
+  const float4 *p = reinterpret_cast<const float4 *>(x), *q = reinterpret_cast<const float4 *>(y);
+  float acc = 0.f;
+#pragma unroll 4
+  for (uint32_t k = 0; k < d / 4; k++) acc = __fadd_rn(acc, group4(p[k], q[k]));
+  return acc;
+}
+
+// MODE: 0 Vamana, 1 NSG, 2 SSG.  EXACT: the pools in f.list in std::sort's
+// order (warp_sort.cuh; in shared memory up to f.keys entries, else in place)
+// and the Vamana refill through libstdc++'s heap steps.
+template <int MODE, bool I8, bool EXACT>
+__global__ void __launch_bounds__(PF_THREADS) k_prune_block(PruneArgs a, PruneFast f) {
+  constexpr bool NSG = MODE != 0;
+  extern __shared__ __align__(16) uint8_t pf_sm[];
+  __shared__ float pd[LINK_MAX_R];
+  __shared__ uint32_t pid[LINK_MAX_R];
+  __shared__ int pnrm[LINK_MAX_R];
+  __shared__ uint32_t wl[PF_NW][32], wc[PF_NW];
+  __shared__ int amb;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  // U: the pool's keys; K: the sorted window (U itself when one window holds
+  // every pool)
+  unsigned long long *U = reinterpret_cast<unsigned long long *>(pf_sm);
+  const bool windows = !EXACT && f.keys > PF_WINDOW;
+  unsigned long long *K = windows ? U + f.keys : U;
+  unsigned long long *saved = U + f.keys + (windows ? PF_WINDOW : 0u);
+  uint32_t *gone = reinterpret_cast<uint32_t *>(saved + PF_SAVED);  // picked or dropped, by position in the window
+  uint8_t *cand = reinterpret_cast<uint8_t *>(gone) + PF_WINDOW / 8;  // 32 rows per warp
+  uint8_t *pick = cand + (size_t)f.cs * 32 * PF_NW;                           // R rows
+  uint8_t *self = pick + (size_t)f.cs * a.R;
+  int *scr = reinterpret_cast<int *>(self + f.cs);  // (EXACT)
+  HeapItem *heap = EXACT ? a.hscr + (size_t)blockIdx.x * a.vcap : nullptr;
+  const uint32_t rb = I8 ? a.d : a.d * 4, d = a.d;
+  const uint8_t *rows = I8 ? f.base8 : reinterpret_cast<const uint8_t *>(a.base);
+  const bool cv = !NSG && a.clean;
+  const uint32_t count = f.nlist ? *f.nlist : a.cnt;
+  auto occludes = [&](float cd, float qd, float dd) {
+    return MODE == 2 ? ssg_occludes(cd, qd, dd, a.threshold) : (NSG ? (dd < cd) : (__fmul_rn(a.alpha, dd) < cd));
+  };
+  for (uint32_t it = blockIdx.x; it < count; it += gridDim.x) {
+    const uint32_t qi = f.list ? f.list[it] : it, node = a.n0 + qi;
     DI *pool = a.vis + (size_t)qi * a.vcap;
-    uint32_t m = min(a.vcnt[qi], a.vcap);
+    const uint32_t mv = min(a.vcnt[qi], a.vcap);
     uint32_t *oid = a.out_ids + (size_t)node * a.R;
     float *od = a.out_dist + (size_t)node * a.R;
-    // clean Vamana (this library's clean build mode): the pool is the visited
-    // set plus the node's own row, as DiskANN's RobustPrune prunes V u
-    // N_out(p); the node itself and repeated ids are dropped, not skipped
-    const bool cv = !NSG && a.clean;
-    if (NSG || cv) {
-      // the node's own row joins the pool, distances recomputed
-      // (component_prune.cpp:26-34); vcap leaves room for it
-      const uint32_t deg = min(a.g_deg[node], a.gw);
-      for (uint32_t j = lane; j < deg; j += 32) {
-        uint32_t id = a.g_ids[(size_t)node * a.gw + j];
-        if (id >= a.n) {
-          set_err(a.status, DEV_BAD_ID);
-          id = 0;
-        }
-        if (m + j < a.vcap) pool[m + j] = DI{l2g(a.base, a.d, node, id), id};
-      }
-      if (m + deg > a.vcap) set_err(a.status, DEV_OVERFLOW);
-      m = min(m + deg, a.vcap);
-      __syncwarp();
-    }
+    const uint32_t deg = (NSG || cv) ? min(a.g_deg[node], a.gw) : 0u;
+    if (mv + deg > a.vcap && tid == 0) set_err(a.status, DEV_OVERFLOW);
+    const uint32_t m = min(mv + deg, a.vcap);
     if (!NSG && m <= a.R && !a.clean) {  // PruneVAMANA keeps a short pool unsorted
-      for (uint32_t j = lane; j < m; j += 32) {
+      for (uint32_t j = tid; j < m; j += PF_THREADS) {
         oid[j] = pool[j].i;
         od[j] = pool[j].d;
       }
-      if (lane == 0) a.out_deg[node] = m;
+      if (tid == 0) a.out_deg[node] = m;
       continue;
     }
     if (m == 0) {
-      if (lane == 0) a.out_deg[node] = 0;
+      if (tid == 0) a.out_deg[node] = 0;
       continue;
     }
-    warp_std_sort(pool, (int)m, DILess(), WarpSortScratch{scr, scr + a.vcap, scr + 2 * a.vcap,
-                                                          scr + 2 * a.vcap + 192}, lane);
-    uint32_t np = 0;   // picked
-    uint32_t ex = 0;   // next pool index to examine
-    uint32_t end = m;  // examination bound
-    uint32_t nskip = 0;
+    if (!EXACT && m > f.keys) {
+      if (tid == 0) {
+        if (f.more) f.more[atomicAdd(f.nmore, 1u)] = qi;
+        else f.redo[atomicAdd(f.nredo, 1u)] = qi;
+      }
+      continue;
+    }
+    __syncthreads();  // the previous node's shared memory is done with
+    if (tid == 0) amb = 0;
+    const uint8_t *srow = rows + (size_t)node * rb;
+    if (f.cs && deg) {
+      for (uint32_t k = tid; k < rb / 16; k += PF_THREADS)
+        reinterpret_cast<uint4 *>(self)[k] = __ldg(reinterpret_cast<const uint4 *>(srow) + k);
+      srow = self;
+    }
+    DI *P = m <= f.keys ? reinterpret_cast<DI *>(K) : pool;  // (EXACT)
+    const uint32_t N = windows ? m : PF_WINDOW;
+    bool bad = false;
+    if (EXACT) {
+      if (P != pool)
+        for (uint32_t i = tid; i < mv; i += PF_THREADS) P[i] = pool[i];
+    }
+    for (uint32_t i = tid; !EXACT && i < N; i += PF_THREADS) {
+      unsigned long long key = ~0ull;
+      if (i < mv) {
+        const DI x = pool[i];
+        key = ((unsigned long long)__float_as_uint(x.d) << 32) | x.i;
+        bad |= __float_as_uint(x.d) > 0x7f800000u;  // (negative or NaN: not ordered by its bits)
+      }
+      if (i < mv || i >= m) U[i] = key;
+    }
+    __syncthreads();
+    // the node's own row joins the pool, distances recomputed
+    // (component_prune.cpp:26-34); vcap leaves room for it
+    for (uint32_t j = tid; j < m - mv; j += PF_THREADS) {
+      uint32_t id = a.g_ids[(size_t)node * a.gw + j];
+      if (id >= a.n) {
+        set_err(a.status, DEV_BAD_ID);
+        id = 0;
+      }
+      const float x = pf_dist<I8>(srow, rows + (size_t)id * rb, d, I8 ? (int)__ldg(a.xnorm + node) : 0,
+                                  I8 ? (int)__ldg(a.xnorm + id) : 0);
+      if (EXACT) {
+        P[mv + j] = DI{x, id};
+      } else {
+        U[mv + j] = ((unsigned long long)__float_as_uint(x) << 32) | id;
+        bad |= __float_as_uint(x) > 0x7f800000u;
+      }
+    }
+    if (bad) amb = 1;
+    __syncthreads();
+    if (!EXACT && amb) {  // block-uniform
+      if (tid == 0) f.redo[atomicAdd(f.nredo, 1u)] = qi;
+      continue;
+    }
+    if (EXACT) {
+      if (warp == 0) {
+        int *sc = P != pool ? scr : a.gscr + (size_t)blockIdx.x * (2 * (size_t)a.vcap + 256);
+        const uint32_t cap = P != pool ? f.keys : a.vcap;
+        warp_std_sort(P, (int)m, DILess(), WarpSortScratch{sc, sc + cap, sc + 2 * cap, sc + 2 * cap + 192}, lane);
+      }
+      __syncthreads();
+    }
+    // the window [w0g, w0g + wn) of the sorted pool in K
+    uint32_t wn = m, wlo = 0;
+    if (!EXACT) {
+      if (windows) {
+        wn = pf_window(U, m, K, wlo, true);
+        if (wn == 0) {  // block-uniform
+          if (tid == 0) f.redo[atomicAdd(f.nredo, 1u)] = qi;
+          continue;
+        }
+      }
+      pf_sort<PF_WINDOW / PF_THREADS>(K);
+    }
+    auto kd = [&](uint32_t i) { return EXACT ? P[i].d : __uint_as_float((uint32_t)(K[i] >> 32)); };
+    auto ki = [&](uint32_t i) { return EXACT ? P[i].i : (uint32_t)K[i]; };
+    // row of sorted entry i into the pick area (a warp)
+    auto put_pick = [&](uint32_t slot, const uint8_t *src) {
+      for (uint32_t k = lane; k < rb / 16; k += 32)
+        reinterpret_cast<uint4 *>(pick + (size_t)slot * f.cs)[k] = reinterpret_cast<const uint4 *>(src)[k];
+    };
+    uint32_t np = 0, ex = 0, end = m, nskip = 0;
     if (NSG) {
       // start skips the node itself at position 0; pool[start] is taken as is
-      uint32_t start = pool[0].i == node ? 1u : 0u;
-      if (start >= m) {
-        if (lane == 0) a.out_deg[node] = 0;
+      const uint32_t start = ki(0) == node ? 1u : 0u;
+      if (start >= wn) {
+        if (tid == 0) {
+          if (start >= m) a.out_deg[node] = 0;
+          else f.redo[atomicAdd(f.nredo, 1u)] = qi;  // (the first window ends before it)
+        }
         continue;
       }
-      if (lane == 0) {
-        pid[0] = pool[start].i;
-        pd[0] = pool[start].d;
+      if (tid == 0) {
+        if (start)
+          for (uint32_t i = 1; i < wn && kd(i) == kd(0); i++)
+            if (ki(i) != node) amb = 1;  // whether the node comes first depends on the sort
+        if (a.R == 1 && start + 1 < wn && kd(start + 1) == kd(start)) amb = 1;
+        pid[0] = ki(start);
+        pd[0] = kd(start);
+        if (I8) pnrm[0] = (int)__ldg(a.xnorm + ki(start));
       }
+      if (f.cs && warp == 0) put_pick(0, rows + (size_t)ki(start) * rb);
       np = 1;
       ex = start + 1;
       end = MODE == 2 ? m : min(m, a.maxc);  // SSG examines the whole pool
-      __syncwarp();
-      if (TC) {
-        const uint32_t id0 = pid[0];
-        if (lane < 16) pt_stage_row(prow, pst, 0, a.base, a.d, id0, lane);
-        if (lane == 0) pxn[0] = __ldg(a.xnorm + id0);
-        __syncwarp();
-      }
     }
+    __syncthreads();
     bool done = np >= a.R;
-    while (!done && ex < end) {
-      const uint32_t cnt = min(32u, end - ex);
-      DI cand = lane < (int)cnt ? pool[ex + lane] : DI{0.f, 0u};
-      float cxn = 0.f;
-      if (TC) {
-        // the batch's rows (rows past cnt: row 0 of the base, never read) and
-        // the tiles candidate x picked-before-the-batch, candidate x candidate
-        for (uint32_t r = lane >> 4; r < PT_ROWS; r += 2) {
-          const uint32_t id = __shfl_sync(0xffffffffu, cand.i, r);
-          pt_stage_row(crow, pst, r, a.base, a.d, r < cnt ? id : 0u, lane & 15);
-        }
-        cxn = lane < (int)cnt ? __ldg(a.xnorm + cand.i) : 0.f;
-        __syncwarp();
-        if (np > 0) pt_gram(crow, prow, pst, a.d, (np + 7) & ~7u, G1, lane);
-        pt_gram(crow, crow, pst, a.d, (cnt + 7) & ~7u, G2, lane);
-        __syncwarp();
-      }
-      // against the rows picked before this batch
-      bool s1 = false, dup1 = false;  // dup1 (clean Vamana): the node itself or an id picked before
-      if (lane < (int)cnt) {
-        if (cv) {
-          dup1 = cand.i == node;
-          for (uint32_t j = 0; j < np && !dup1; j++) dup1 = pid[j] == cand.i;
-          s1 = dup1;
-        }
-        for (uint32_t j = 0; j < np && !s1; j++) {
-          if (NSG && pid[j] == cand.i) s1 = true;
-          else {
-            float dd = TC ? (pxn[j] + cxn) - 2.f * G1[lane * PT_ROWS + j] : l2g(a.base, a.d, pid[j], cand.i);
-            s1 = MODE == 2 ? ssg_occludes(cand.d, pd[j], dd, a.threshold)
-                           : (NSG ? (dd < cand.d) : (__fmul_rn(a.alpha, dd) < cand.d));
-          }
-        }
-      }
-      // which earlier batch members would occlude this one
-      uint32_t occl = 0;
-      uint32_t dupo = 0;  // clean Vamana: earlier batch members with the same id
-      for (int b = 0; b < (int)cnt; b++) {
-        const uint32_t bid = __shfl_sync(FULL, cand.i, b);
-        const float bd = __shfl_sync(FULL, cand.d, b);
-        const float bxn = TC ? __shfl_sync(FULL, cxn, b) : 0.f;
-        if (b < lane && lane < (int)cnt) {
-          bool hit;
-          if ((NSG || cv) && bid == cand.i) {
-            hit = true;
-            if (cv) dupo |= 1u << b;
-          } else {
-            float dd = TC ? (bxn + cxn) - 2.f * G2[lane * PT_ROWS + b] : l2g(a.base, a.d, bid, cand.i);
-            hit = MODE == 2 ? ssg_occludes(cand.d, bd, dd, a.threshold)
-                            : (NSG ? (dd < cand.d) : (__fmul_rn(a.alpha, dd) < cand.d));
-          }
-          if (hit) occl |= 1u << b;
-        }
-      }
-      // the sequential walk of the reference over this batch
-      const uint32_t np0 = np;
-      uint32_t pm = 0;
-      uint32_t stop = cnt;
-      for (int b = 0; b < (int)cnt; b++) {
-        const bool sb = __shfl_sync(FULL, s1, b);
-        const uint32_t ob = __shfl_sync(FULL, occl, b);
-        const bool db = __shfl_sync(FULL, dup1, b) || (__shfl_sync(FULL, dupo, b) & pm);
-        const DI cb = DI{__shfl_sync(FULL, cand.d, b), __shfl_sync(FULL, cand.i, b)};
-        const bool skip = sb || (ob & pm);
-        if (!skip) {
-          pm |= 1u << b;
-          if (lane == 0) {
-            pid[np] = cb.i;
-            pd[np] = cb.d;
-          }
-          np++;
-          if (np == a.R) {
-            stop = b + 1;
-            done = true;
-            break;
-          }
-        } else if (!NSG && !db) {
-          if (lane == 0) heap[nskip] = HeapItem{cb.d, cb};
-          nskip++;
-        }
-      }
-      __syncwarp();
-      if (TC) {
-        // the rows picked in this batch join the picked rows (and norms)
-        uint32_t k = np0;
-        for (uint32_t mm = pm; mm; mm &= mm - 1, k++) {
-          const int b = __ffs(mm) - 1;
-          const float bxn = __shfl_sync(FULL, cxn, b);
-          for (uint32_t o = (uint32_t)lane * 16; o < a.d * 2; o += 32 * 16)
-            *reinterpret_cast<uint4 *>(prow + (size_t)k * pst + o) =
-                *reinterpret_cast<const uint4 *>(crow + (size_t)b * pst + o);
-          if (lane == 0) pxn[k] = bxn;
-        }
-        __syncwarp();
-      }
-      ex += stop;
+    uint32_t wbase = 0, nsaved = 0;  // pool position of the window; keys in `saved`
+    bool all_saved = true;
+    while (true) {  // windows
+    const uint32_t wend = min(wn, end - wbase);
+    if (!EXACT) {
+      for (uint32_t i = tid; i < PF_WINDOW / 32; i += PF_THREADS) gone[i] = 0;
+      __syncthreads();
     }
-    if (!NSG && np < a.R && nskip > 0) {
-      // refill from the skipped min-heap (component_prune.cpp:276-279)
+    while (!done && ex < wend) {
+      const uint32_t g0 = EXACT ? ex : 0u;  // position of gone's first bit
+      if (EXACT) {
+        if (tid < PF_NW) gone[tid] = 0;
+        __syncthreads();
+      }
+      const uint32_t w0 = ex + 32 * warp;
+      const uint32_t wcnt = w0 < wend ? min(32u, wend - w0) : 0u;
+      float cd = 0.f;
+      uint32_t cid = 0;
+      int cn = 0;
+      if (lane < wcnt) {
+        cd = kd(w0 + lane);
+        cid = ki(w0 + lane);
+        if (I8) cn = (int)__ldg(a.xnorm + cid);
+      }
+      uint8_t *wrow = cand + (size_t)f.cs * 32 * warp;
+      if (f.cs) {
+        const uint32_t ch = rb / 16;
+        for (uint32_t e = lane; e < ch * 32; e += 32) {  // (warp-uniform trips: e / ch is any row)
+          const uint32_t r = e / ch, k = e % ch;
+          const uint32_t id = __shfl_sync(FULL, cid, r);
+          if (r < wcnt) cp_async16(wrow + (size_t)r * f.cs + k * 16, rows + (size_t)id * rb + k * 16);
+        }
+        cp_async_wait_all();
+        __syncwarp();
+      }
+      auto row_of = [&](uint32_t c, uint32_t id) { return f.cs ? wrow + (size_t)c * f.cs : rows + (size_t)id * rb; };
+      auto pick_row = [&](uint32_t p) { return f.cs ? pick + (size_t)p * f.cs : rows + (size_t)pid[p] * rb; };
+      // drops candidate c (bit of the sorted position): clean Vamana's node
+      // itself and ids picked before
+      auto drop = [&](uint32_t c) { atomicOr(&gone[(w0 - g0 + c) >> 5], 1u << ((w0 - g0 + c) & 31)); };
+      // the candidates against the picks so far; wl[warp]: those left, in order
+      bool self_hit = cv && lane < wcnt && cid == node;
+      if (self_hit) drop(lane);
+      unsigned am = __ballot_sync(FULL, lane < wcnt && !self_hit);
+      uint32_t A = __popc(am);
+      if ((am >> lane) & 1u) wl[warp][__popc(am & lt)] = lane;
+      __syncwarp();
+      for (uint32_t j = 0; j < np && A > 0;) {
+        const uint32_t W = A <= 8 ? 8u : A <= 16 ? 16u : 32u, G = 32 / W;
+        const uint32_t at = lane & (W - 1), p = j + lane / W;
+        const bool on = at < A && p < np;
+        const uint32_t c = at < A ? wl[warp][at] : 0u;
+        const float xd = __shfl_sync(FULL, cd, c);
+        const uint32_t xi = __shfl_sync(FULL, cid, c);
+        const int xn = __shfl_sync(FULL, cn, c);
+        bool hit = false;
+        if (on) {
+          if ((NSG || cv) && pid[p] == xi) {
+            hit = true;
+            if (cv) drop(c);
+          } else {
+            hit = occludes(xd, pd[p], pf_dist<I8>(pick_row(p), row_of(c, xi), d, I8 ? pnrm[p] : 0, xn));
+            if (hit && pd[p] == xd && pid[p] != xi) amb = 1;
+          }
+        }
+        unsigned hm = __ballot_sync(FULL, hit);
+        if (G >= 2) hm |= hm >> 16;
+        if (G >= 4) hm |= hm >> 8;
+        am = ~hm & (A >= 32 ? FULL : (1u << A) - 1u);
+        __syncwarp();
+        if (lane < A && ((am >> lane) & 1u)) wl[warp][__popc(am & lt)] = c;
+        A = __popc(am);
+        __syncwarp();
+        j += G;
+      }
+      if (lane == 0) wc[warp] = A;
+      __syncthreads();
+      // the survivors in order: each pick is tested against the rest
+      while (true) {
+        int fw = 0;
+        while (fw < PF_NW && wc[fw] == 0) fw++;
+        if (fw == PF_NW) break;  // block-uniform
+        const uint32_t c = wl[fw][0], pos = ex + 32 * fw + c;
+        const uint32_t xi = ki(pos);
+        const float xd = kd(pos);
+        __syncthreads();  // everyone has read the lists
+        if (warp == fw) {
+          if (lane == 0) {
+            if (np > 0 && pd[np - 1] == xd && pid[np - 1] != xi) amb = 1;
+            pid[np] = xi;
+            pd[np] = xd;
+            if (I8) pnrm[np] = (int)__ldg(a.xnorm + xi);
+            gone[(pos - g0) >> 5] |= 1u << ((pos - g0) & 31);
+          }
+          if (f.cs) put_pick(np, cand + (size_t)f.cs * (32 * fw + c));
+          const uint32_t nx = lane + 1 < A ? wl[warp][lane + 1] : 0u;
+          __syncwarp();
+          wl[warp][lane] = nx;
+          A--;
+        }
+        np++;
+        __syncthreads();
+        if (np == a.R) {
+          // a later entry of the last pick's distance could have come first
+          if (tid == 0)
+            for (uint32_t i = pos + 1; i < wn && kd(i) == xd; i++)
+              if (ki(i) != xi) amb = 1;
+          done = true;
+          break;
+        }
+        if (A > 0) {
+          const uint32_t y = lane < A ? wl[warp][lane] : 0u;
+          const float yd = __shfl_sync(FULL, cd, y);
+          const uint32_t yi = __shfl_sync(FULL, cid, y);
+          const int yn = __shfl_sync(FULL, cn, y);
+          bool hit = false;
+          if (lane < A) {
+            if ((NSG || cv) && xi == yi) {
+              hit = true;
+              if (cv) drop(y);
+            } else {
+              hit = occludes(yd, xd, pf_dist<I8>(pick_row(np - 1), row_of(y, yi), d, I8 ? pnrm[np - 1] : 0, yn));
+              if (hit && xd == yd && xi != yi) amb = 1;
+            }
+          }
+          const unsigned keep = __ballot_sync(FULL, lane < A && !hit);
+          __syncwarp();
+          if ((keep >> lane) & 1u) wl[warp][__popc(keep & lt)] = y;
+          A = __popc(keep);
+          __syncwarp();
+        }
+        if (lane == 0) wc[warp] = A;
+        __syncthreads();
+      }
+      if (EXACT && !NSG && !done && warp == 0)  // the skipped entries, in order
+        for (uint32_t w = 0; w < PF_NW; w++) {
+          const uint32_t pos = ex + 32 * w + lane;
+          const bool skip = pos < wend && !((gone[w] >> lane) & 1u);
+          const unsigned sm = __ballot_sync(FULL, skip);
+          if (skip) heap[nskip + __popc(sm & lt)] = HeapItem{kd(pos), DI{kd(pos), ki(pos)}};
+          nskip += __popc(sm);
+        }
+      ex += 32 * PF_NW;
+      __syncthreads();
+    }
+    if (EXACT || done) break;
+    // equal distances on both sides of the bound: which were examined?
+    if (tid == 0 && wbase + wend == end && wend < wn) {
+      const float bd = kd(wend);
+      const uint32_t bi = ki(wend);
+      if (wend > 0 && kd(wend - 1) == bd) {
+        for (uint32_t i = wend + 1; i < wn && kd(i) == bd; i++)
+          if (ki(i) != bi) amb = 1;
+        for (uint32_t i = wend; i-- > 0 && kd(i) == bd;)
+          if (ki(i) != bi) amb = 1;
+      }
+    }
+    // the least skipped keys, for the Vamana refill: the first window's
+    if (!NSG && wbase == 0) {
+      if (warp == 0) {
+        uint32_t c = 0;
+        for (uint32_t b = 0; b < wend && c < PF_SAVED; b += 32) {
+          const bool skip = b + lane < wend && !((gone[b >> 5] >> lane) & 1u);
+          const unsigned sm = __ballot_sync(FULL, skip);
+          const uint32_t at = c + __popc(sm & lt);
+          if (skip && at < PF_SAVED) saved[at] = K[b + lane];
+          c += __popc(sm);
+        }
+        nsaved = min(c, PF_SAVED);
+        all_saved = wend == end && c < PF_SAVED;
+      }
+    }
+    wbase += wend;
+    if (wbase >= end) break;
+    __syncthreads();
+    wn = pf_window(U, m, K, wlo, false);
+    if (wn == 0) {  // a bin beyond the window's size
+      if (tid == 0) amb = 1;
+      break;
+    }
+    pf_sort<PF_WINDOW / PF_THREADS>(K);
+    ex = 0;
+    }
+    __syncthreads();
+    if (EXACT && !NSG && np < a.R && warp == 0) {
       if (lane == 0) {
         for (uint32_t k = 1; k <= nskip; k++) stl::push_heap(heap, (int)k, HeapItemLess());
         uint32_t hs = nskip;
@@ -381,16 +673,50 @@ __global__ void __launch_bounds__(PR_WARPS * 32) k_prune(PruneArgs a) {
           stl::pop_heap(heap, (int)hs, HeapItemLess());
           hs--;
         }
+        wc[0] = np;
       }
-      np = __shfl_sync(FULL, np, 0);
-      __syncwarp();
+    } else if (!NSG && np < a.R && warp == 0) {
+      // refill from the skipped min-heap (component_prune.cpp:276-279): the
+      // skipped entries in ascending order
+      float ld = -1.f;
+      uint32_t li = 0, i = 0;
+      for (; i < nsaved; i++) {
+        const float xd = __uint_as_float((uint32_t)(saved[i] >> 32));
+        const uint32_t xi = (uint32_t)saved[i];
+        if (xd == ld && xi != li && lane == 0) amb = 1;
+        if (np == a.R) {  // the entries past the last taken are looked at for a tie
+          if (xd != ld) break;
+          continue;
+        }
+        ld = xd;
+        li = xi;
+        bool again = false;  // clean Vamana: an id skipped twice is taken once
+        if (cv)
+          for (uint32_t j = lane; j < np; j += 32) again |= pid[j] == xi;
+        if (__any_sync(FULL, again)) continue;
+        if (lane == 0) {
+          pid[np] = xi;
+          pd[np] = xd;
+        }
+        np++;
+        __syncwarp();
+      }
+      if (i == nsaved && !all_saved && lane == 0) amb = 1;  // more were skipped than kept here
+      if (lane == 0) wc[0] = np;
+    } else if (tid == 0) {
+      wc[0] = np;
     }
-    for (uint32_t j = lane; j < np; j += 32) {
+    __syncthreads();
+    if (!EXACT && amb) {
+      if (tid == 0) f.redo[atomicAdd(f.nredo, 1u)] = qi;
+      continue;
+    }
+    np = wc[0];
+    for (uint32_t j = tid; j < np; j += PF_THREADS) {
       oid[j] = pid[j];
       od[j] = pd[j];
     }
-    if (lane == 0) a.out_deg[node] = np;
-    __syncwarp();
+    if (tid == 0) a.out_deg[node] = np;
   }
 }
 
@@ -1150,8 +1476,7 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   WV_CUDA(c, e);
   if (shared_seeds && !ssg)
     WV_CUDA(c, cudaMemcpyAsync(dseeds, ep_row.data(), p.L * 4, cudaMemcpyHostToDevice, c->stream));
-  const int prune_blocks = c->sms * 8;
-  const size_t nwarps = (size_t)prune_blocks * PR_WARPS;
+  const int prune_blocks = c->sms * 4;  // of the EXACT launch
   const float threshold = ssg ? ssg_threshold(p.A) : 0.f;
   for (uint32_t n0 = 0; n0 < n; n0 += CH) {
     const uint32_t cnt = std::min(CH, n - n0);
@@ -1166,8 +1491,8 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
     while (true) {
       DI *vis = c->buf<DI>("lk_vis", (size_t)cnt * vcap, &e);
       uint32_t *vcnt = c->buf<uint32_t>("lk_vcnt", cnt, &e);
-      int *gscr = c->buf<int>("lk_gscr", nwarps * (2 * (size_t)vcap + 256), &e);
-      HeapItem *hscr = c->buf<HeapItem>("lk_hscr", nwarps * (size_t)vcap, &e);
+      int *gscr = c->buf<int>("lk_gscr", prune_blocks * (2 * (size_t)vcap + 256), &e);
+      HeapItem *hscr = c->buf<HeapItem>("lk_hscr", prune_blocks * (size_t)vcap, &e);
       WV_CUDA(c, e);
       int rc = ssg ? run_prop2(c, n0, cnt, p.L, vis, vcnt, vcap)
                    : run_build_search(c, c->base.as<float>() + (size_t)n0 * c->d, cnt, dseeds,
@@ -1208,29 +1533,57 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
       pa.out_dist = p_dist;
       pa.out_deg = p_deg;
       pa.status = c->d_status();
-      // integer data (d % 32 == 0, d <= 128) and R <= 32: the pair distances
-      // from Gram tiles, the same values (WV_LINK_PRUNE=fp32 keeps the
+      // integer data with byte rows (d a multiple of 16 up to 256): the pair
+      // distances as exact integers (WV_LINK_PRUNE=fp32 keeps the
       // exact-order FP32 sums)
       const char *pr_env = getenv("WV_LINK_PRUNE");
-      const bool tc = c->base_int && c->d % 32 == 0 && c->d <= 128 && R <= PT_ROWS &&
-                      !(pr_env && std::string(pr_env) == "fp32");
-      pa.xnorm = tc ? c->xnorm.as<float>() : nullptr;
-      const size_t tsm = tc ? (size_t)PR_WARPS * pt_warp_bytes(c->d) : 0;
-      if (tc) {
-        if (ssg) WV_CUDA(c, cudaFuncSetAttribute(k_prune<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-        else if (!vamana) WV_CUDA(c, cudaFuncSetAttribute(k_prune<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-        else WV_CUDA(c, cudaFuncSetAttribute(k_prune<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+      const bool i8 = c->base_int && c->base8.p && !(pr_env && std::string(pr_env) == "fp32");
+      pa.xnorm = i8 ? c->xnorm.as<float>() : nullptr;
+      uint32_t *lists = c->buf<uint32_t>("lk_plist", PF_SIZES * (size_t)cnt, &e);
+      uint32_t *lcnts = c->buf<uint32_t>("lk_plcnt", PF_SIZES, &e);
+      WV_CUDA(c, e);
+      WV_CUDA(c, cudaMemsetAsync(lcnts, 0, PF_SIZES * 4, c->stream));
+      PruneFast pf{};
+      pf.base8 = i8 ? c->base8.as<uint8_t>() : nullptr;
+      // rows in shared memory where 4 warps' candidates and the picks fit
+      // (an odd multiple of 16 bytes apart: no bank conflicts)
+      const uint32_t rb16 = i8 ? c->d : c->d * 4;
+      auto row_stride = [&](bool exact) -> uint32_t {
+        const uint32_t cs = rb16 / 16 % 2 ? rb16 : rb16 + 16;
+        return pf_smem(pf.keys, cs, R, exact) <= 200 * 1024 ? cs : 0;
+      };
+      pf.redo = lists + (PF_SIZES - 1) * (size_t)cnt;
+      pf.nredo = lcnts + PF_SIZES - 1;
+      auto launch = [&](auto exact) -> cudaError_t {
+        constexpr bool X = decltype(exact)::value;
+        const size_t sm = pf_smem(pf.keys, pf.cs, R, X);
+        auto go = [&](auto kern) -> cudaError_t {
+          cudaError_t x = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+          int per = 0;
+          if (x == cudaSuccess) x = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, PF_THREADS, sm);
+          if (x != cudaSuccess) return x;
+          const uint32_t grid = X ? (uint32_t)prune_blocks : (uint32_t)(c->sms * std::max(per, 1) * 4);
+          kern<<<std::min<uint32_t>(cnt, grid), PF_THREADS, sm, c->stream>>>(pa, pf);
+          return cudaGetLastError();
+        };
+        if (ssg) return i8 ? go(k_prune_block<2, true, X>) : go(k_prune_block<2, false, X>);
+        if (!vamana) return i8 ? go(k_prune_block<1, true, X>) : go(k_prune_block<1, false, X>);
+        return i8 ? go(k_prune_block<0, true, X>) : go(k_prune_block<0, false, X>);
+      };
+      for (int l = 0; l < PF_SIZES; l++) {
+        pf.keys = pf_keys(l);
+        pf.cs = row_stride(false);
+        pf.list = l ? lists + (size_t)(l - 1) * cnt : nullptr;
+        pf.nlist = l ? lcnts + (l - 1) : nullptr;
+        pf.more = l < PF_SIZES - 1 ? lists + (size_t)l * cnt : nullptr;
+        pf.nmore = l < PF_SIZES - 1 ? lcnts + l : nullptr;
+        WV_CUDA(c, launch(std::false_type{}));
       }
-      if (ssg) {
-        if (tc) k_prune<2, true><<<prune_blocks, PR_WARPS * 32, tsm, c->stream>>>(pa);
-        else k_prune<2, false><<<prune_blocks, PR_WARPS * 32, 0, c->stream>>>(pa);
-      } else if (!vamana) {
-        if (tc) k_prune<1, true><<<prune_blocks, PR_WARPS * 32, tsm, c->stream>>>(pa);
-        else k_prune<1, false><<<prune_blocks, PR_WARPS * 32, 0, c->stream>>>(pa);
-      } else {
-        if (tc) k_prune<0, true><<<prune_blocks, PR_WARPS * 32, tsm, c->stream>>>(pa);
-        else k_prune<0, false><<<prune_blocks, PR_WARPS * 32, 0, c->stream>>>(pa);
-      }
+      pf.keys = pf_keys(1);
+      pf.cs = row_stride(true);
+      pf.list = pf.redo;
+      pf.nlist = pf.nredo;
+      WV_CUDA(c, launch(std::true_type{}));
       WV_CUDA(c, cudaGetLastError());
       rc = check_device_status(c, "prune");
       if (rc) return rc;
