@@ -25,13 +25,12 @@
 //    itself into each neighbour's row (dedup, append, or re-prune).  Node n's
 //    row at that moment is its pruned row plus the insertions from nodes < n
 //    that still listed n -- and those can only be nodes m < n with n in m's
-//    PRUNED row.  So nodes are processed by level (level(n) = 1 + max level
-//    of such m): all nodes of a level run in parallel, each applying the
-//    insertions from lower ids in id order, which gives its row at its turn
-//    (kept as a snapshot).  Then every row applies, in id order, the
-//    insertions from higher ids, read from their snapshots.  Each warp keeps
-//    the vectors' pairwise distances of its row in shared memory, so an
-//    insertion costs one new distance column.
+//    PRUNED row.  So nodes run in id order across all warps, each waiting for
+//    those lower ids' rows and applying their insertions in id order, which
+//    gives its row at its turn (kept as a snapshot).  Then every row applies,
+//    in id order, the insertions from higher ids, read from their snapshots.
+//    Each warp keeps its row's vectors and their pairwise distances in shared
+//    memory, so an insertion costs one new distance column.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -723,31 +722,35 @@ __global__ void __launch_bounds__(PF_THREADS) k_prune_block(PruneArgs a, PruneFa
 // ---------------------------------------------------------------- InterInsert
 struct IIArgs {
   const float *base;
+  const uint8_t *base8;    // byte rows (integer data, d a multiple of 16 up to 256), with their squared norms
+  const float *xnorm;
   uint32_t d, n, R;
   float alpha;
-  int vamana;
   int clean;               // Vamana re-prune closest first, each candidate against its own distance
-  int ssg;                 // SSG re-prune: angle test, sentinel after a short result
-  int ints;                // integer rows in [0, 255], d <= 256: any summation order is exact
   float threshold;
+  uint32_t cs;             // bytes between row vectors in shared memory (0: read where they lie)
+  uint32_t spare;          // vector slots beyond the R + 1 of a re-prune
+  const uint8_t *pops;     // Vamana: pops[64 N + k], the k-th item popped off a heap of N items of equal keys
   const uint32_t *p_ids;   // pruned rows (width R)
   const float *p_dist;
   const uint32_t *p_deg;
   uint32_t *s_ids;         // rows at each node's turn (width R)
   float *s_dist;
   uint32_t *s_deg;
+  uint32_t *s_kept;        // (NSG) IIRow::kept of those rows
   uint32_t *f_ids;         // final rows (width R)
   float *f_dist;
   uint32_t *f_deg;
-  const uint32_t *nodes;   // nodes of this launch
-  uint32_t nn;
+  uint32_t *done;          // level(n) + 1 once row n is at its turn, 0 before
+  uint32_t *next, *maxlev; // forward: the next node, the highest level
   const unsigned long long *req;  // per target: (sender << 32 | index) sorted
   const uint32_t *req_off, *req_cnt;
   int *status;
 };
 
 constexpr int II_WARPS = 4;
-constexpr int II_SLOTS = LINK_MAX_R + 1;
+constexpr uint32_t II_SPARE = 4;          // senders whose rows and vectors are loaded together
+constexpr uint32_t II_POLLS = 1u << 26;   // polls of a sender's flag before the wait gives up
 
 struct Ent3 {
   float d;
@@ -762,346 +765,531 @@ struct HeapIdx {  // MinHeap item of the re-prune: key and temp index
   uint32_t k;
 };
 struct HeapIdxLess {
-  __device__ bool operator()(const HeapIdx &a, const HeapIdx &b) const { return a.key > b.key; }
+  __host__ __device__ bool operator()(const HeapIdx &a, const HeapIdx &b) const { return a.key > b.key; }
 };
 
-// per-warp state: the row (with the slot holding each entry's vector), the
-// re-prune scratch, and -- in the dynamic tail -- the pairwise distances of
-// the slot vectors (S x S, S = R + 1) and the vectors themselves (S rows)
+// A warp holds one row: entry j in lane j % 32's set j / 32 of registers, and
+// in shared memory the re-prune's scratch, the row vectors in slots, their
+// norms (bytes) or ids, and the slots' pairwise distances.
 struct IIWarp {
-  Ent3 row[II_SLOTS];
-  Ent3 tmp[II_SLOTS];
-  uint32_t sid[II_SLOTS];  // id held by each slot
-  uint32_t res[II_SLOTS];
-  HeapIdx heap[II_SLOTS];
-  float *D;                // S x S
-  float *V;                // S x vs floats, or null: distances from global memory
+  Ent3 *tmp;      // 64
+  HeapIdx *heap;  // 64 (clean Vamana)
+  uint32_t *res;  // 64
+  uint32_t *sid;  // NS: id of each slot's vector
+  float *D;       // NS x NS
+  uint8_t *V;     // NS x cs
+  uint32_t NS;
 };
-
-__host__ __device__ inline size_t ii_warp_bytes(uint32_t R, uint32_t vs) {
-  const size_t S = R + 1;
-  return ((sizeof(IIWarp) + 15) & ~size_t(15)) + ((S * S * 4 + 15) & ~size_t(15)) + S * vs * 4;
+__host__ __device__ inline uint32_t ii_slots(uint32_t R, uint32_t spare) { return R + 1 + spare; }
+__host__ __device__ inline size_t ii_warp_bytes(uint32_t R, uint32_t cs, uint32_t spare) {
+  const size_t S = ii_slots(R, spare);
+  return 64 * sizeof(Ent3) + 64 * sizeof(HeapIdx) + 64 * 4 + ((S * 4 + 15) & ~size_t(15)) +
+         ((S * S * 4 + 15) & ~size_t(15)) + S * cs;
 }
-
-__device__ inline IIWarp &ii_carve(uint8_t *smem, int warp, uint32_t R, uint32_t vs) {
-  uint8_t *p = smem + (size_t)warp * ii_warp_bytes(R, vs);
-  IIWarp &w = *reinterpret_cast<IIWarp *>(p);
-  p += (sizeof(IIWarp) + 15) & ~size_t(15);
+__device__ inline IIWarp ii_carve(uint8_t *p, uint32_t R, uint32_t spare) {
+  IIWarp w;
+  w.NS = ii_slots(R, spare);
+  w.tmp = reinterpret_cast<Ent3 *>(p);
+  p += 64 * sizeof(Ent3);
+  w.heap = reinterpret_cast<HeapIdx *>(p);
+  p += 64 * sizeof(HeapIdx);
+  w.res = reinterpret_cast<uint32_t *>(p);
+  p += 64 * 4;
+  w.sid = reinterpret_cast<uint32_t *>(p);
+  p += ((size_t)w.NS * 4 + 15) & ~size_t(15);
   w.D = reinterpret_cast<float *>(p);
-  p += ((size_t)(R + 1) * (R + 1) * 4 + 15) & ~size_t(15);
-  w.V = vs ? reinterpret_cast<float *>(p) : nullptr;
+  p += ((size_t)w.NS * w.NS * 4 + 15) & ~size_t(15);
+  w.V = p;
   return w;
 }
 
-// copies base row `id` into vector slot f (one warp, 16-byte pieces)
-__device__ __forceinline__ void ii_stage(const IIArgs &a, IIWarp &w, uint32_t vs, uint32_t f, uint32_t id, int lane) {
-  if (!w.V) return;
-  const float4 *src = reinterpret_cast<const float4 *>(a.base + (size_t)id * a.d);
-  float4 *dst = reinterpret_cast<float4 *>(w.V + (size_t)f * vs);
-  for (uint32_t k = lane; k < (a.d >> 2); k += 32) dst[k] = __ldg(src + k);
-}
+struct IIRow {
+  float d[2];
+  uint32_t i[2], slot[2];
+  uint32_t rs;   // entries
+  bool vvalid;   // every entry has a slot holding its vector
+  bool dvalid;   // D holds the slots' pairwise distances
+  // (NSG) a full row, strictly ascending, no entry occluded by a nearer one:
+  // what a prune or re-prune that takes R entries with distinct keys leaves.
+  // Re-pruning it with s then needs only the distances to s: the nearer
+  // entries are taken, s unless one of them occludes it (the row stays as it
+  // was), the farther ones unless s occludes them.
+  bool kept;
+  unsigned long long free;  // slots not in use
+};
 
-// exact-order distance between the vectors of slots x and y
-__device__ __forceinline__ float ii_dist(const IIArgs &a, const IIWarp &w, uint32_t vs, uint32_t x, uint32_t y) {
-  if (!w.V) return l2g(a.base, a.d, w.sid[x], w.sid[y]);
-  const float4 *p = reinterpret_cast<const float4 *>(w.V + (size_t)x * vs);
-  const float4 *q = reinterpret_cast<const float4 *>(w.V + (size_t)y * vs);
-  const uint32_t d4 = a.d >> 2;
-  if (a.ints) {
-    // every partial sum is an integer below 2^24, so four chains give the
-    // exact-order value
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-    uint32_t g = 0;
-    for (; g + 4 <= d4; g += 4) {
-      s0 = __fadd_rn(s0, group4(p[g], q[g]));
-      s1 = __fadd_rn(s1, group4(p[g + 1], q[g + 1]));
-      s2 = __fadd_rn(s2, group4(p[g + 2], q[g + 2]));
-      s3 = __fadd_rn(s3, group4(p[g + 3], q[g + 3]));
-    }
-    for (; g < d4; g++) s0 = __fadd_rn(s0, group4(p[g], q[g]));
-    return __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
-  }
-  float acc = 0.f;
-#pragma unroll 4
-  for (uint32_t g = 0; g < d4; g++) acc = __fadd_rn(acc, group4(p[g], q[g]));
-  return acc;
-}
+template <bool I8>
+struct II {
+  const IIArgs &a;
+  IIWarp w;
+  int lane;
 
-// gives row entry j (slot INVALID) a free slot, its vector and its distance
-// column to the other slotted entries (dvalid rows only)
-__device__ void ii_slot_entry(const IIArgs &a, IIWarp &w, uint32_t vs, uint32_t rs, uint32_t j, int lane) {
-  const uint32_t S = a.R + 1;
-  unsigned long long used = 0;
-  for (uint32_t t = 0; t < rs; t++)
-    if (t != j) used |= 1ull << w.row[t].slot;
-  const uint32_t f = __ffsll(~used) - 1;
-  if (lane == 0) {
-    w.row[j].slot = f;
-    w.sid[f] = w.row[j].i;
+  __device__ const uint8_t *vec(uint32_t slot) const {
+    if (a.cs) return w.V + (size_t)slot * a.cs;
+    return I8 ? a.base8 + (size_t)w.sid[slot] * a.d
+              : reinterpret_cast<const uint8_t *>(a.base + (size_t)w.sid[slot] * a.d);
   }
-  __syncwarp();
-  ii_stage(a, w, vs, f, w.row[j].i, lane);
-  __syncwarp();
-  for (uint32_t t = lane; t < rs; t += 32) {
-    if (t == j) continue;
-    const uint32_t o = w.row[t].slot;
-    const float dd = ii_dist(a, w, vs, o, f);
-    w.D[f * S + o] = dd;
-    w.D[o * S + f] = dd;
+  // starts the copy of row `id` into slot f (a warp); the caller waits
+  __device__ void stage(uint32_t f, uint32_t id) const {
+    if (lane == 0) w.sid[f] = id;
+    if (!a.cs) return;
+    const uint8_t *src = I8 ? a.base8 + (size_t)id * a.d : reinterpret_cast<const uint8_t *>(a.base + (size_t)id * a.d);
+    const uint32_t ch = (I8 ? a.d : a.d * 4) / 16;
+    for (uint32_t k = lane; k < ch; k += 32) cp_async16(w.V + (size_t)f * a.cs + k * 16, src + k * 16);
   }
-  __syncwarp();
-}
-
-// applies "insert `s` (distance dist, sender index i) into this row" exactly
-// as InterInsert does to des_pool (component_refine.cpp:484-540 / 884-949).
-// `kept` (NSG): the last re-prune took R entries with distinct keys, so the
-// row is sorted and no entry is occluded by a nearer one.  Re-pruning such a
-// row with s gives the same row when s ties no key and is either farther
-// than every entry (the walk is full before it reaches s) or occluded by a
-// nearer entry (s is skipped and every entry is taken again), so those
-// insertions stop early.
-__device__ void ii_apply(const IIArgs &a, IIWarp &w, uint32_t vs, uint32_t &rs, bool &dvalid, bool &kept, uint32_t s,
-                         float dist, uint32_t i, int lane) {
-  bool dup = false;
-  for (uint32_t j = lane; j < rs; j += 32) dup |= w.row[j].i == s;
-  if (__any_sync(FULL, dup)) return;
-  const uint32_t R = a.R, S = R + 1;
-  if (rs + 1 <= R) {  // room: append at the sentinel
-    if (lane == 0) w.row[rs] = Ent3{dist, s, INVALID};
+  __device__ void landed() const {
+    cp_async_wait_all();
     __syncwarp();
-    if (dvalid) ii_slot_entry(a, w, vs, rs + 1, rs, lane);
-    rs++;
-    kept = false;
-    return;
   }
-  const bool nsg = !a.vamana && !a.ssg;
-  bool tie_s = false;
-  if (nsg && kept) {
-    bool far = true;
-    for (uint32_t j = lane; j < rs; j += 32) {
-      const float rd = w.row[j].d;
-      tie_s |= rd == dist;
-      far &= rd < dist;
+  __device__ float dist(uint32_t x, uint32_t y) const {
+    return pf_dist<I8>(vec(x), vec(y), a.d, I8 ? (int)__ldg(a.xnorm + w.sid[x]) : 0,
+                       I8 ? (int)__ldg(a.xnorm + w.sid[y]) : 0);
+  }
+  __device__ unsigned long long used(const IIRow &r) const {
+    unsigned lo = 0, hi = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      if (lane + 32 * h < (int)r.rs) {
+        const uint32_t s = r.slot[h];
+        if (s < 32) lo |= 1u << s;
+        else hi |= 1u << (s - 32);
+      }
+    lo = __reduce_or_sync(FULL, lo);
+    hi = __reduce_or_sync(FULL, hi);
+    return ((unsigned long long)hi << 32) | lo;
+  }
+  // kept: whether the row, if full and strictly ascending, is a prune's or a
+  // re-prune's result
+  __device__ void load(IIRow &r, const uint32_t *ids, const float *dist, uint32_t deg, bool kept) const {
+    r.rs = deg;
+    r.vvalid = r.dvalid = false;
+    bool asc = kept && deg == a.R;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint32_t j = lane + 32 * h;
+      r.d[h] = j < deg ? dist[j] : 0.f;
+      r.i[h] = j < deg ? ids[j] : INVALID;
+      r.slot[h] = 0;
     }
-    tie_s = __any_sync(FULL, tie_s);
-    if (!tie_s && __all_sync(FULL, far)) return;
+    float up0 = __shfl_up_sync(FULL, r.d[0], 1), up1 = __shfl_up_sync(FULL, r.d[1], 1);
+    const float last0 = __shfl_sync(FULL, r.d[0], 31);
+    if (lane == 0) up1 = last0;
+    if (lane > 0 && lane < (int)deg) asc &= up0 < r.d[0];
+    if (lane + 32 < (int)deg) asc &= up1 < r.d[1];
+    r.kept = __all_sync(FULL, asc);
+    r.free = ~0ull >> (64 - w.NS);
   }
-  // a re-prune needs the pairwise distances of row + s
-  if (!dvalid) {
-    for (uint32_t j = lane; j < rs; j += 32) {
-      w.row[j].slot = j;
-      w.sid[j] = w.row[j].i;
-    }
-    __syncwarp();
-    for (uint32_t j = 0; j < rs; j++) ii_stage(a, w, vs, j, w.row[j].i, lane);
-    __syncwarp();
-    for (uint32_t p = lane; p < rs * rs; p += 32) {
-      const uint32_t x = p / rs, y = p % rs;
-      if (x < y) {
-        const float dd = ii_dist(a, w, vs, x, y);
-        w.D[x * S + y] = dd;
-        w.D[y * S + x] = dd;
+  __device__ void store(const IIRow &r, uint32_t *ids, float *dist) const {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint32_t j = lane + 32 * h;
+      if (j < r.rs) {
+        ids[j] = r.i[h];
+        dist[j] = r.d[h];
       }
     }
-    dvalid = true;
+  }
+  // slots and vectors for the whole row
+  __device__ void give_slots(IIRow &r) const {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      unsigned long long f = r.free;  // entry j takes the j-th free slot
+      const uint32_t j = lane + 32 * h;
+      if (j < r.rs) {
+        for (uint32_t k = 0; k < j; k++) f &= f - 1;
+        r.slot[h] = __ffsll(f) - 1;
+      }
+    }
+    for (uint32_t j = 0; j < r.rs; j++) {
+      const uint32_t id = j < 32 ? __shfl_sync(FULL, r.i[0], j) : __shfl_sync(FULL, r.i[1], j - 32);
+      const uint32_t sl = j < 32 ? __shfl_sync(FULL, r.slot[0], j) : __shfl_sync(FULL, r.slot[1], j - 32);
+      stage(sl, id);
+    }
+    r.free &= ~used(r);
+    r.vvalid = true;
+  }
+  __device__ void all_pairs(IIRow &r) const {
+    const uint32_t np = r.rs * (r.rs - 1) / 2;
+    for (uint32_t p0 = 0; p0 < np; p0 += 32) {
+      const uint32_t p = p0 + lane;
+      // pair p of the triangle y < x: x (x - 1) / 2 + y
+      uint32_t x = (uint32_t)((1.f + sqrtf(1.f + 8.f * (float)p)) * 0.5f);
+      while (x * (x - 1) / 2 > p) x--;
+      while ((x + 1) * x / 2 <= p) x++;
+      const uint32_t y = p - x * (x - 1) / 2;
+      const uint32_t sx0 = __shfl_sync(FULL, r.slot[0], x & 31), sx1 = __shfl_sync(FULL, r.slot[1], x & 31);
+      const uint32_t sy0 = __shfl_sync(FULL, r.slot[0], y & 31), sy1 = __shfl_sync(FULL, r.slot[1], y & 31);
+      if (p < np) {
+        const uint32_t sx = x < 32 ? sx0 : sx1, sy = y < 32 ? sy0 : sy1;
+        const float dd = dist(sx, sy);
+        w.D[sx * w.NS + sy] = dd;
+        w.D[sy * w.NS + sx] = dd;
+      }
+    }
+    r.dvalid = true;
     __syncwarp();
   }
-  // s takes the free slot (the row holds at most R of the R + 1 slots)
-  if (lane == 0) w.row[rs] = Ent3{dist, s, INVALID};
-  __syncwarp();
-  ii_slot_entry(a, w, vs, rs + 1, rs, lane);
-  if (nsg && kept && !tie_s) {
-    const uint32_t fs = w.row[rs].slot;
-    bool occ = false;
-    for (uint32_t j = lane; j < rs; j += 32) {
-      const Ent3 r = w.row[j];
-      occ |= r.d < dist && w.D[r.slot * S + fs] < dist;
-    }
-    if (__any_sync(FULL, occ)) return;
-  }
-  const uint32_t T = rs + 1;
-  bool any_tie = false;
-  // std::sort(temp_pool) (component_refine.cpp:503 / 901): with distinct keys
-  // the sorted array is unique, so each lane places its entries by rank;
-  // tied keys take the one-lane replica of std::sort
-  {
-    const Ent3 e0 = lane < T ? w.row[lane] : Ent3{0.f, 0u, 0u};
-    const Ent3 e1 = lane + 32 < T ? w.row[lane + 32] : Ent3{0.f, 0u, 0u};
-    uint32_t r0 = 0, r1 = 0;
-    bool tie = false;
-    for (uint32_t t = 0; t < T; t++) {
-      const float kt = w.row[t].d;
-      r0 += kt < e0.d;
-      r1 += kt < e1.d;
-      tie |= (lane < T && t != lane && kt == e0.d) || (lane + 32 < T && t != lane + 32 && kt == e1.d);
-    }
-    any_tie = __any_sync(FULL, tie);
-    if (any_tie) {
-      for (uint32_t j = lane; j < T; j += 32) w.tmp[j] = w.row[j];
+
+  // "insert `s` (distance sd, sender index si) into this row" exactly as
+  // InterInsert does to des_pool (component_refine.cpp:484-540 / 884-949 /
+  // 660-720).  fs: the slot s's vector is being copied to, or INVALID
+  template <int MODE>
+  __device__ void apply(IIRow &r, uint32_t s, float sd, uint32_t si, uint32_t fs) const {
+    constexpr bool NSG = MODE == 1;
+    const uint32_t R = a.R, NS = w.NS, rs = r.rs;
+    const bool h0 = lane < (int)rs, h1 = lane + 32 < (int)rs;
+    auto give_back = [&]() {
+      if (fs != INVALID) r.free |= 1ull << fs;
+    };
+    if (__any_sync(FULL, (h0 && r.i[0] == s) || (h1 && r.i[1] == s))) return give_back();
+    auto column = [&](uint32_t f, float (&x)[2]) {  // distances of the row's entries to slot f
+      x[0] = x[1] = 0.f;
+      if (h0) x[0] = dist(r.slot[0], f);
+      if (h1) x[1] = dist(r.slot[1], f);
+      if (r.dvalid) {
+        if (h0) w.D[f * NS + r.slot[0]] = w.D[r.slot[0] * NS + f] = x[0];
+        if (h1) w.D[f * NS + r.slot[1]] = w.D[r.slot[1] * NS + f] = x[1];
+      }
       __syncwarp();
-      if (lane == 0) stl::sort(w.tmp, (int)T, Ent3Less());
+    };
+    auto slot_for = [&]() {
+      if (fs == INVALID) {
+        fs = __ffsll(r.free) - 1;
+        r.free &= r.free - 1;
+        stage(fs, s);
+      }
+      landed();
+    };
+    if (rs + 1 <= R) {  // room: append at the sentinel
+      if (r.vvalid) {
+        slot_for();
+        float x[2];
+        if (r.dvalid) column(fs, x);
+      } else {
+        give_back();
+        fs = 0;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        if (lane + 32 * h == (int)rs) {
+          r.d[h] = sd;
+          r.i[h] = s;
+          r.slot[h] = fs;
+        }
+      r.rs = rs + 1;
+      r.kept = false;
+      return;
+    }
+    const unsigned n0 = __ballot_sync(FULL, h0 && r.d[0] < sd), n1 = __ballot_sync(FULL, h1 && r.d[1] < sd);
+    const bool tie_s = __any_sync(FULL, (h0 && r.d[0] == sd) || (h1 && r.d[1] == sd));
+    const uint32_t nnear = __popc(n0) + __popc(n1);
+    const bool quick = NSG && r.kept && !tie_s;
+    if (quick && nnear == rs) return give_back();  // farther than a full row's entries
+    if (!r.vvalid) give_slots(r);
+    slot_for();
+    const unsigned long long old_slots = used(r);
+    if (!quick && !r.dvalid) all_pairs(r);
+    float x[2];
+    column(fs, x);
+    uint32_t nres = 0;
+    if (quick) {
+      if (__any_sync(FULL, (h0 && r.d[0] < sd && x[0] < sd) || (h1 && r.d[1] < sd && x[1] < sd))) {
+        r.free |= 1ull << fs;
+        return;
+      }
+      // the survivors, in order, with s after the nearer ones
+      const bool k0 = h0 && (r.d[0] < sd || !(x[0] < r.d[0])), k1 = h1 && (r.d[1] < sd || !(x[1] < r.d[1]));
+      const unsigned m0 = __ballot_sync(FULL, k0), m1 = __ballot_sync(FULL, k1);
+      const unsigned lt = (1u << lane) - 1u;
+      const uint32_t p0 = __popc(m0 & lt) + (r.d[0] < sd ? 0u : 1u);
+      const uint32_t p1 = __popc(m0) + __popc(m1 & lt) + (r.d[1] < sd ? 0u : 1u);
+      if (k0) w.tmp[p0] = Ent3{r.d[0], r.i[0], r.slot[0]};
+      if (k1) w.tmp[p1] = Ent3{r.d[1], r.i[1], r.slot[1]};
+      if (lane == 0) w.tmp[nnear] = Ent3{sd, s, fs};
+      __syncwarp();
+      nres = min(R, (uint32_t)__popc(m0) + __popc(m1) + 1);
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        if (lane + 32 * h < (int)nres) {
+          const Ent3 e = w.tmp[lane + 32 * h];
+          r.d[h] = e.d;
+          r.i[h] = e.i;
+          r.slot[h] = e.slot;
+        }
+      r.kept = nres == R;
+      // (a shorter result leaves the old entries at the remaining positions)
     } else {
+      const uint32_t T = rs + 1;
+      // the row and s in order: std::sort(temp_pool) (component_refine.cpp:503
+      // / 901): with distinct keys the sorted array is unique, so each lane
+      // places its entries by rank; tied keys take the one-lane replica
+      Ent3 e0 = h0 ? Ent3{r.d[0], r.i[0], r.slot[0]} : Ent3{sd, s, fs};
+      Ent3 e1 = h1 ? Ent3{r.d[1], r.i[1], r.slot[1]} : Ent3{sd, s, fs};
+      uint32_t r0 = 0, r1 = 0;
+      bool tie = false;
+      for (uint32_t t = 0; t < T; t++) {
+        const float kt = t < 32 ? __shfl_sync(FULL, e0.d, t) : __shfl_sync(FULL, e1.d, t - 32);
+        r0 += kt < e0.d;
+        r1 += kt < e1.d;
+        tie |= (lane < T && t != lane && kt == e0.d) || (lane + 32 < T && t != lane + 32 && kt == e1.d);
+      }
+      const bool any_tie = __any_sync(FULL, tie);
+      if (any_tie) {
+        r0 = lane;
+        r1 = lane + 32;
+      }
       if (lane < T) w.tmp[r0] = e0;
       if (lane + 32 < T) w.tmp[r1] = e1;
-    }
-    __syncwarp();
-  }
-  uint32_t nres = 0;
-  if (a.vamana) {
-    // compat: farthest first, every candidate against temp_pool[i].d (the
-    // outer index, refine.cpp:907); clean: closest first, each candidate
-    // against its own distance (the rule of PruneVAMANA)
-    uint32_t nskip = 0;
-    for (int kk = 0; kk < (int)T; kk++) {
-      const int k = a.clean ? kk : (int)T - 1 - kk;
-      const float cur = a.clean ? w.tmp[k].d : w.tmp[i].d;
-      const uint32_t ks = w.tmp[k].slot;
-      bool hit = false;
-      for (uint32_t j = lane; j < nres; j += 32) hit |= __fmul_rn(a.alpha, w.D[w.tmp[w.res[j]].slot * S + ks]) < cur;
-      const bool skip = __any_sync(FULL, hit);
-      if (!skip) {
-        if (lane == 0) w.res[nres] = (uint32_t)k;
-        nres++;
+      __syncwarp();
+      if (any_tie && lane == 0) stl::sort(w.tmp, (int)T, Ent3Less());
+      __syncwarp();
+      const Ent3 p0 = lane < T ? w.tmp[lane] : Ent3{0.f, 0u, 0u};
+      const Ent3 p1 = lane + 32 < T ? w.tmp[lane + 32] : Ent3{0.f, 0u, 0u};
+      // bit q of o0 / o1: sorted entry q would occlude this lane's entry
+      // (q before p, or any q for Vamana's farthest-first walk)
+      unsigned long long o0 = 0, o1 = 0;
+      const float cur = MODE == 0 && !a.clean ? w.tmp[si].d : 0.f;
+      for (uint32_t q = 0; q < T; q++) {
+        const Ent3 e = w.tmp[q];
+        auto occ = [&](const Ent3 &p, uint32_t at) -> bool {
+          if (at >= T || at == q || (MODE != 0 && q > at)) return false;
+          const float dd = w.D[e.slot * NS + p.slot];
+          if (MODE == 0) return __fmul_rn(a.alpha, dd) < (a.clean ? p.d : cur);
+          return e.i == p.i || (MODE == 2 ? ssg_occludes(p.d, e.d, dd, a.threshold) : (dd < p.d));
+        };
+        if (occ(p0, lane)) o0 |= 1ull << q;
+        if (T > 32 && occ(p1, lane + 32)) o1 |= 1ull << q;
+      }
+      auto mask_of = [&](uint32_t st) { return st < 32 ? __shfl_sync(FULL, o0, st) : __shfl_sync(FULL, o1, st - 32); };
+      if (MODE == 0) {
+        // compat: farthest first, every candidate against temp_pool[i].d (the
+        // outer index, refine.cpp:907); clean: closest first, each candidate
+        // against its own distance (the rule of PruneVAMANA)
+        unsigned long long taken = 0;
+        uint32_t nskip = 0;
+        for (uint32_t kk = 0; kk < T && nres < R; kk++) {
+          const uint32_t k = a.clean ? kk : T - 1 - kk;
+          if (!(mask_of(k) & taken)) {
+            taken |= 1ull << k;
+            if (lane == 0) w.res[nres] = k;
+            nres++;
+          } else {
+            if (lane == 0) w.heap[nskip] = HeapIdx{a.clean ? w.tmp[k].d : cur, k};
+            nskip++;
+          }
+        }
+        __syncwarp();
+        const uint32_t take = min(R - nres, nskip);
+        if (take > 0) {
+          if (!a.clean) {
+            // every key is `cur`: the heap's pops follow from its size
+            for (uint32_t t = lane; t < take; t += 32) w.res[nres + t] = w.heap[a.pops[64 * nskip + t]].k;
+          } else if (lane == 0) {
+            for (uint32_t k = 1; k <= nskip; k++) stl::push_heap(w.heap, (int)k, HeapIdxLess());
+            for (uint32_t t = 0; t < take; t++) {
+              w.res[nres + t] = w.heap[0].k;
+              stl::pop_heap(w.heap, (int)(nskip - t), HeapIdxLess());
+            }
+          }
+          nres += take;
+          __syncwarp();
+        }
       } else {
-        if (lane == 0) {
-          w.heap[nskip] = HeapIdx{cur, (uint32_t)k};
-          stl::push_heap(w.heap, (int)(nskip + 1), HeapIdxLess());
+        // entry 0, then each entry that no taken entry occludes, up to R
+        // (component_refine.cpp:505-526)
+        unsigned long long taken = 1ull;
+        nres = 1;
+        for (uint32_t st = 1; nres < R && st < T; st++)
+          if (!(mask_of(st) & taken)) {
+            taken |= 1ull << st;
+            nres++;
+          }
+        if (lane < T && ((taken >> lane) & 1ull)) w.res[__popcll(taken & ((1ull << lane) - 1ull))] = lane;
+        if (lane + 32 < T && ((taken >> (lane + 32)) & 1ull))
+          w.res[__popcll(taken & ((1ull << (lane + 32)) - 1ull))] = lane + 32;
+        __syncwarp();
+      }
+      // des_pool[t] = result[t] for t < result.size() (refine.cpp:527-530,
+      // 943-946, 706-712).  Vamana results always hold R entries; an NSG
+      // result may be shorter and then, with no sentinel written, the old
+      // entries at positions result.size()..R-1 stay in the row; SSG writes
+      // the sentinel.
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        if (lane + 32 * h < (int)nres) {
+          const Ent3 e = w.tmp[w.res[lane + 32 * h]];
+          r.d[h] = e.d;
+          r.i[h] = e.i;
+          r.slot[h] = e.slot;
         }
-        nskip++;
-      }
-      __syncwarp();
-      if (nres == R) break;
+      r.kept = NSG && nres == R && !any_tie;
+      if (MODE != 1) r.rs = nres;
     }
-    if (nres < R && nskip > 0) {
-      if (lane == 0) {
-        uint32_t hs = nskip;
-        while (nres < R && hs > 0) {
-          w.res[nres++] = w.heap[0].k;
-          stl::pop_heap(w.heap, (int)hs, HeapIdxLess());
-          hs--;
-        }
-      }
-      nres = __shfl_sync(FULL, nres, 0);
-      __syncwarp();
-    }
-  } else if (!a.ssg) {
-    // NSG (component_refine.cpp:505-526): bit r of o0 / o1 is set when sorted
-    // entry r < p occludes this lane's entry p = lane / lane + 32 (the same
-    // id, or nearer to p than p is to the node); the walk then takes entry 0
-    // and each later entry that no taken entry occludes, up to R
-    const Ent3 p0 = lane < T ? w.tmp[lane] : Ent3{0.f, 0u, 0u};
-    const Ent3 p1 = lane + 32 < T ? w.tmp[lane + 32] : Ent3{0.f, 0u, 0u};
-    unsigned long long o0 = 0, o1 = 0;
-    for (uint32_t r = 0; r + 1 < T; r++) {
-      const Ent3 q = w.tmp[r];
-      if (r < lane && lane < T && (q.i == p0.i || w.D[q.slot * S + p0.slot] < p0.d)) o0 |= 1ull << r;
-      if (r < lane + 32 && lane + 32 < T && (q.i == p1.i || w.D[q.slot * S + p1.slot] < p1.d)) o1 |= 1ull << r;
-    }
-    unsigned long long taken = 1ull;
-    nres = 1;
-    for (uint32_t st = 1; nres < R && st < T; st++) {
-      const unsigned long long o = st < 32 ? __shfl_sync(FULL, o0, st) : __shfl_sync(FULL, o1, st - 32);
-      if (!(o & taken)) {
-        taken |= 1ull << st;
-        nres++;
-      }
-    }
-    if (lane < T && ((taken >> lane) & 1ull)) w.res[__popcll(taken & ((1ull << lane) - 1ull))] = lane;
-    if (lane + 32 < T && ((taken >> (lane + 32)) & 1ull))
-      w.res[__popcll(taken & ((1ull << (lane + 32)) - 1ull))] = lane + 32;
     __syncwarp();
-  } else {
-    if (lane == 0) w.res[0] = 0;
-    nres = 1;
-    __syncwarp();
-    for (uint32_t st = 1; nres < R && st < T; st++) {
-      const Ent3 p = w.tmp[st];
-      bool occ = false;
-      for (uint32_t j = lane; j < nres; j += 32) {
-        const Ent3 r = w.tmp[w.res[j]];
-        const float djk = w.D[r.slot * S + p.slot];
-        occ |= (r.i == p.i) || (a.ssg ? ssg_occludes(p.d, r.d, djk, a.threshold) : (djk < p.d));
-      }
-      if (!__any_sync(FULL, occ)) {
-        if (lane == 0) w.res[nres] = st;
-        nres++;
-      }
-      __syncwarp();
-    }
+    // the slots of entries that left (and s's, if it was not taken) are free;
+    // those of pending vectors stay taken
+    r.free = (r.free | old_slots | (1ull << fs)) & ~used(r);
   }
-  // des_pool[t] = result[t] for t < result.size() (refine.cpp:527-530,
-  // 943-946, 706-712).  Vamana results always hold R entries; an NSG result
-  // may be shorter and then, with no sentinel written, the old entries at
-  // positions result.size()..R-1 stay in the row; SSG writes the sentinel.
-  for (uint32_t j = lane; j < nres; j += 32) w.row[j] = w.tmp[w.res[j]];
-  __syncwarp();
-  kept = nsg && nres == R && !any_tie;
-  if (a.vamana || a.ssg) rs = nres;  // SSG writes a sentinel after a short result
-  __syncwarp();
+};
+
+__device__ __forceinline__ uint32_t ii_acquire(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
 
-__device__ void ii_load_row(IIWarp &w, const uint32_t *ids, const float *dist, uint32_t deg, int lane) {
-  for (uint32_t j = lane; j < deg; j += 32) w.row[j] = Ent3{dist[j], ids[j], INVALID};
-  __syncwarp();
-}
-
-// forward: each node of this level applies the insertions from lower ids
-// (senders m < n whose row at their turn lists n), then snapshots its row
-__global__ void __launch_bounds__(II_WARPS * 32) k_ii_forward(IIArgs a, uint32_t vs) {
+// Forward: every node applies the insertions from lower ids (senders m < n
+// whose row at their turn lists n), in id order, and publishes its row at its
+// turn.  One cooperative launch: the warps, all resident, take nodes in id
+// order and wait for a sender's flag where it is not up yet -- a sender has a
+// lower id, so a running or finished warp holds it and every wait ends (each
+// is bounded all the same, and a warp that gives up raises the status word
+// the other waits look at).  Bound by the longest chains (a hub's re-prunes,
+// one after the other).  A launch per dependency level, with a barrier after
+// each level's slowest node, took 62 ms on the 200k x 128 NSG link and 79 ms
+// on two 20k x 96 Vamana passes; this takes 10.2 ms and 12.5 ms (the backward
+// launches 8.3 -> 4.6 and 7.5 -> 5.0 ms).
+template <int MODE, bool I8>
+__global__ void __launch_bounds__(II_WARPS * 32) k_ii_forward(IIArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  IIWarp &w = ii_carve(smem, warp, a.R, vs);
-  for (uint32_t t = blockIdx.x * II_WARPS + warp; t < a.nn; t += gridDim.x * II_WARPS) {
-    const uint32_t n = a.nodes[t];
-    uint32_t rs = a.p_deg[n];
-    ii_load_row(w, a.p_ids + (size_t)n * a.R, a.p_dist + (size_t)n * a.R, rs, lane);
-    bool dvalid = false, kept = false;
+  const II<I8> t{a, ii_carve(smem + (size_t)warp * ii_warp_bytes(a.R, a.cs, a.spare), a.R, a.spare), lane};
+  const uint32_t R = a.R;
+  while (true) {
+    uint32_t n = 0;
+    if (lane == 0) n = atomicAdd(a.next, 1u);
+    n = __shfl_sync(FULL, n, 0);
+    if (n >= a.n) return;
+    IIRow r;
+    t.load(r, a.p_ids + (size_t)n * R, a.p_dist + (size_t)n * R, a.p_deg[n], MODE == 1);
     const uint32_t off = a.req_off[n], cnt = a.req_cnt[n];
-    for (uint32_t r = 0; r < cnt; r++) {
-      const uint32_t m = (uint32_t)(a.req[off + r] >> 32);
-      // each position of n in m's row at m's turn sends one insertion
-      // (an NSG row can list an id twice), in position order
-      const uint32_t mdeg = a.s_deg[m];
-      for (uint32_t b = 0; b < mdeg; b += 32) {
-        const uint32_t j = b + lane;
-        unsigned hits = __ballot_sync(FULL, j < mdeg && a.s_ids[(size_t)m * a.R + j] == n);
-        while (hits) {
-          const uint32_t pos = b + __ffs(hits) - 1;
-          hits &= hits - 1;
-          ii_apply(a, w, vs, rs, dvalid, kept, m, a.s_dist[(size_t)m * a.R + pos], pos, lane);
+    uint32_t level = 0;
+    for (uint32_t r0 = 0; r0 < cnt;) {
+      const uint32_t nb = min(II_SPARE, cnt - r0);
+      const uint32_t m = lane < nb ? (uint32_t)(a.req[off + r0 + lane] >> 32) : 0u;
+      uint32_t up = lane < nb ? ii_acquire(a.done + m) : 0u;
+      // the senders that are at hand, in order; the first is waited for
+      if (__shfl_sync(FULL, up, 0) == 0) {
+        bool ok = true;
+        if (lane == 0) {
+          uint32_t polls = 0;
+          while ((up = ii_acquire(a.done + m)) == 0) {
+            if (++polls >= II_POLLS) {
+              set_err(a.status, DEV_TIMEOUT);
+              ok = false;
+              break;
+            }
+            if ((polls & 255u) == 0 && *reinterpret_cast<volatile int *>(a.status) != 0) {
+              ok = false;
+              break;
+            }
+            __nanosleep(40);
+          }
+        }
+        if (!__shfl_sync(FULL, ok, 0)) return;
+      }
+      const uint32_t have = __ffs(~__ballot_sync(FULL, up != 0)) - 1;
+      for (uint32_t k = 0; k < have; k++) level = max(level, __shfl_sync(FULL, up, k));
+      // their rows (read past the L1, which other warps' rows may share lines with)
+      uint32_t mk[II_SPARE], id[II_SPARE][2], dg[II_SPARE], fs[II_SPARE];
+      float ds[II_SPARE][2];
+#pragma unroll
+      for (int k = 0; k < (int)II_SPARE; k++) {
+        mk[k] = __shfl_sync(FULL, m, k);
+        const bool on = k < (int)have;
+        dg[k] = on ? __ldcg(a.s_deg + mk[k]) : 0u;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const uint32_t j = lane + 32 * h;
+          const bool in = on && j < R;
+          id[k][h] = in ? __ldcg(a.s_ids + (size_t)mk[k] * R + j) : INVALID;
+          ds[k][h] = in ? __ldcg(a.s_dist + (size_t)mk[k] * R + j) : 0.f;
         }
       }
+      unsigned hit[II_SPARE][2];
+#pragma unroll
+      for (int k = 0; k < (int)II_SPARE; k++) {
+        hit[k][0] = __ballot_sync(FULL, lane < dg[k] && id[k][0] == n);
+        hit[k][1] = __ballot_sync(FULL, lane + 32 < dg[k] && id[k][1] == n);
+        fs[k] = INVALID;
+        if (k < (int)a.spare && (hit[k][0] | hit[k][1]) && (r.vvalid || r.rs == R)) {
+          fs[k] = __ffsll(r.free) - 1;
+          r.free &= r.free - 1;
+          t.stage(fs[k], mk[k]);
+        }
+      }
+      // each position of n in a sender's row sends one insertion (an NSG row
+      // can list an id twice), in position order
+#pragma unroll
+      for (int k = 0; k < (int)II_SPARE; k++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          unsigned hm = hit[k][h];
+          while (hm) {
+            const int b = __ffs(hm) - 1;
+            hm &= hm - 1;
+            const float sd = __shfl_sync(FULL, ds[k][h], b);
+            t.template apply<MODE>(r, mk[k], sd, (uint32_t)(b + 32 * h), fs[k]);
+            fs[k] = INVALID;
+          }
+        }
+      r0 += have;
     }
-    for (uint32_t j = lane; j < rs; j += 32) {
-      a.s_ids[(size_t)n * a.R + j] = w.row[j].i;
-      a.s_dist[(size_t)n * a.R + j] = w.row[j].d;
+    t.store(r, a.s_ids + (size_t)n * R, a.s_dist + (size_t)n * R);
+    if (lane == 0) {
+      a.s_deg[n] = r.rs;
+      a.s_kept[n] = r.kept;
     }
-    if (lane == 0) a.s_deg[n] = rs;
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) {
+      atomicMax(a.maxlev, level);
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.done + n), "r"(level + 1) : "memory");
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");  // (a vector whose insertion was refused may still be in flight)
     __syncwarp();
   }
 }
 
 // backward: every row applies the insertions from higher ids in id order
-__global__ void __launch_bounds__(II_WARPS * 32) k_ii_backward(IIArgs a, uint32_t vs) {
+template <int MODE, bool I8>
+__global__ void __launch_bounds__(II_WARPS * 32) k_ii_backward(IIArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  IIWarp &w = ii_carve(smem, warp, a.R, vs);
-  for (uint32_t r = blockIdx.x * II_WARPS + warp; r < a.n; r += gridDim.x * II_WARPS) {
-    uint32_t rs = a.s_deg[r];
-    ii_load_row(w, a.s_ids + (size_t)r * a.R, a.s_dist + (size_t)r * a.R, rs, lane);
-    bool dvalid = false, kept = false;
-    const uint32_t off = a.req_off[r], cnt = a.req_cnt[r];
-    for (uint32_t q = 0; q < cnt; q++) {
-      const unsigned long long key = a.req[off + q];
-      const uint32_t m = (uint32_t)(key >> 32), pos = (uint32_t)key;
-      ii_apply(a, w, vs, rs, dvalid, kept, m, a.s_dist[(size_t)m * a.R + pos], pos, lane);
+  const II<I8> t{a, ii_carve(smem + (size_t)warp * ii_warp_bytes(a.R, a.cs, a.spare), a.R, a.spare), lane};
+  const uint32_t R = a.R;
+  while (true) {
+    uint32_t n = 0;
+    if (lane == 0) n = atomicAdd(a.next, 1u);
+    n = __shfl_sync(FULL, n, 0);
+    if (n >= a.n) return;
+    IIRow r;
+    t.load(r, a.s_ids + (size_t)n * R, a.s_dist + (size_t)n * R, a.s_deg[n], MODE == 1 && a.s_kept[n]);
+    const uint32_t off = a.req_off[n], cnt = a.req_cnt[n];
+    for (uint32_t r0 = 0; r0 < cnt; r0 += 32) {
+      const unsigned long long key = r0 + lane < cnt ? a.req[off + r0 + lane] : 0ull;
+      const uint32_t ml = (uint32_t)(key >> 32), pl = (uint32_t)key;
+      const float dl = r0 + lane < cnt ? a.s_dist[(size_t)ml * R + pl] : 0.f;
+      const uint32_t nb = min(32u, cnt - r0);
+      uint32_t nxt = INVALID;  // the slot the next sender's vector goes to
+      for (uint32_t q = 0; q < nb; q++) {
+        const uint32_t m = __shfl_sync(FULL, ml, q), pos = __shfl_sync(FULL, pl, q);
+        const float sd = __shfl_sync(FULL, dl, q);
+        const uint32_t cur = nxt;
+        nxt = INVALID;
+        if (cur != INVALID) t.landed();
+        if (q + 1 < nb && a.spare > 0 && r.vvalid) {
+          nxt = __ffsll(r.free) - 1;
+          r.free &= r.free - 1;
+          t.stage(nxt, __shfl_sync(FULL, ml, q + 1));
+        }
+        t.template apply<MODE>(r, m, sd, pos, cur);
+      }
     }
-    for (uint32_t j = lane; j < rs; j += 32) {
-      a.f_ids[(size_t)r * a.R + j] = w.row[j].i;
-      a.f_dist[(size_t)r * a.R + j] = w.row[j].d;
-    }
-    if (lane == 0) a.f_deg[r] = rs;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncwarp();
+    t.store(r, a.f_ids + (size_t)n * R, a.f_dist + (size_t)n * R);
+    if (lane == 0) a.f_deg[n] = r.rs;
   }
 }
 
@@ -1123,30 +1311,6 @@ __global__ void k_req_fill(uint32_t n, uint32_t R, const uint32_t *ids, const ui
     if (t < n && (fwd ? m < t : m > t))
       req[off[t] + atomicAdd(&cur[t], 1u)] = ((unsigned long long)m << 32) | j;
   }
-}
-
-// level(t) = max(level(t), level(m) + 1) over forward edges of the pruned rows
-__global__ void k_level_relax(uint32_t n, uint32_t R, const uint32_t *ids, const uint32_t *deg, uint32_t *level,
-                              uint32_t *changed) {
-  const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= n) return;
-  const uint32_t lm = level[m];
-  for (uint32_t j = 0; j < deg[m]; j++) {
-    const uint32_t t = ids[(size_t)m * R + j];
-    if (t < n && m < t && level[t] < lm + 1) {
-      atomicMax(&level[t], lm + 1);
-      *changed = 1;
-    }
-  }
-}
-__global__ void k_level_count(uint32_t n, const uint32_t *level, uint32_t *lcnt) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(&lcnt[level[i]], 1u);
-}
-__global__ void k_level_fill(uint32_t n, const uint32_t *level, const uint32_t *loff, uint32_t *lcur,
-                             uint32_t *order) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) order[loff[level[i]] + atomicAdd(&lcur[level[i]], 1u)] = i;
 }
 
 // ---------------------------------------------------------------- centroid
@@ -1591,8 +1755,9 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
     }
   }
   // ---- InterInsert
-  uint32_t *level = c->buf<uint32_t>("lk_level", n, &e);
-  uint32_t *flag = c->buf<uint32_t>("lk_flag", 4, &e);
+  uint32_t *done = c->buf<uint32_t>("lk_done", n, &e);
+  uint32_t *kept = c->buf<uint32_t>("lk_kept", n, &e);
+  uint32_t *iis = c->buf<uint32_t>("lk_iis", 4, &e);  // [0] next node, [1] highest level
   uint32_t *rcnt = c->buf<uint32_t>("lk_rcnt", n, &e);
   uint32_t *roff = c->buf<uint32_t>("lk_roff", n + 1, &e);
   uint32_t *rcur = c->buf<uint32_t>("lk_rcur", n, &e);
@@ -1601,38 +1766,9 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   uint32_t *s_ids = c->buf<uint32_t>("lk_sids", (size_t)n * R, &e);
   float *s_dist = c->buf<float>("lk_sdist", (size_t)n * R, &e);
   uint32_t *s_deg = c->buf<uint32_t>("lk_sdeg", n, &e);
-  uint32_t *order = c->buf<uint32_t>("lk_order", n, &e);
+  uint8_t *pops = c->buf<uint8_t>("lk_pops", 65 * 64, &e);
   WV_CUDA(c, e);
   const int nb = (int)((n + 255) / 256);
-  WV_CUDA(c, cudaMemsetAsync(level, 0, (size_t)n * 4, c->stream));
-  uint32_t iters = 0;
-  while (true) {
-    WV_CUDA(c, cudaMemsetAsync(flag, 0, 4, c->stream));
-    k_level_relax<<<nb, 256, 0, c->stream>>>(n, R, p_ids, p_deg, level, flag);
-    uint32_t ch = 0;
-    WV_CUDA(c, cudaMemcpyAsync(&ch, flag, 4, cudaMemcpyDeviceToHost, c->stream));
-    WV_CUDA(c, cudaStreamSynchronize(c->stream));
-    iters++;
-    if (!ch) break;
-    WV_CHECK(c, iters <= n + 1, WV_ERR_DEVICE, "level relaxation did not converge");
-  }
-  std::vector<uint32_t> hlevel(n);
-  WV_CUDA(c, cudaMemcpyAsync(hlevel.data(), level, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
-  WV_CUDA(c, cudaStreamSynchronize(c->stream));
-  const uint32_t nlev = *std::max_element(hlevel.begin(), hlevel.end()) + 1;
-  S.levels = nlev;
-  uint32_t *lcnt = c->buf<uint32_t>("lk_lcnt", nlev + 1, &e);
-  uint32_t *loff = c->buf<uint32_t>("lk_loff", nlev + 1, &e);
-  uint32_t *lcur = c->buf<uint32_t>("lk_lcur", nlev + 1, &e);
-  uint32_t *scan_l = c->buf<uint32_t>("lk_scanl", scan_scratch_words(nlev + 1), &e);
-  WV_CUDA(c, e);
-  WV_CUDA(c, cudaMemsetAsync(lcnt, 0, (size_t)(nlev + 1) * 4, c->stream));
-  WV_CUDA(c, cudaMemsetAsync(lcur, 0, (size_t)(nlev + 1) * 4, c->stream));
-  k_level_count<<<nb, 256, 0, c->stream>>>(n, level, lcnt);
-  WV_CUDA(c, exclusive_scan_u32(lcnt, loff, nlev + 1, scan_l, c->stream));
-  k_level_fill<<<nb, 256, 0, c->stream>>>(n, level, loff, lcur, order);
-  std::vector<uint32_t> hloff(nlev + 1);
-  WV_CUDA(c, cudaMemcpyAsync(hloff.data(), loff, (size_t)(nlev + 1) * 4, cudaMemcpyDeviceToHost, c->stream));
   // forward request lists from the pruned rows, sorted by sender
   WV_CUDA(c, cudaMemsetAsync(rcnt, 0, (size_t)n * 4, c->stream));
   WV_CUDA(c, cudaMemsetAsync(rcur, 0, (size_t)n * 4, c->stream));
@@ -1641,43 +1777,77 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   k_req_fill<<<nb, 256, 0, c->stream>>>(n, R, p_ids, p_deg, 1, roff, rcur, req);
   int rc = segsort_u64(c, req, roff, rcnt, n);
   if (rc) return rc;
+  std::vector<uint8_t> hpops;
+  if (vamana && !p.clean) {
+    // the order in which libstdc++'s heap steps pop N items of equal keys
+    hpops.assign(65 * 64, 0);
+    for (int N = 1; N <= 64; N++) {
+      HeapIdx h[64];
+      for (int k = 0; k < N; k++) {
+        h[k] = HeapIdx{0.f, (uint32_t)k};
+        stl::push_heap(h, k + 1, HeapIdxLess());
+      }
+      for (int k = 0; k < N; k++) {
+        hpops[64 * N + k] = (uint8_t)h[0].k;
+        stl::pop_heap(h, N - k, HeapIdxLess());
+      }
+    }
+    WV_CUDA(c, cudaMemcpyAsync(pops, hpops.data(), hpops.size(), cudaMemcpyHostToDevice, c->stream));
+  }
+  const bool ii8 = c->base_int && c->base8.p;
   IIArgs ia{};
   ia.base = c->base.as<float>();
+  ia.base8 = ii8 ? c->base8.as<uint8_t>() : nullptr;
+  ia.xnorm = ii8 ? c->xnorm.as<float>() : nullptr;
   ia.d = c->d;
   ia.n = n;
   ia.R = R;
   ia.alpha = p.alpha;
-  ia.vamana = vamana;
   ia.clean = p.clean ? 1 : 0;
-  ia.ssg = ssg;
-  ia.ints = c->base_int && c->d <= 256;
   ia.threshold = threshold;
+  ia.spare = std::min(II_SPARE, LINK_MAX_R - R);
+  // row vectors in shared memory when they fit (an odd multiple of 16 bytes
+  // apart: no bank conflicts), else read where they lie
+  const uint32_t irb = ii8 ? c->d : c->d * 4;
+  ia.cs = irb / 16 % 2 ? irb : irb + 16;
+  if (II_WARPS * ii_warp_bytes(R, ia.cs, ia.spare) > 200 * 1024) ia.cs = 0;
+  ia.pops = pops;
   ia.p_ids = p_ids;
   ia.p_dist = p_dist;
   ia.p_deg = p_deg;
   ia.s_ids = s_ids;
   ia.s_dist = s_dist;
   ia.s_deg = s_deg;
+  ia.s_kept = kept;
+  ia.done = done;
+  ia.next = iis;
+  ia.maxlev = iis + 1;
   ia.req = req;
   ia.req_off = roff;
   ia.req_cnt = rcnt;
   ia.status = c->d_status();
-  // row vectors in shared memory when they fit, else read from global memory
-  uint32_t vs = ((c->d + 3) & ~3u) + 4;
-  if (II_WARPS * ii_warp_bytes(R, vs) > 200 * 1024) vs = 0;
-  const size_t ii_smem = II_WARPS * ii_warp_bytes(R, vs);
-  WV_CUDA(c, cudaFuncSetAttribute(k_ii_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ii_smem));
-  WV_CUDA(c, cudaFuncSetAttribute(k_ii_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ii_smem));
+  const size_t ii_smem = II_WARPS * ii_warp_bytes(R, ia.cs, ia.spare);
+  auto ii_launch = [&](auto kern, bool coop) -> cudaError_t {
+    cudaError_t x = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ii_smem);
+    int per = 0;
+    if (x == cudaSuccess) x = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, II_WARPS * 32, ii_smem);
+    if (x != cudaSuccess) return x;
+    const dim3 grid(std::max(1u, std::min<uint32_t>((uint32_t)(per * c->sms), (n + II_WARPS - 1) / II_WARPS)));
+    void *args[] = {&ia};
+    if (coop) return cudaLaunchCooperativeKernel((const void *)kern, grid, dim3(II_WARPS * 32), args, ii_smem, c->stream);
+    return cudaLaunchKernel((const void *)kern, grid, dim3(II_WARPS * 32), args, ii_smem, c->stream);
+  };
+  WV_CUDA(c, cudaMemsetAsync(done, 0, (size_t)n * 4, c->stream));
+  WV_CUDA(c, cudaMemsetAsync(iis, 0, 16, c->stream));
+  if (ssg) WV_CUDA(c, ii8 ? ii_launch(k_ii_forward<2, true>, true) : ii_launch(k_ii_forward<2, false>, true));
+  else if (vamana) WV_CUDA(c, ii8 ? ii_launch(k_ii_forward<0, true>, true) : ii_launch(k_ii_forward<0, false>, true));
+  else WV_CUDA(c, ii8 ? ii_launch(k_ii_forward<1, true>, true) : ii_launch(k_ii_forward<1, false>, true));
+  rc = check_device_status(c, "inter-insert");
+  if (rc) return rc;
+  uint32_t maxlev = 0;
+  WV_CUDA(c, cudaMemcpyAsync(&maxlev, iis + 1, 4, cudaMemcpyDeviceToHost, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
-  for (uint32_t t = 0; t < nlev; t++) {
-    const uint32_t cnt = hloff[t + 1] - hloff[t];
-    if (!cnt) continue;
-    ia.nodes = order + hloff[t];
-    ia.nn = cnt;
-    const int blocks = (int)std::min<uint32_t>((cnt + II_WARPS - 1) / II_WARPS, (uint32_t)c->sms * 16);
-    k_ii_forward<<<blocks, II_WARPS * 32, ii_smem, c->stream>>>(ia, vs);
-  }
-  WV_CUDA(c, cudaGetLastError());
+  S.levels = maxlev + 1;
   // backward request lists from the snapshots, sorted by sender
   WV_CUDA(c, cudaMemsetAsync(rcnt, 0, (size_t)n * 4, c->stream));
   WV_CUDA(c, cudaMemsetAsync(rcur, 0, (size_t)n * 4, c->stream));
@@ -1693,8 +1863,10 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   ia.f_ids = c->fg_ids.as<uint32_t>();
   ia.f_dist = c->fg_dist.as<float>();
   ia.f_deg = c->fg_deg.as<uint32_t>();
-  k_ii_backward<<<c->sms * 16, II_WARPS * 32, ii_smem, c->stream>>>(ia, vs);
-  WV_CUDA(c, cudaGetLastError());
+  WV_CUDA(c, cudaMemsetAsync(iis, 0, 16, c->stream));
+  if (ssg) WV_CUDA(c, ii8 ? ii_launch(k_ii_backward<2, true>, false) : ii_launch(k_ii_backward<2, false>, false));
+  else if (vamana) WV_CUDA(c, ii8 ? ii_launch(k_ii_backward<0, true>, false) : ii_launch(k_ii_backward<0, false>, false));
+  else WV_CUDA(c, ii8 ? ii_launch(k_ii_backward<1, true>, false) : ii_launch(k_ii_backward<1, false>, false));
   rc = check_device_status(c, "inter-insert");
   if (rc) return rc;
   c->fg_w = R;
