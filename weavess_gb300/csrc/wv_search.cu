@@ -161,7 +161,9 @@ __device__ void sort_seeds(WarpSmem &s, int L, uint32_t hwords, uint32_t *gscrat
 
 
 __device__ __forceinline__ float cand_dist(const SearchArgs &a, bool ints, uint32_t my, int cnt, const float *qv,
-                                           int lane, float qn) {
+                                           uint4 qc, int lane, float qn) {
+  // bytes of integer data: the exact value, as FP32 and bf16 rows give it
+  if (ints && a.base8 && a.storage != 2) return rows_dist_i8(a.base8, a.xnorm, a.d, my, cnt, qc, qn, lane);
   if (a.storage != 0)
     // the norm form unless integer data at d > 128 (where only the
     // difference form stays exact)
@@ -193,13 +195,13 @@ __device__ __forceinline__ float shifted_seed_dist(const float *__restrict__ bas
 //   marked visited, and every visited (id, dist) -- the seeds in drawn order,
 //   then each newly visited id in visit order -- is appended to the query's
 //   visit list (vis, vcap apart, vlimit entries kept, count in vcnt).
-template <bool BUILD, int W>
+template <bool BUILD>
 __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t wbytes = warp_smem_bytes(a.d, a.Lmax, a.cap, a.hcap);
   WarpSmem s = carve(smem + warp * wbytes, a.d, a.Lmax, a.cap, a.hcap);
-  const uint32_t slot = blockIdx.x * W + warp;
+  const uint32_t slot = blockIdx.x * (blockDim.x >> 5) + warp;
   const uint32_t hs = hash_slots(a.Lmax, a.hcap);
   const uint32_t nq = a.nq_dev ? *a.nq_dev : a.nq;
   Visited vis;
@@ -238,6 +240,8 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
     for (int o = 16; o > 0; o >>= 1) qn += __shfl_xor_sync(FULL, qn, o);
     // integer base and query: any summation order gives the reference's value
     const bool ints = a.int_exact && a.d <= 256 && __all_sync(FULL, qint);
+    __syncwarp();
+    const uint4 qc = ints && a.base8 ? query_chunk_i8(s.qv, a.d, lane) : make_uint4(0u, 0u, 0u, 0u);
     // ---- seeds (SearchEntryInner): distances in drawn order, as (dist, id)
     // pairs over the pool region ----
     const uint32_t *seeds = a.seeds + (size_t)q * a.seed_stride;
@@ -253,7 +257,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         id = 0;
       }
       const float dist = (!BUILD && a.seed_shift) ? (lane < cnt ? shifted_seed_dist(a.base, a.d, id, s.qv) : 0.f)
-                                                 : cand_dist(a, ints, id, cnt, s.qv, lane, qn);
+                                                 : cand_dist(a, ints, id, cnt, s.qv, qc, lane, qn);
       if (lane < cnt) {
         drawn[b + lane] = DI{dist, id};
         if (BUILD && nvis + lane < a.vlimit) vis_out[nvis + lane] = DI{dist, id};
@@ -341,7 +345,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         const int cnt = (int)min(32u, nfresh - b);
         const uint32_t raw = lane < cnt ? s.si[b + lane] : 0u;
         const uint32_t my = raw & ID_MASK;
-        const float dist = cand_dist(a, ints, my, cnt, s.qv, lane, qn);
+        const float dist = cand_dist(a, ints, my, cnt, s.qv, qc, lane, qn);
         if (BUILD) {
           if (lane < cnt && nvis + lane < a.vlimit) vis_out[nvis + lane] = DI{dist, my};
           nvis += cnt;
@@ -477,8 +481,9 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
       for (int b = 0; b < R; b += 32) {
         const int cnt = min(32, R - b);
         const uint32_t id = lane < cnt ? (pi[b + lane] & ID_MASK) : 0u;
-        const float ex = ints ? batch_dist<true>(a.base, a.d, id, cnt, s.qv, lane, qn, a.d <= 128 ? a.xnorm : nullptr)
-                              : batch_dist<false>(a.base, a.d, id, cnt, s.qv, lane);
+        const float ex = ints && a.base8 ? rows_dist_i8(a.base8, a.xnorm, a.d, id, cnt, qc, qn, lane)
+                         : ints          ? batch_dist<true>(a.base, a.d, id, cnt, s.qv, lane, qn, a.d <= 128 ? a.xnorm : nullptr)
+                                         : batch_dist<false>(a.base, a.d, id, cnt, s.qv, lane);
         if (lane < cnt) {
           xd[b + lane] = ex;
           xi[b + lane] = id;
@@ -518,18 +523,12 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   }
 }
 
-template <bool B, int W>
-cudaError_t launch_w(const SearchArgs &a, int blocks, size_t smem, cudaStream_t stream) {
-  k_search<B, W><<<blocks, W * 32, smem, stream>>>(a);
-  return cudaGetLastError();
-}
-
-template <bool B, int W>
-int max_blocks_w(size_t smem) {
-  if (cudaFuncSetAttribute(k_search<B, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+template <bool B>
+int max_blocks(int W, size_t smem) {
+  if (cudaFuncSetAttribute(k_search<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return -1;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<B, W>, W * 32, smem) != cudaSuccess) return -1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<B>, W * 32, smem) != cudaSuccess) return -1;
   return per_sm;
 }
 
@@ -556,14 +555,9 @@ int search_grid(uint32_t d, uint32_t Lmax, uint32_t cap, int device, SearchShape
   if (!shape_ok(sh)) return 0;
   const size_t smem = search_block_smem(d, Lmax, cap, sh);
   if (smem > 227 * 1024) return 0;
-  int per_sm = -1;
-  // (the build variant exists in the default shape only)
-  switch (sh.wpb) {
-    case 1: per_sm = max_blocks_w<false, 1>(smem); break;
-    case 2: per_sm = max_blocks_w<false, 2>(smem); break;
-    case 4: per_sm = std::min(max_blocks_w<false, 4>(smem), max_blocks_w<true, 4>(smem)); break;
-    default: per_sm = max_blocks_w<false, 8>(smem); break;
-  }
+  // (the build variant runs in the default shape only)
+  int per_sm = max_blocks<false>(sh.wpb, smem);
+  if (sh.wpb == WARPS) per_sm = std::min(per_sm, max_blocks<true>(sh.wpb, smem));
   if (per_sm <= 0) {
     cudaGetLastError();
     return 0;
@@ -639,13 +633,10 @@ cudaError_t launch_search(const SearchArgs &a, SearchShape sh, int blocks, cudaS
   b.hcap = sh.hcap;
   b.wide_hash = sh.wide ? 1 : 0;
   const size_t smem = search_block_smem(a.d, a.Lmax, a.cap, sh);
-  if (a.vis) return sh.wpb == WARPS ? launch_w<true, WARPS>(b, blocks, smem, stream) : cudaErrorInvalidValue;
-  switch (sh.wpb) {
-    case 1: return launch_w<false, 1>(b, blocks, smem, stream);
-    case 2: return launch_w<false, 2>(b, blocks, smem, stream);
-    case 4: return launch_w<false, 4>(b, blocks, smem, stream);
-    default: return launch_w<false, 8>(b, blocks, smem, stream);
-  }
+  if (a.vis && sh.wpb != WARPS) return cudaErrorInvalidValue;
+  if (a.vis) k_search<true><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  else k_search<false><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  return cudaGetLastError();
 }
 cudaError_t launch_search_exact(const SearchArgs &a, int blocks, cudaStream_t stream) {
   return launch_search(a, SearchShape{}, blocks, stream);

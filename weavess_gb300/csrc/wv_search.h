@@ -14,6 +14,7 @@ struct SearchArgs {
   const uint32_t *gids;  // graph rows, width gw
   const uint32_t *gdeg;
   uint32_t gw;
+  const uint8_t *base8;  // integer base (d a multiple of 16 up to 256): the rows as bytes, or null
   const float *queries;  // nq x d
   uint32_t nq;
   const uint32_t *nq_dev;  // if set, the query count is read from here (captured launches)
