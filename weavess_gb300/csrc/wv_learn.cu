@@ -28,6 +28,7 @@
 #include <string>
 #include <vector>
 
+#include "wv_colsum.cuh"
 #include "wv_common.cuh"
 #include "wv_ctx.h"
 #include "wv_learn.h"
@@ -100,7 +101,8 @@ __global__ void k_gather_norm(const float *x, const uint32_t *rows, uint32_t B, 
 // softmax cross-entropy on O[:, :C] and squared error on O[:, C];
 // dO = d(mean loss) / dO; loss sums into loss[0] (ce) and loss[1] (mse)
 __global__ void k_loss_grad(const float *O, uint32_t B, uint32_t C, const uint32_t *yc, const float *yr,
-                            const uint32_t *rows, float lam, float *dO, __nv_bfloat16 *dOb, float *loss) {
+                            const uint32_t *rows, float lam, float *dO, __nv_bfloat16 *dOb, uint32_t ldb,
+                            float *loss) {
   const int lane = threadIdx.x & 31;
   const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (b >= B) return;
@@ -118,13 +120,13 @@ __global__ void k_loss_grad(const float *O, uint32_t B, uint32_t C, const uint32
     const float p = expf(o[c] - m) / se;
     const float g = (p - (c == y ? 1.f : 0.f)) / (float)B;
     dO[(size_t)b * W + c] = g;
-    dOb[(size_t)b * W + c] = __float2bfloat16_rn(g);
+    dOb[(size_t)b * ldb + c] = __float2bfloat16_rn(g);
   }
   if (lane == 0) {
     const float e = o[C] - yr[r];
     const float g = 2.f * lam * e / (float)B;
     dO[(size_t)b * W + C] = g;
-    dOb[(size_t)b * W + C] = __float2bfloat16_rn(g);
+    dOb[(size_t)b * ldb + C] = __float2bfloat16_rn(g);
     atomicAdd(&loss[0], (logf(se) + m - o[y]) / (float)B);
     atomicAdd(&loss[1], e * e / (float)B);
   }
@@ -137,15 +139,6 @@ __global__ void k_relu_bwd(const float *dH, const float *H, size_t count, float 
   const float v = H[i] > 0.f ? dH[i] : 0.f;
   dZ[i] = v;
   dZb[i] = __float2bfloat16_rn(v);
-}
-
-// db[n] = sum_b dY[b, n]
-__global__ void k_colsum(const float *dY, uint32_t B, uint32_t N, float *db) {
-  const uint32_t nidx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nidx >= N) return;
-  float s = 0.f;
-  for (uint32_t b = 0; b < B; b++) s += dY[(size_t)b * N + nidx];
-  db[nidx] = s;
 }
 
 __global__ void k_adam(float *p, const float *g, float *m, float *v, size_t count, float lr, float b1, float b2,
@@ -173,17 +166,40 @@ __global__ void k_to_bf16(const float *x, size_t count, __nv_bfloat16 *out) {
   if (i < count) out[i] = __float2bfloat16_rn(x[i]);
 }
 
-// per query: entry cluster(s), beam width and seeds from the model output
+// the ids of `plain` (np of them) that are not in sq[0..t) yet, in order, up
+// to L entries (a warp); returns the new count
+__device__ uint32_t fill_plain(uint32_t *sq, uint32_t t, uint32_t L, const uint32_t *plain, uint32_t np, int lane) {
+  for (uint32_t j0 = 0; t < L && j0 < np; j0 += 32) {
+    __syncwarp();  // sq[0..t) is written
+    const uint32_t id = j0 + lane < np ? plain[j0 + lane] : INVALID;
+    bool dup = j0 + lane >= np;
+    for (uint32_t u = 0; u < t; u++) dup |= sq[u] == id;
+    const unsigned same = __match_any_sync(FULL, id);
+    dup |= (__ffs(same) - 1) != lane;  // of equal ids in these 32 the first is taken
+    const unsigned m = __ballot_sync(FULL, !dup);
+    const uint32_t at = t + __popc(m & ((1u << lane) - 1u));
+    if (!dup && at < L) sq[at] = id;
+    t = min(L, t + (uint32_t)__popc(m));
+  }
+  __syncwarp();
+  return t;
+}
+
+// per query (a warp each): entry cluster(s), beam width and seeds from the
+// model output.  A thread per query wrote its seeds one by one, 41 us for
+// 10,000 queries.
 __global__ void k_learn_seeds(const float *O, uint32_t nq, uint32_t C, const uint32_t *lists, uint32_t SL,
                               const uint32_t *llen, float margin, uint32_t Lmin, uint32_t Lmax, float fallback_p,
                               uint32_t L_plain, const uint32_t *plain_seeds, uint32_t *seeds, uint32_t stride,
                               uint32_t *Lq, uint32_t K, uint32_t *used_fallback) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (q >= nq) return;
   const float *o = O + (size_t)q * (C + 1);
-  uint32_t c1 = 0, c2 = 0;
+  // the two best clusters (ties: the lower number first)
   float v1 = -3.4e38f, v2 = -3.4e38f;
-  for (uint32_t c = 0; c < C; c++) {
+  uint32_t c1 = 0, c2 = 0;
+  for (uint32_t c = lane; c < C; c += 32) {
     const float v = o[c];
     if (v > v1) {
       v2 = v1;
@@ -195,56 +211,70 @@ __global__ void k_learn_seeds(const float *O, uint32_t nq, uint32_t C, const uin
       c2 = c;
     }
   }
-  float se = 0.f;
-  for (uint32_t c = 0; c < C; c++) se += expf(o[c] - v1);
-  const float p1 = 1.f / se;
-  uint32_t *sq = seeds + (size_t)q * stride;
-  if (plain_seeds && p1 < fallback_p) {  // the plain search
-    for (uint32_t j = 0; j < L_plain; j++) sq[j] = plain_seeds[(size_t)q * L_plain + j];
-    Lq[q] = L_plain;
-    atomicAdd(used_fallback, 1u);
-    return;
+  for (int s = 16; s > 0; s >>= 1) {
+    const float w1 = __shfl_xor_sync(FULL, v1, s), w2 = __shfl_xor_sync(FULL, v2, s);
+    const uint32_t d1 = __shfl_xor_sync(FULL, c1, s), d2 = __shfl_xor_sync(FULL, c2, s);
+    const bool other = w1 > v1 || (w1 == v1 && d1 < c1);
+    const float lv = other ? v1 : w1;  // the loser of the firsts and the winner's second
+    const uint32_t lc = other ? c1 : d1;
+    const float sv = other ? w2 : v2;
+    const uint32_t sc = other ? d2 : c2;
+    if (other) {
+      v1 = w1;
+      c1 = d1;
+    }
+    const bool loser = lv > sv || (lv == sv && lc < sc);
+    v2 = loser ? lv : sv;
+    c2 = loser ? lc : sc;
   }
-  float lf = exp2f(o[C]) * margin;
+  uint32_t *sq = seeds + (size_t)q * stride;
+  if (plain_seeds && fallback_p > 0.f) {
+    // softmax of the best: the terms summed in cluster order
+    float se = 0.f;
+    for (uint32_t b = 0; b < C; b += 32) {
+      const float ex = b + lane < C ? expf(o[b + lane] - v1) : 0.f;
+      for (uint32_t k = 0; k < min(32u, C - b); k++) se += __shfl_sync(FULL, ex, k);
+    }
+    if (1.f / se < fallback_p) {  // the plain search
+      for (uint32_t j = lane; j < L_plain; j += 32) sq[j] = plain_seeds[(size_t)q * L_plain + j];
+      if (lane == 0) {
+        Lq[q] = L_plain;
+        atomicAdd(used_fallback, 1u);
+      }
+      return;
+    }
+  }
+  const float lf = exp2f(o[C]) * margin;
   uint32_t L = (uint32_t)ceilf(lf);
   L = max(Lmin, min(Lmax, max(L, K)));
-  Lq[q] = L;
   // seeds: the first cluster's list; when the second cluster is close in
-  // probability (p2 > p1 / 4), alternate between the two lists
+  // probability (p2 > p1 / 4), the two lists alternate until one ends
   const bool two = (expf(v2 - v1) > 0.25f) && llen[c2] > 0;
-  uint32_t a = 0, b = 0, t = 0;
-  while (t < L) {
-    const bool from1 = !two || (t & 1) == 0 || b >= llen[c2];
-    if (from1 && a < llen[c1]) sq[t++] = lists[(size_t)c1 * SL + a++];
-    else if (two && b < llen[c2]) sq[t++] = lists[(size_t)c2 * SL + b++];
-    else break;
+  const uint32_t n1 = llen[c1], n2 = two ? llen[c2] : 0u, both = min(n1, n2);
+  uint32_t t = min(L, n1 + n2);
+  for (uint32_t j = lane; j < t; j += 32) {
+    const bool alt = j < 2 * both;
+    const bool first = alt ? (j & 1) == 0 : n1 > n2;
+    sq[j] = lists[(size_t)(first ? c1 : c2) * SL + (alt ? j / 2 : j - both)];
   }
   // short lists: fill with the plain seeds not already taken
-  for (uint32_t j = 0; plain_seeds && t < L && j < L_plain; j++) {
-    const uint32_t id = plain_seeds[(size_t)q * L_plain + j];
-    bool dup = false;
-    for (uint32_t u = 0; u < t && !dup; u++) dup = sq[u] == id;
-    if (!dup) sq[t++] = id;
-  }
-  Lq[q] = t;
+  if (plain_seeds) t = fill_plain(sq, t, L, plain_seeds + (size_t)q * L_plain, L_plain, lane);
+  if (lane == 0) Lq[q] = t;
 }
 
-// seeds of the label cluster at a fixed beam (trace labelling)
+// seeds of the label cluster at a fixed beam (trace labelling), a warp per
+// query
 __global__ void k_cluster_seeds(const uint32_t *label, uint32_t nq, const uint32_t *lists, uint32_t SL,
                                 const uint32_t *llen, uint32_t L, const uint32_t *plain_seeds, uint32_t Lp,
                                 uint32_t *seeds) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (q >= nq) return;
   const uint32_t c = label[q];
   uint32_t *sq = seeds + (size_t)q * L;
-  uint32_t t = 0;
-  for (; t < L && t < llen[c]; t++) sq[t] = lists[(size_t)c * SL + t];
-  for (uint32_t j = 0; t < L && j < Lp; j++) {
-    const uint32_t id = plain_seeds[(size_t)q * Lp + j];
-    bool dup = false;
-    for (uint32_t u = 0; u < t && !dup; u++) dup = sq[u] == id;
-    if (!dup) sq[t++] = id;
-  }
+  const uint32_t t = min(L, llen[c]);
+  for (uint32_t j = lane; j < t; j += 32) sq[j] = lists[(size_t)c * SL + j];
+  fill_plain(sq, t, L, plain_seeds + (size_t)q * Lp, Lp, lane);
 }
 
 }  // namespace
@@ -298,6 +328,9 @@ void learn_free(wv_ctx *c) {
 
 namespace {
 
+// rows of dOb start on 16 bytes (the GEMM's 16-byte loads)
+inline uint32_t pad8(uint32_t x) { return (x + 7) & ~7u; }
+
 struct Work {  // activations and gradients of one batch
   __nv_bfloat16 *Xb, *H1b, *H2b, *dOb, *dZ2b, *dZ1b;
   float *H1, *H2, *O, *dO, *dH2, *dZ2, *dH1, *dZ1;
@@ -317,7 +350,7 @@ int alloc_work(wv_ctx *c, uint32_t B, uint32_t D, uint32_t C, Work &w, const std
   w.H2 = c->buf<float>(nm("H2").c_str(), (size_t)B * HID, &e);
   w.O = c->buf<float>(nm("O").c_str(), (size_t)B * (C + 1), &e);
   if (grads) {
-    w.dOb = c->buf<__nv_bfloat16>(nm("dOb").c_str(), (size_t)B * (C + 1), &e);
+    w.dOb = c->buf<__nv_bfloat16>(nm("dOb").c_str(), (size_t)B * pad8(C + 1), &e);
     w.dZ2b = c->buf<__nv_bfloat16>(nm("dZ2b").c_str(), (size_t)B * HID, &e);
     w.dZ1b = c->buf<__nv_bfloat16>(nm("dZ1b").c_str(), (size_t)B * HID, &e);
     w.dO = c->buf<float>(nm("dO").c_str(), (size_t)B * (C + 1), &e);
@@ -372,21 +405,22 @@ int backward(wv_ctx *c, LearnState &S, const uint32_t *yc, const float *yr, cons
              float lam, Work &w, float *loss) {
   const __nv_bfloat16 *Pb = S.Pb.as<__nv_bfloat16>();
   float *G = S.G.as<float>();
-  const uint32_t W = S.C + 1;
-  k_loss_grad<<<nblk((size_t)B * 32), 256, 0, c->stream>>>(w.O, B, S.C, yc, yr, rows, lam, w.dO, w.dOb, loss);
+  const __nv_bfloat16 *Pt = S.PbT.as<__nv_bfloat16>();
+  const uint32_t W = S.C + 1, Wb = pad8(W);
+  k_loss_grad<<<nblk((size_t)B * 32), 256, 0, c->stream>>>(w.O, B, S.C, yc, yr, rows, lam, w.dO, w.dOb, Wb, loss);
   // layer 3
-  WV_CUDA(c, gemm_bf16_umma(gm(w.H2b, 1, HID, w.dOb, W, 1, G + S.oW3, nullptr, W, nullptr, 0, HID, W, B), c->d_status(), c->stream));
-  k_colsum<<<nblk(W), 256, 0, c->stream>>>(w.dO, B, W, G + S.ob3);
-  WV_CUDA(c, gemm_bf16_umma(gm(w.dOb, W, 1, Pb + S.oW3, 1, W, w.dH2, nullptr, HID, nullptr, 0, B, HID, W), c->d_status(), c->stream));
+  WV_CUDA(c, gemm_bf16_umma(gm(w.H2b, 1, HID, w.dOb, Wb, 1, G + S.oW3, nullptr, W, nullptr, 0, HID, W, B), c->d_status(), c->stream));
+  WV_CUDA(c, col_chain(w.dO, B, W, false, G + S.ob3, c->stream));
+  WV_CUDA(c, gemm_bf16_umma(gm(w.dOb, Wb, 1, Pt + S.oW3, HID, 1, w.dH2, nullptr, HID, nullptr, 0, B, HID, W), c->d_status(), c->stream));
   k_relu_bwd<<<nblk((size_t)B * HID), 256, 0, c->stream>>>(w.dH2, w.H2, (size_t)B * HID, w.dZ2, w.dZ2b);
   // layer 2
   WV_CUDA(c, gemm_bf16_umma(gm(w.H1b, 1, HID, w.dZ2b, HID, 1, G + S.oW2, nullptr, HID, nullptr, 0, HID, HID, B), c->d_status(), c->stream));
-  k_colsum<<<nblk(HID), 256, 0, c->stream>>>(w.dZ2, B, HID, G + S.ob2);
+  WV_CUDA(c, col_chain(w.dZ2, B, HID, false, G + S.ob2, c->stream));
   WV_CUDA(c, gemm_bf16_umma(gm(w.dZ2b, HID, 1, Pb + S.oW2, 1, HID, w.dH1, nullptr, HID, nullptr, 0, B, HID, HID), c->d_status(), c->stream));
   k_relu_bwd<<<nblk((size_t)B * HID), 256, 0, c->stream>>>(w.dH1, w.H1, (size_t)B * HID, w.dZ1, w.dZ1b);
   // layer 1
   WV_CUDA(c, gemm_bf16_umma(gm(w.Xb, 1, S.D, w.dZ1b, HID, 1, G + S.oW1, nullptr, HID, nullptr, 0, S.D, HID, B), c->d_status(), c->stream));
-  k_colsum<<<nblk(HID), 256, 0, c->stream>>>(w.dZ1, B, HID, G + S.ob1);
+  WV_CUDA(c, col_chain(w.dZ1, B, HID, false, G + S.ob1, c->stream));
   WV_CUDA(c, cudaGetLastError());
   return WV_OK;
 }
@@ -556,7 +590,7 @@ int learn_fit(wv_ctx *c, const float *train_q, uint32_t nt, const LearnParams &p
   std::vector<uint32_t> hg((size_t)nt * 10);
   for (uint32_t L : grid) {
     if (L >= n || L > S.SL + p.L_trace) break;
-    k_cluster_seeds<<<nblk(nt), 256, 0, c->stream>>>(dlab, nt, S.lists.as<uint32_t>(), S.SL, S.llen.as<uint32_t>(), L,
+    k_cluster_seeds<<<nblk(nt, 8), 256, 0, c->stream>>>(dlab, nt, S.lists.as<uint32_t>(), S.SL, S.llen.as<uint32_t>(), L,
                                                     pseeds, p.L_trace, gseeds);
     rc = search_dev(c, dq, nt, gseeds, L, nullptr, L, L, 10, gans, nullptr);
     if (rc) return rc;
@@ -711,7 +745,7 @@ int learn_search(wv_ctx *c, const float *dq, uint32_t nq, uint32_t K, uint32_t *
   rc = forward(c, S, dq, nullptr, nq, w);
   if (rc) return rc;
   WV_CUDA(c, cudaMemsetAsync(fb, 0, 4, c->stream));
-  k_learn_seeds<<<nblk(nq, 128), 128, 0, c->stream>>>(w.O, nq, S.C, S.lists.as<uint32_t>(), S.SL, S.llen.as<uint32_t>(),
+  k_learn_seeds<<<nblk(nq, 4), 128, 0, c->stream>>>(w.O, nq, S.C, S.lists.as<uint32_t>(), S.SL, S.llen.as<uint32_t>(),
                                                  S.margin, S.Lmin, S.Lmax, S.fallback_p, S.L_plain, d_plain_seeds,
                                                  seeds, stride, Lq, K, fb);
   WV_CUDA(c, cudaGetLastError());
@@ -759,7 +793,7 @@ int learn_enqueue(wv_ctx *c, const char *pfx, const float *dq, uint32_t nq_max, 
   rc = forward(c, S, dq, nullptr, nq_max, w);
   if (rc) return rc;
   WV_CUDA(c, cudaMemsetAsync(fb, 0, 4, c->stream));
-  k_learn_seeds<<<nblk(nq_max, 128), 128, 0, c->stream>>>(
+  k_learn_seeds<<<nblk(nq_max, 4), 128, 0, c->stream>>>(
       w.O, nq_max, S.C, S.lists.as<uint32_t>(), S.SL, S.llen.as<uint32_t>(), S.margin, S.Lmin, S.Lmax, S.fallback_p,
       S.L_plain, d_plain_seeds, seeds, stride, Lq, K, fb);
   WV_CUDA(c, cudaGetLastError());
