@@ -40,6 +40,7 @@
 
 #include "warp_sort.cuh"
 #include "wv_bfs.cuh"
+#include "wv_colsum.cuh"
 #include "wv_common.cuh"
 #include "wv_link.h"
 #include "wv_scan.h"
@@ -1313,16 +1314,6 @@ __global__ void k_req_fill(uint32_t n, uint32_t R, const uint32_t *ids, const ui
   }
 }
 
-// ---------------------------------------------------------------- centroid
-// EntryCentroid's FP32 column sums in the reference's order (i ascending)
-__global__ void k_centroid(const float *base, uint32_t n, uint32_t d, float *center) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= d) return;
-  float acc = 0.f;
-  for (uint32_t i = 0; i < n; i++) acc = __fadd_rn(acc, base[(size_t)i * d + j]);
-  center[j] = __fdiv_rn(acc, (float)n);
-}
-
 // ---------------------------------------------------------------- Propagation2
 // ComponentCandidatePropagation2::CandidateInner (component_candidate.cpp:90-109):
 // the pool takes the unseen neighbours of the node's neighbours, walking the
@@ -1601,8 +1592,8 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   // (its RefineInner leaves the entry step out) and draws no rand() here
   uint32_t ep = 0;
   if (!ssg) {
-  k_centroid<<<(c->d + 127) / 128, 128, 0, c->stream>>>(c->base.as<float>(), n, c->d, center);
-  WV_CUDA(c, cudaGetLastError());
+  // EntryCentroid's FP32 column sums in the reference's order (i ascending)
+  WV_CUDA(c, col_chain(c->base.as<float>(), n, c->d, true, center, c->stream));
   ep = (uint32_t)c->rnd.next() % n;
   if (p.entry_L == 0) {
     ep = 0;  // get_neighbors with L = 0 leaves retset[0] value-initialised
