@@ -481,9 +481,14 @@ __global__ void k_bucket_apply(Nnd s, const uint32_t *boff, const uint32_t *bcnt
 // a single cursor and one per offer to group them had bound the join.  What
 // bounds it now: latency between a node's short phases (lists, rows, tile,
 // counts, entries) at 16 warps per SM.  Integer rows come from the byte copy
-// (128 bytes a row at d = 128): seven joins of 100k x 128 (S 10, L 40, R 100)
-// take 12.2 ms, with the FP32 rows, the tcgen05 Gram tile and the two atomics
-// 28.6 ms; six of 60k x 96 real-valued (FP32) 14.3 ms against 18.6 ms.
+// (128 bytes a row at d = 128), widened to FP16 once where they are staged
+// (not at every fragment, a third of the tile's instructions) and read by
+// ldmatrix; the offers are counted and written by a lane per target, without
+// a vote per 32 pairs.  The 100k x 128 build (S 10, L 40, R 100) takes
+// 31.2 ms; 33.2 ms with fragments widened on the fly and votes; its seven
+// joins had been 28.6 ms of 82 with the FP32 rows, the tcgen05 Gram tile and
+// the two atomics.  Six joins of 60k x 96 real-valued (FP32): 14.5 ms
+// against 18.6 ms.
 struct JoinOut {
   uint2 *ent;                  // {distance bits, candidate id}
   uint16_t *eq;                // the candidate's position in the node's list (new ++ old): the replay's key
@@ -499,15 +504,15 @@ struct JoinCfg {
   uint32_t gcap;   // floats of G in shared memory; larger tiles take the block's slab of gscr
   float *gscr;
   size_t gslab;
-  uint32_t *lscr;  // the node's lists (4 (capn + capo) words per block) when they do not fit shared memory
+  uint32_t *lscr;  // the node's lists (4 + warps words per entry and block) when they do not fit shared memory
 };
 
 constexpr int J_THREADS = 256;
 constexpr int J_TI = 16;  // FP32: new rows per i tile
 constexpr int J_TJ = 64;  // FP32: rows per j tile (new ++ old); fewer for long rows (the tile must fit shared memory)
 constexpr int JI_THREADS = 128;       // integer rows
-constexpr uint32_t JI_ROWS = 128;     // integer rows staged at once (all of a node's rows, or a 64 x 64 tile)
-constexpr uint32_t J_GCAP = 4096;     // floats of G in shared memory
+constexpr uint32_t JI_ROWS = 96;      // integer rows staged at once (all of a node's rows, or a 48 x 48 tile)
+constexpr uint32_t J_GCAP = 3072;     // floats of G in shared memory
 
 // occurrences of every id in the lists of nodes [n0, n1), a warp per node,
 // and the largest tile a node needs
@@ -531,11 +536,11 @@ __global__ void k_pool_max(Nnd s, float *mx) {
   if (i < s.n) mx[i] = s.psz[i] > 0 ? s.pool[(size_t)i * s.L].d : __int_as_float(0xff800000);
 }
 
-// row stride of integer rows in shared memory: an odd multiple of 16 bytes
-// (the fragments' word loads then fall into different banks)
-__host__ __device__ inline uint32_t ji_stride(uint32_t d) { return (d / 16) % 2 ? d : d + 16; }
+// row stride of integer rows (FP16) in shared memory: an odd multiple of 16
+// bytes (ldmatrix then reads eight rows from different banks)
+__host__ __device__ inline uint32_t ji_stride(uint32_t d) { return d * 2 + 16; }
 
-// bytes b0..b3 of an integer row as two half pairs: 0x6400 | b is 1024 + b
+// 16 bytes of an integer row as 16 halves: 0x6400 | b is 1024 + b
 __device__ __forceinline__ void ji_halves(uint32_t w, uint32_t &lo, uint32_t &hi) {
   const uint32_t k = 0x64646464u, m = 0x64006400u;
   const uint32_t l = __byte_perm(w, k, 0x4140), h = __byte_perm(w, k, 0x4342);
@@ -547,6 +552,12 @@ __device__ __forceinline__ void ji_mma(float (&c)[4], const uint32_t (&a)[4], ui
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void ji_ldm(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
 
 // distances of rows J (tj of them) x rows I (ti) into G (row j0 + j, column
 // i0 + i): dot products of the integer values on the tensor cores (exact in
@@ -554,39 +565,49 @@ __device__ __forceinline__ void ji_mma(float (&c)[4], const uint32_t (&a)[4], ui
 // 32-bit integers, converted to the FP32 value the reference's sum gives.
 // Rows past ti / tj (in the staging area, whatever it holds) only reach
 // columns / rows of the tile that are dropped.
-__device__ __forceinline__ void ji_tile(const uint8_t *I, const uint8_t *J, uint32_t stride, uint32_t d, uint32_t ti, uint32_t tj,
-                        uint32_t i0, uint32_t j0, const int *nrm, float *G, uint32_t gs, int warp, int nwarps,
-                        int lane) {
+__device__ __forceinline__ void ji_tile(const uint8_t *I, const uint8_t *J, uint32_t stride, uint32_t d, uint32_t ti,
+                                        uint32_t tj, uint32_t i0, uint32_t j0, const int *nrm, float *G, uint32_t gs,
+                                        int warp, int nwarps, int lane) {
   const int g = lane >> 2, j = lane & 3;
+  // ldmatrix: lanes 8 m .. 8 m + 7 give the rows of matrix m.  A: rows 0..7
+  // and 8..15 at k, then at k + 8; B: columns 0..7 at k and k + 8, columns
+  // 8..15 at k and k + 8
+  const uint32_t asm0 = (uint32_t)__cvta_generic_to_shared(J) + (uint32_t)(lane & 15) * stride + (lane >> 4) * 16;
+  const uint32_t bsm0 = (uint32_t)__cvta_generic_to_shared(I) + (uint32_t)((lane & 7) + (lane >> 4) * 8) * stride +
+                        ((lane >> 3) & 1) * 16;
   for (uint32_t mt = warp; mt * 16 < tj; mt += nwarps) {
     for (uint32_t nb = 0; nb < ti; nb += 32) {
       float acc[4][4];
 #pragma unroll
       for (int t = 0; t < 4; t++) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-      const uint32_t *ja = reinterpret_cast<const uint32_t *>(J + (size_t)(mt * 16 + g) * stride) + j;
-      const uint32_t *jb = reinterpret_cast<const uint32_t *>(J + (size_t)(mt * 16 + g + 8) * stride) + j;
-      const uint32_t *ib = reinterpret_cast<const uint32_t *>(I + (size_t)(nb + g) * stride) + j;
-      for (uint32_t k = 0; k < d / 4; k += 4) {
-        uint32_t a[4];
-        ji_halves(ja[k], a[0], a[2]);
-        ji_halves(jb[k], a[1], a[3]);
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-          if (nb + t * 8 < ti) {
-            uint32_t b0, b1;
-            ji_halves(ib[(size_t)t * 2 * stride + k], b0, b1);
-            ji_mma(acc[t], a, b0, b1);
-          }
+      const uint32_t as = asm0 + mt * 16 * stride, bs = bsm0 + nb * stride;
+      const bool two = nb + 16 < ti;
+#pragma unroll 4
+      for (uint32_t k = 0; k < d * 2; k += 32) {
+        uint32_t a[4], b[4], b2[4];
+        ji_ldm(a, as + k);
+        ji_ldm(b, bs + k);
+        ji_mma(acc[0], a, b[0], b[1]);
+        ji_mma(acc[1], a, b[2], b[3]);
+        if (two) {
+          ji_ldm(b2, bs + 16 * stride + k);
+          ji_mma(acc[2], a, b2[0], b2[1]);
+          ji_mma(acc[3], a, b2[2], b2[3]);
         }
       }
 #pragma unroll
-      for (int t = 0; t < 4; t++) {
+      for (int h = 0; h < 2; h++) {
+        const uint32_t jj = mt * 16 + g + h * 8;
+        if (jj >= tj) continue;
+        const int nj = nrm[j0 + jj];
+        float *row = G + (size_t)(j0 + jj) * gs + i0;
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const uint32_t jj = mt * 16 + g + (e >> 1) * 8, ii = nb + t * 8 + 2 * j + (e & 1);
-          if (jj < tj && ii < ti)
-            G[(size_t)(j0 + jj) * gs + i0 + ii] =
-                (float)(nrm[j0 + jj] + nrm[i0 + ii] - 2 * __float2int_rn(acc[t][e]));
+        for (int t = 0; t < 4; t++) {
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const uint32_t ii = nb + t * 8 + 2 * j + e;
+            if (ii < ti) row[ii] = (float)(nj + nrm[i0 + ii] - 2 * __float2int_rn(acc[t][2 * h + e]));
+          }
         }
       }
     }
@@ -603,15 +624,15 @@ __global__ void __launch_bounds__(I8 ? JI_THREADS : J_THREADS)
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ unsigned long long ebase;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const unsigned lt = (1u << lane) - 1u;
   const uint32_t capt = s.capn + s.capo;
   const uint32_t stride = I8 ? ji_stride(s.d) : (((s.d + 3) & ~3u) + 4) * 4;  // bytes
   const size_t rbytes = (size_t)(I8 ? JI_ROWS : J_TI + cf.tj) * stride;
   float *Gs = reinterpret_cast<float *>(smem + rbytes);
-  uint32_t *ids = cf.lscr ? cf.lscr + (size_t)blockIdx.x * 4 * capt : reinterpret_cast<uint32_t *>(Gs + cf.gcap);
+  uint32_t *ids = cf.lscr ? cf.lscr + (size_t)blockIdx.x * (4 + NW) * capt : reinterpret_cast<uint32_t *>(Gs + cf.gcap);
   float *mx = reinterpret_cast<float *>(ids + capt);
-  uint32_t *cnt = reinterpret_cast<uint32_t *>(mx + capt);  // entries per target, then their offsets
-  int *nrm = reinterpret_cast<int *>(cnt + capt);           // (I8 only)
+  uint32_t *tend = reinterpret_cast<uint32_t *>(mx + capt);  // end of each target's entries
+  int *nrm = reinterpret_cast<int *>(tend + capt);           // (I8 only)
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(nrm + capt);  // NW x capt
   unsigned long long npairs = 0;
   for (uint32_t n = n0 + blockIdx.x; n < n1; n += gridDim.x) {
     const uint32_t a = s.lnew[n], b = s.lold[n];
@@ -629,25 +650,44 @@ __global__ void __launch_bounds__(I8 ? JI_THREADS : J_THREADS)
     if constexpr (I8) {
       const uint32_t ch = s.d / 16;
       auto stage = [&](uint8_t *dst, uint32_t r0, uint32_t cntr) {
-        for (uint32_t e = tid; e < cntr * ch; e += T) {
-          const uint32_t r = e / ch, k = e % ch;
-          cp_async16(dst + (size_t)r * stride + k * 16, s.base8 + (size_t)ids[r0 + r] * s.d + k * 16);
+        constexpr int U = 4;  // chunks in flight per thread
+        for (uint32_t e0 = tid; e0 < cntr * ch; e0 += U * T) {
+          uint4 v[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const uint32_t e = e0 + u * T;
+            if (e < cntr * ch)
+              v[u] = __ldg(reinterpret_cast<const uint4 *>(s.base8 + (size_t)ids[r0 + e / ch] * s.d) + e % ch);
+          }
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const uint32_t e = e0 + u * T;
+            if (e < cntr * ch) {
+              uint4 lo, hi;
+              ji_halves(v[u].x, lo.x, lo.y);
+              ji_halves(v[u].y, lo.z, lo.w);
+              ji_halves(v[u].z, hi.x, hi.y);
+              ji_halves(v[u].w, hi.z, hi.w);
+              uint4 *p = reinterpret_cast<uint4 *>(dst + (size_t)(e / ch) * stride) + 2 * (e % ch);
+              p[0] = lo;
+              p[1] = hi;
+            }
+          }
         }
       };
       if (tot <= JI_ROWS) {
         stage(smem, 0, tot);
-        cp_async_wait_all();
         __syncthreads();
         ji_tile(smem, smem, stride, s.d, a, tot, 0, 0, nrm, G, gs, warp, NW, lane);
       } else {
-        uint8_t *J = smem + (size_t)64 * stride;
-        for (uint32_t i0 = 0; i0 < a; i0 += 64)
-          for (uint32_t j0 = 0; j0 < tot; j0 += 64) {
-            const uint32_t ti = min(64u, a - i0), tj = min(64u, tot - j0);
+        constexpr uint32_t H = JI_ROWS / 2;
+        uint8_t *J = smem + (size_t)H * stride;
+        for (uint32_t i0 = 0; i0 < a; i0 += H)
+          for (uint32_t j0 = 0; j0 < tot; j0 += H) {
+            const uint32_t ti = min(H, a - i0), tj = min(H, tot - j0);
             __syncthreads();
             if (j0 == 0) stage(smem, i0, ti);
             stage(J, j0, tj);
-            cp_async_wait_all();
             __syncthreads();
             ji_tile(smem, J, stride, s.d, ti, tj, i0, j0, nrm, G, gs, warp, NW, lane);
           }
@@ -690,73 +730,86 @@ __global__ void __launch_bounds__(I8 ? JI_THREADS : J_THREADS)
       }
     }
     __syncthreads();
-    // offers per target: pairs of different ids (a pair of new rows is
-    // evaluated in one of its two orders, whatever the positions)
-    for (uint32_t p = warp; p < tot; p += NW) {
-      const uint32_t pid = ids[p];
-      const float m = mx[p];
-      const uint32_t end = p < a ? tot : a;
-      uint32_t c = 0;
-      for (uint32_t q0 = 0; q0 < end; q0 += 32) {
-        const uint32_t q = q0 + lane;
-        bool diff = false, ok = false;
-        if (q < end) {
-          diff = ids[q] != pid;
-          ok = diff && (q < a ? G[(size_t)p * gs + q] : G[(size_t)q * gs + p]) <= m;
+    // Offers per target: pairs of different ids (a pair of new rows is
+    // evaluated in one of its two orders, whatever the positions).  A lane
+    // takes a target, a warp every NW-th partner of 32 targets: the tile is
+    // read along its rows or columns without conflicts, and nothing is voted
+    // on.  cnt[w * capt + p]: warp w's entries for target p, then their ends.
+    for (uint32_t p0 = 0; p0 < tot; p0 += 32) {
+      const uint32_t p = p0 + lane;
+      if (p < tot) {
+        const uint32_t pid = ids[p];
+        const float m = mx[p];
+        uint32_t c = 0, np = 0;
+        for (uint32_t q = warp; q < a; q += NW) {
+          const uint32_t id = ids[q];
+          c += id != pid && G[(size_t)p * gs + q] <= m;
+          np += pid < id;
         }
-        c += __popc(__ballot_sync(FULL, ok));
-        if (p < a && pairs) npairs += diff && (q >= a || pid < ids[q]);
+        if (p < a) {
+          for (uint32_t q = a + warp; q < tot; q += NW) {
+            const bool diff = ids[q] != pid;
+            c += diff && G[(size_t)q * gs + p] <= m;
+            np += diff;
+          }
+          npairs += np;
+        }
+        cnt[warp * capt + p] = c;
       }
-      if (lane == 0) cnt[p] = c;
     }
     __syncthreads();
     if (warp == 0) {
       uint32_t run = 0;
       for (uint32_t p0 = 0; p0 < tot; p0 += 32) {
         const uint32_t p = p0 + lane;
-        const uint32_t c = p < tot ? cnt[p] : 0u;
+        uint32_t c = 0;
+#pragma unroll
+        for (int w = 0; w < NW; w++) c += p < tot ? cnt[w * capt + p] : 0u;
         uint32_t x = c;
         for (int k = 1; k < 32; k <<= 1) {
           const uint32_t y = __shfl_up_sync(FULL, x, k);
           if (lane >= k) x += y;
         }
-        if (p < tot) cnt[p] = run + x;  // inclusive ends
+        if (p < tot) {
+          uint32_t at = run + x - c;  // each warp's first entry of target p
+#pragma unroll
+          for (int w = 0; w < NW; w++) {
+            const uint32_t n1 = cnt[w * capt + p];
+            cnt[w * capt + p] = at;
+            at += n1;
+          }
+          tend[p] = at;
+        }
         run += __shfl_sync(FULL, x, 31);
       }
       if (lane == 0) ebase = run ? atomicAdd(o.cursor, (unsigned long long)run) : 0ull;
     }
     __syncthreads();
-    const uint32_t total = cnt[tot - 1];
+    const uint32_t total = tend[tot - 1];
     if (total == 0 || ebase + total > o.cap) continue;  // block-uniform
     for (uint32_t p = tid; p < tot; p += T) {
-      const uint32_t e0 = p ? cnt[p - 1] : 0u, c = cnt[p] - e0;
+      const uint32_t e0 = cnt[p], c = tend[p] - e0;
       if (c) {
         const uint32_t t = ids[p];
         o.desc[o.toff[t] + atomicAdd(&o.tcur[t], 1u)] = make_uint4((uint32_t)(ebase + e0), c, n, p);
       }
     }
-    for (uint32_t p = warp; p < tot; p += NW) {
-      const uint32_t e0 = p ? cnt[p - 1] : 0u;
-      if (cnt[p] == e0) continue;
-      const uint32_t pid = ids[p];
-      const float m = mx[p];
-      const uint32_t end = p < a ? tot : a;
-      size_t at = (size_t)ebase + e0;
-      for (uint32_t q0 = 0; q0 < end; q0 += 32) {
-        const uint32_t q = q0 + lane;
-        float dist = 0.f;
-        bool ok = false;
-        if (q < end && ids[q] != pid) {
-          dist = q < a ? G[(size_t)p * gs + q] : G[(size_t)q * gs + p];
-          ok = dist <= m;
-        }
-        const unsigned om = __ballot_sync(FULL, ok);
-        if (ok) {
-          const size_t w = at + __popc(om & lt);
-          o.ent[w] = make_uint2(__float_as_uint(dist), ids[q]);
-          o.eq[w] = (uint16_t)q;
-        }
-        at += __popc(om);
+    for (uint32_t p0 = 0; p0 < tot; p0 += 32) {
+      const uint32_t p = p0 + lane;
+      if (p < tot && tend[p] > cnt[p]) {
+        const uint32_t pid = ids[p];
+        const float m = mx[p];
+        size_t at = (size_t)ebase + cnt[warp * capt + p];
+        auto put = [&](uint32_t q, uint32_t id, float dist) {
+          if (id != pid && dist <= m) {
+            o.ent[at] = make_uint2(__float_as_uint(dist), id);
+            o.eq[at] = (uint16_t)q;
+            at++;
+          }
+        };
+        for (uint32_t q = warp; q < a; q += NW) put(q, ids[q], G[(size_t)p * gs + q]);
+        if (p < a)
+          for (uint32_t q = a + warp; q < tot; q += NW) put(q, ids[q], G[(size_t)q * gs + p]);
       }
     }
   }
@@ -1428,7 +1481,8 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
   if (!join_i8)
     while (jc.tj > 32 && (size_t)(J_TI + jc.tj) * fstride * 4 > 200 * 1024) jc.tj -= 32;
   size_t join_smem = join_i8 ? (size_t)JI_ROWS * ji_stride(c->d) : (size_t)(J_TI + jc.tj) * fstride * 4;
-  const size_t lists = (size_t)capt * 16;
+  const uint32_t lwords = 4 + (join_i8 ? JI_THREADS : J_THREADS) / 32;  // words per list entry
+  const size_t lists = (size_t)capt * lwords * 4;
   const bool lists_smem = join_smem + lists <= 200 * 1024;
   if (lists_smem) join_smem += lists;
   if (join_smem + (size_t)jc.gcap * 4 <= 220 * 1024) join_smem += (size_t)jc.gcap * 4;
@@ -1444,7 +1498,7 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
   }
   WV_CHECK(c, jper > 0, WV_ERR_LIMIT, "the local join does not fit the device (d=%u)", c->d);
   const uint32_t jgrid = (uint32_t)(c->sms * jper);
-  if (!lists_smem) jc.lscr = c->buf<uint32_t>("join_l", (size_t)jgrid * 4 * capt, &e);
+  if (!lists_smem) jc.lscr = c->buf<uint32_t>("join_l", (size_t)jgrid * lwords * capt, &e);
   WV_CUDA(c, e);
   const size_t af_smem = AF_WARPS * af_warp_words(p.L) * 4;
   WV_CUDA(c, cudaFuncSetAttribute(k_apply_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)af_smem));
