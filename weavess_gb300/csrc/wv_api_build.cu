@@ -69,6 +69,8 @@ int wv_load_built_graph(wv_ctx *c) {
   WV_CUDA(c, c->gdeg.ensure(n * 4));
   WV_CUDA(c, cudaMemcpyAsync(c->gids.p, c->fg_ids.p, n * w * 4, cudaMemcpyDeviceToDevice, c->stream));
   WV_CUDA(c, cudaMemcpyAsync(c->gdeg.p, c->fg_deg.p, n * 4, cudaMemcpyDeviceToDevice, c->stream));
+  WV_CUDA(c, wv::rows_repeat(c->gids.as<uint32_t>(), c->gdeg.as<uint32_t>(), (uint32_t)n, (uint32_t)w, c->d_repeats(),
+                             c->sms, c->stream));
   const uint32_t ep = c->fg_has_ep ? c->fg_ep : 0;
   uint32_t dep = 0;
   WV_CUDA(c, cudaMemcpyAsync(&dep, c->fg_deg.as<uint32_t>() + ep, 4, cudaMemcpyDeviceToHost, c->stream));

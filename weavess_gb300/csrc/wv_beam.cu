@@ -438,6 +438,7 @@ __global__ void __maxnreg__(128) k_beam(SearchArgs a) {
   vis.touched = a.touched + (size_t)slot * a.words;
   unsigned long long dcount = 0, hcount = 0;
   const unsigned lt = (1u << lane) - 1u;
+  const bool distinct = a.repeats && *a.repeats == 0;
   float *pd = s.pd;
   uint32_t *pi = s.pi;
 
@@ -590,8 +591,7 @@ __global__ void __maxnreg__(128) k_beam(SearchArgs a) {
             set_err(a.status, DEV_BAD_ID);
             id = INVALID;
           }
-          const unsigned same = __match_any_sync(FULL, id);
-          const bool leader = (__ffs(same) - 1) == lane;
+          const bool leader = distinct || (__ffs(__match_any_sync(FULL, id)) - 1) == lane;
           bool ws;
           const bool fresh = vis.test_and_set(id != INVALID && leader, id, lane, ws);
           const unsigned fm = __ballot_sync(FULL, fresh);

@@ -1461,7 +1461,7 @@ namespace {
 
 int run_build_search(wv_ctx *c, const float *d_queries, uint32_t nq, const uint32_t *d_seeds, uint32_t seed_stride,
                      uint32_t L, const uint32_t *gids, const uint32_t *gdeg, uint32_t gw, DI *vis, uint32_t *vcnt,
-                     uint32_t vcap, uint32_t *out_ids, uint32_t K, uint32_t vlimit = 0) {
+                     uint32_t vcap, uint32_t *out_ids, uint32_t K, const int *repeats, uint32_t vlimit = 0) {
   if (vlimit == 0) vlimit = vcap;
   const uint32_t cap = gw + 32;
   int blocks = search_grid(c->d, L, cap, c->device);
@@ -1485,6 +1485,7 @@ int run_build_search(wv_ctx *c, const float *d_queries, uint32_t nq, const uint3
   a.gids = gids;
   a.gdeg = gdeg;
   a.gw = gw;
+  a.repeats = repeats;
   a.queries = d_queries;
   a.nq = nq;
   a.seeds = d_seeds;
@@ -1588,6 +1589,7 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   uint32_t *seed1 = c->buf<uint32_t>("seed1", p.L, &e);
   uint32_t *one = c->buf<uint32_t>("one", 4, &e);
   WV_CUDA(c, e);
+  WV_CUDA(c, rows_repeat(c->fg_ids.as<uint32_t>(), c->fg_deg.as<uint32_t>(), n, gw, c->d_link_repeats(), c->sms, c->stream));
   // ---- entry point (ComponentRefineEntryCentroid::EntryInner); SSG has none
   // (its RefineInner leaves the entry step out) and draws no rand() here
   uint32_t ep = 0;
@@ -1606,7 +1608,7 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
     DI *v1 = c->buf<DI>("vis1", (size_t)n + p.entry_L + 64, &e);
     WV_CUDA(c, e);
     rc = run_build_search(c, center, 1, seed1, p.entry_L, p.entry_L, c->fg_ids.as<uint32_t>(),
-                          c->fg_deg.as<uint32_t>(), gw, v1, one + 1, n + p.entry_L + 64, one, 1);
+                          c->fg_deg.as<uint32_t>(), gw, v1, one + 1, n + p.entry_L + 64, one, 1, c->d_link_repeats());
     if (rc) return rc;
     WV_CUDA(c, cudaMemcpyAsync(&ep, one, 4, cudaMemcpyDeviceToHost, c->stream));
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1653,7 +1655,7 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
       int rc = ssg ? run_prop2(c, n0, cnt, p.L, vis, vcnt, vcap)
                    : run_build_search(c, c->base.as<float>() + (size_t)n0 * c->d, cnt, dseeds,
                                       shared_seeds ? 0 : p.L, p.L, c->fg_ids.as<uint32_t>(),
-                                      c->fg_deg.as<uint32_t>(), gw, vis, vcnt, vcap, nullptr, 1,
+                                      c->fg_deg.as<uint32_t>(), gw, vis, vcnt, vcap, nullptr, 1, c->d_link_repeats(),
                                       vcap - ((vamana && !p.clean) ? 0 : gw));
       if (rc) return rc;
       int st0 = 0;
@@ -2063,7 +2065,7 @@ int conn_dfs_gpu(wv_ctx *c, uint32_t L_refine, uint32_t *added) {
       vis = c->buf<DI>("conn_vis", (size_t)B * vcap, &e);
       WV_CUDA(c, e);
       rc = run_build_search(c, dq, B, dseed, L_refine, L_refine, c->fg_ids.as<uint32_t>(), c->fg_deg.as<uint32_t>(),
-                            w, vis, dvc, vcap, dout, 1);
+                            w, vis, dvc, vcap, dout, 1, nullptr);
       if (rc) return rc;
       int st0 = 0;
       WV_CUDA(c, cudaMemcpyAsync(&st0, c->d_status(), 4, cudaMemcpyDeviceToHost, c->stream));

@@ -210,6 +210,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   vis.touched = a.touched + (size_t)slot * a.words;
   unsigned long long dcount = 0, hcount = 0;
   const unsigned lt = (1u << lane) - 1u;
+  const bool distinct = a.repeats && *a.repeats == 0;
   float *pd = s.pd;
   uint32_t *pi = s.pi;
 
@@ -323,8 +324,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
           id = INVALID;
         }
         // a repeated id inside this chunk: only its first position visits it
-        const unsigned same = __match_any_sync(FULL, id);
-        const bool leader = (__ffs(same) - 1) == lane;
+        const bool leader = distinct || (__ffs(__match_any_sync(FULL, id)) - 1) == lane;
         bool was_seed;
         const bool fresh = vis.test_and_set(id != INVALID && leader, id, lane, was_seed);
         const unsigned fm = __ballot_sync(FULL, fresh);
@@ -441,7 +441,12 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         // pool entry j moves down by the number of candidates placed before
         // it (those with ub <= j); in place, from the end, 32 at a time: a
         // chunk is read before it is written and only moves to higher slots
+        // (no other chunk reads those), and every final slot is written once.
+        // Up to 4 candidates (the usual case) are counted from registers.
         const int lo = (int)ub[0];
+        const bool few = ncand <= 4;
+        const int u0 = lo, u1 = ncand > 1 ? (int)ub[1] : L, u2 = ncand > 2 ? (int)ub[2] : L,
+                  u3 = ncand > 3 ? (int)ub[3] : L;
         for (int jt = L; jt > lo; jt -= 32) {
           const int j = jt - 32 + lane;
           const bool act = j >= lo;
@@ -451,15 +456,16 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
           if (act) {
             v = pd[j];
             id = pi[j];
-            pos = j + upper_bound_of(ub, ncand, (uint32_t)j);
+            pos = j + (few ? (j >= u0) + (j >= u1) + (j >= u2) + (j >= u3)
+                           : upper_bound_of(ub, ncand, (uint32_t)j));
           }
           __syncwarp();
           if (act && pos < L) {
             pd[pos] = v;
             pi[pos] = id;
           }
-          __syncwarp();
         }
+        __syncwarp();
         for (int c = lane; c < ncand; c += 32) {
           const int pos = (int)ub[c] + c;
           if (pos < L) {
@@ -568,6 +574,28 @@ int search_grid(uint32_t d, uint32_t Lmax, uint32_t cap, int device, SearchShape
 }
 int search_grid(uint32_t d, uint32_t Lmax, uint32_t cap, int device) {
   return search_grid(d, Lmax, cap, device, SearchShape{});
+}
+
+static __global__ void k_rows_repeat(const uint32_t *ids, const uint32_t *deg, uint32_t n, uint32_t w, int *flag) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
+    const uint32_t d = min(deg[v], w);
+    for (uint32_t m0 = 0; m0 < d; m0 += 32) {
+      const bool in = m0 + lane < d;
+      const unsigned live = __ballot_sync(FULL, in);
+      const uint32_t id = in ? ids[(size_t)v * w + m0 + lane] : 0u;
+      const unsigned same = __match_any_sync(FULL, id) & live;
+      if (in && (same & (same - 1))) *flag = 1;
+    }
+  }
+}
+cudaError_t rows_repeat(const uint32_t *ids, const uint32_t *deg, uint32_t n, uint32_t w, int *flag, int sms,
+                        cudaStream_t stream) {
+  const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), stream);
+  if (e != cudaSuccess) return e;
+  k_rows_repeat<<<sms * 8, 256, 0, stream>>>(ids, deg, n, w, flag);
+  return cudaGetLastError();
 }
 
 // the dispatch order of a launch with per-query beams: a counting sort of
