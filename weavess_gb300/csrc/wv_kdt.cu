@@ -61,62 +61,62 @@ constexpr int KW = 4;                     // warps per block
 constexpr uint32_t KDT_MAX_K = 1024;
 
 // ---------------------------------------------------------------- shuffle
-// std::random_shuffle of 0..n-1 (libstdc++: step i swaps positions i and
-// j = rand() % (i + 1)); before step i position i still holds i, so a step is
-// a[i] = a[j]; a[j] = i.  The steps run in blocks of SH_W: the SH_W reads of
-// a block are issued together (they see every store of earlier blocks), and
-// a read of a position an earlier step of the same block wrote takes that
-// step's value from registers instead.
-constexpr int SH_W = 16;
+// std::random_shuffle of 0..n-1 (libstdc++: step t swaps positions t and
+// j_t = rand() % (t + 1)); before step t position t still holds t, so a step
+// is a[t] = a[j_t]; a[j_t] = t.  Read from the values: i enters at position
+// j_i in step i, the next step t that draws the same position moves it to
+// position t, the first step that draws t moves it on, and so on to its last
+// position.  So one block per tree links the steps by the position they draw
+// (k_kdt_links: `next` = the next step drawing the same position, `head` =
+// the first step drawing a position), and every value walks its own chain
+// (k_kdt_place; about ln n links).  A block links LT steps at a time, last
+// first; steps of one block that draw the same position take turns, the
+// latest first (two rounds are usual).  Eight trees of 60,000 ids: 0.23 ms;
+// 10.2 ms as one thread's chain of 60,000 dependent swaps per tree.
+constexpr int LT = 1024;
+constexpr uint32_t NO_STEP = 0xffffffffu;
 
-__device__ __forceinline__ void shuffle_steps(uint32_t *a, const int *rt, uint32_t n) {
-  a[0] = 0;
-  uint32_t i0 = 1;
-  for (; i0 + SH_W <= n; i0 += SH_W) {
-    uint32_t j[SH_W], v[SH_W];
-#pragma unroll
-    for (int k = 0; k < SH_W; k++) {
-      j[k] = (uint32_t)((long long)rt[i0 + k - 1] % (long long)(i0 + k + 1));
-      v[k] = a[j[k]];
-    }
-#pragma unroll
-    for (int k = 0; k < SH_W; k++) {
-#pragma unroll
-      for (int m = 0; m < k; m++) {
-        if (j[k] == i0 + m) v[k] = v[m];  // step m wrote a[i_m] = (its read)
-        if (j[k] == j[m]) v[k] = i0 + m;  // ... then a[j_m] = i_m (a[i_m] when j_m == i_m)
+__device__ __forceinline__ uint32_t drawn_pos(const int *r, uint32_t t) {
+  return t ? (uint32_t)__ldg(r + t - 1) % (t + 1) : 0u;
+}
+
+// claim: zero, head: NO_STEP
+__global__ void __launch_bounds__(LT)
+    k_kdt_links(uint32_t n, const int *r, unsigned long long *claim, uint32_t *head, uint32_t *next) {
+  const size_t tree = blockIdx.x;
+  r += tree * (n - 1);
+  claim += tree * n;
+  head += tree * n;
+  next += tree * n;
+  unsigned long long round = 0;
+  const uint32_t chunks = (n + LT - 1) / LT;
+  for (uint32_t c = chunks; c-- > 0;) {
+    const uint32_t t = c * LT + threadIdx.x;
+    bool pend = t < n;
+    const uint32_t j = pend ? drawn_pos(r, t) : 0u;
+    do {
+      round++;
+      const unsigned long long mine = (round << 32) | t;
+      if (pend) atomicMax(claim + j, mine);
+      __syncthreads();
+      if (pend && __ldcg(claim + j) == mine) {
+        __stcg(next + t, __ldcg(head + j));
+        __stcg(head + j, t);
+        pend = false;
       }
-    }
-#pragma unroll
-    for (int k = 0; k < SH_W; k++) {
-      const uint32_t i = i0 + k;
-      if (j[k] == i) {
-        a[i] = i;
-      } else {
-        a[i] = v[k];
-        a[j[k]] = i;
-      }
-    }
-  }
-  for (uint32_t i = i0; i < n; i++) {
-    const uint32_t jj = (uint32_t)((long long)rt[i - 1] % (long long)(i + 1));
-    if (jj == i) {
-      a[i] = i;
-    } else {
-      a[i] = a[jj];
-      a[jj] = i;
-    }
+    } while (__syncthreads_or(pend));
   }
 }
 
-__global__ void k_kdt_shuffle(uint32_t n, const int *r, uint32_t *leaf, int in_smem) {
-  extern __shared__ uint32_t sh[];
-  if (threadIdx.x != 0) return;
-  const uint32_t t = blockIdx.x;
-  uint32_t *a = in_smem ? sh : leaf + (size_t)t * n;
-  shuffle_steps(a, r + (size_t)t * (n - 1), n);
-  if (in_smem)
-    for (uint32_t i = 0; i < n; i++) leaf[(size_t)t * n + i] = a[i];
+__global__ void k_kdt_place(uint32_t n, size_t total, const int *r, const uint32_t *head, const uint32_t *next,
+                            uint32_t *leaf) {
+  for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < total; x += (size_t)gridDim.x * blockDim.x) {
+    const size_t tree = x / n, off = tree * n;
+    const uint32_t i = (uint32_t)(x - off);
+    uint32_t p = drawn_pos(r + tree * (n - 1), i);
+    for (uint32_t t = next[x]; t != NO_STEP; t = head[off + t]) p = t;
+    leaf[off + p] = i;
+  }
 }
 
 // ---------------------------------------------------------------- split
@@ -172,17 +172,19 @@ struct Split {
   float val;
 };
 
-// meanSplit (component_init.cpp:648-696) of ids[0, count) with the rng
-// output rv; mean / var: d floats of the warp's shared memory
-__device__ Split warp_split(const float *__restrict__ base, uint32_t d, uint32_t *ids, uint32_t count, uint32_t rv,
-                            float *mean, float *var, uint32_t *scr, int lane) {
+// the sample mean and the sum of squared deviations of each dimension, a
+// thread (tid of nthr) per dimension
+__device__ __forceinline__ void dim_stats(const float *__restrict__ base, uint32_t d, const uint32_t *ids,
+                                          uint32_t count, float *mean, float *var, uint32_t tid, uint32_t nthr) {
   const uint32_t cnt = min(KDT_SAMPLE + 1, count);
   const float div = __fdiv_rn(1.f, (float)cnt);
-  for (uint32_t k = lane; k < d; k += 32) {
+  for (uint32_t k = tid; k < d; k += nthr) {
     float m = 0.f;
+#pragma unroll 8
     for (uint32_t j = 0; j < cnt; j++) m = __fadd_rn(m, coord(base, d, ids[j], k));
     m = __fmul_rn(m, div);
     float v = 0.f;
+#pragma unroll 8
     for (uint32_t j = 0; j < cnt; j++) {
       const float dd = __fsub_rn(coord(base, d, ids[j], k), m);
       v = __fadd_rn(v, __fmul_rn(dd, dd));
@@ -190,38 +192,47 @@ __device__ Split warp_split(const float *__restrict__ base, uint32_t d, uint32_t
     mean[k] = m;
     var[k] = v;
   }
-  __syncwarp();
-  int dim = 0;
-  if (lane == 0) {
-    // selectDivision (component_init.cpp:732-756)
-    int num = 0;
-    uint32_t top[KDT_RAND_DIM];
-    for (uint32_t i = 0; i < d; i++) {
-      if (num < KDT_RAND_DIM || var[i] > var[top[num - 1]]) {
-        if (num < KDT_RAND_DIM) top[num++] = i;
-        else top[num - 1] = i;
-        int j = num - 1;
-        while (j > 0 && var[top[j]] > var[top[j - 1]]) {
-          const uint32_t x = top[j];
-          top[j] = top[j - 1];
-          top[j - 1] = x;
-          --j;
-        }
+}
+
+// selectDivision (component_init.cpp:732-756)
+__device__ int pick_dim(uint32_t d, const float *var, uint32_t rv) {
+  int num = 0;
+  uint32_t top[KDT_RAND_DIM];
+  for (uint32_t i = 0; i < d; i++) {
+    if (num < KDT_RAND_DIM || var[i] > var[top[num - 1]]) {
+      if (num < KDT_RAND_DIM) top[num++] = i;
+      else top[num - 1] = i;
+      int j = num - 1;
+      while (j > 0 && var[top[j]] > var[top[j - 1]]) {
+        const uint32_t x = top[j];
+        top[j] = top[j - 1];
+        top[j - 1] = x;
+        --j;
       }
     }
-    dim = (int)top[rv % (uint32_t)num];
   }
+  return (int)top[rv % (uint32_t)num];
+}
+
+__device__ __forceinline__ uint32_t split_at(uint32_t count, uint32_t lim1, uint32_t lim2) {
+  if (lim1 == count || lim2 == 0) return count / 2;
+  return lim1 > count / 2 ? lim1 : lim2 < count / 2 ? lim2 : count / 2;
+}
+
+// meanSplit (component_init.cpp:648-696) of ids[0, count) with the rng
+// output rv; mean / var: d floats of the warp's shared memory
+__device__ Split warp_split(const float *__restrict__ base, uint32_t d, uint32_t *ids, uint32_t count, uint32_t rv,
+                            float *mean, float *var, uint32_t *scr, int lane) {
+  dim_stats(base, d, ids, count, mean, var, lane, 32);
+  __syncwarp();
+  int dim = 0;
+  if (lane == 0) dim = pick_dim(d, var, rv);
   dim = __shfl_sync(FULL, dim, 0);
   const float cut = mean[dim];
   const uint32_t lim1 = warp_hoare(base, d, dim, ids, 0, count, cut, false, scr, lane);
   const uint32_t lim2 = warp_hoare(base, d, dim, ids, lim1, count, cut, true, scr, lane);
-  uint32_t idx;
-  if (lim1 > count / 2) idx = lim1;
-  else if (lim2 < count / 2) idx = lim2;
-  else idx = count / 2;
-  if (lim1 == count || lim2 == 0) idx = count / 2;
   __syncwarp();
-  return Split{idx, dim, cut};
+  return Split{split_at(count, lim1, lim2), dim, cut};
 }
 
 __device__ __forceinline__ KNode child_node(uint32_t start, uint32_t end, int parent, int depth, int tree) {
@@ -237,29 +248,122 @@ __device__ __forceinline__ KNode child_node(uint32_t start, uint32_t end, int pa
   return x;
 }
 
-// one level of the active set: warp i splits node act[i], its children go to
+// meanSplit by a block of LV threads: warp_split for the active levels,
+// where few nodes of many ids are split at once (the first level of eight
+// trees of 60,000 ids held eight warps busy for 3.8 ms, the eight levels
+// 7.4 ms, now 0.69 ms).  Each warp has a contiguous part of the ids, counts it, and places
+// its misplaced positions behind those of the warps before it.  Bound by the
+// latency of the gathers id -> coordinate, four per lane in flight.
+constexpr int LV = 1024, LW = LV / 32, LU = 4;
+
+struct LevelSmem {
+  uint32_t a[LW], b[LW];
+  int dim;
+};
+
+// the counts of the warps in `w` (LW of them): those before `warp` and all
+__device__ __forceinline__ void warp_offsets(const uint32_t *w, int warp, int lane, uint32_t &before, uint32_t &all) {
+  const uint32_t v = lane < LW ? w[lane] : 0u;
+  before = __reduce_add_sync(FULL, lane < warp ? v : 0u);
+  all = __reduce_add_sync(FULL, v);
+}
+
+__device__ uint32_t block_hoare(const float *__restrict__ base, uint32_t d, int dim, uint32_t *ids, uint32_t lo,
+                                uint32_t hi, float cut, bool le, uint32_t *scr, LevelSmem &sm) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t seg = (hi - lo + LV - 1) / LV * 32;
+  const uint32_t w0 = min(hi, lo + warp * seg), w1 = min(hi, w0 + seg);
+  // f(p, left of the cut) for the warp's positions in order, 32 at a time
+  // (p >= w1: past them, not left)
+  auto each = [&](auto f) {
+    for (uint32_t p0 = w0; p0 < w1; p0 += 32 * LU) {
+      uint32_t id[LU];
+      float v[LU];
+#pragma unroll
+      for (int u = 0; u < LU; u++) id[u] = p0 + 32 * u + lane < w1 ? ids[p0 + 32 * u + lane] : 0u;
+#pragma unroll
+      for (int u = 0; u < LU; u++) v[u] = coord(base, d, id[u], dim);
+#pragma unroll
+      for (int u = 0; u < LU; u++) {
+        const uint32_t p = p0 + 32 * u + lane;
+        f(p, p < w1 && (le ? v[u] <= cut : v[u] < cut));
+      }
+    }
+  };
+  uint32_t c = 0, before, all;
+  each([&](uint32_t, bool left) { c += __popc(__ballot_sync(FULL, left)); });
+  if (lane == 0) sm.a[warp] = c;
+  __syncthreads();
+  warp_offsets(sm.a, warp, lane, before, all);
+  const uint32_t m = lo + all;
+  __syncthreads();
+  uint32_t ca = 0, cb = 0;
+  each([&](uint32_t p, bool left) {
+    ca += __popc(__ballot_sync(FULL, p < w1 && p < m && !left));
+    cb += __popc(__ballot_sync(FULL, p >= m && left));
+  });
+  if (lane == 0) {
+    sm.a[warp] = ca;
+    sm.b[warp] = cb;
+  }
+  __syncthreads();
+  uint32_t a0, s, b0, sb;
+  warp_offsets(sm.a, warp, lane, a0, s);
+  warp_offsets(sm.b, warp, lane, b0, sb);
+  uint32_t *A = scr, *B = scr + (hi - lo) / 2;  // s <= (hi - lo) / 2 of each
+  each([&](uint32_t p, bool left) {
+    const bool fa = p < w1 && p < m && !left, fb = p >= m && left;
+    const unsigned ma = __ballot_sync(FULL, fa), mb = __ballot_sync(FULL, fb);
+    if (fa) A[a0 + __popc(ma & lt)] = p;
+    if (fb) B[s - 1 - (b0 + __popc(mb & lt))] = p;
+    a0 += __popc(ma);
+    b0 += __popc(mb);
+  });
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < s; k += LV) {
+    const uint32_t a = A[k], b = B[k];
+    const uint32_t x = ids[a];
+    ids[a] = ids[b];
+    ids[b] = x;
+  }
+  __syncthreads();
+  return m;
+}
+
+// one level of the active set: a block per node act[i], its children go to
 // nodes child_base + 2i, + 2i + 1
-__global__ void __launch_bounds__(KW * 32)
+__global__ void __launch_bounds__(LV)
     k_kdt_level(const float *__restrict__ base, uint32_t d, uint32_t n, uint32_t *leaf, uint32_t *scr, KNode *nodes,
                 const int *act, uint32_t nact, uint32_t child_base, uint32_t rv0) {
   extern __shared__ float ksm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float *mean = ksm + (size_t)warp * 2 * d, *var = mean + d;
-  for (uint32_t i = blockIdx.x * KW + warp; i < nact; i += gridDim.x * KW) {
+  __shared__ LevelSmem sm;
+  float *mean = ksm, *var = mean + d;
+  for (uint32_t i = blockIdx.x; i < nact; i += gridDim.x) {
     const int nd = act[i];
     const KNode x = nodes[nd];
     const size_t off = (size_t)x.tree * n + x.start;
-    const Split sp = warp_split(base, d, leaf + off, x.end - x.start, rv0, mean, var, scr + off, lane);
-    if (lane == 0) {
+    uint32_t *ids = leaf + off;
+    const uint32_t count = x.end - x.start;
+    dim_stats(base, d, ids, count, mean, var, threadIdx.x, LV);
+    __syncthreads();
+    if (threadIdx.x == 0) sm.dim = pick_dim(d, var, rv0);
+    __syncthreads();
+    const int dim = sm.dim;
+    const float cut = mean[dim];
+    const uint32_t lim1 = block_hoare(base, d, dim, ids, 0, count, cut, false, scr + off, sm);
+    const uint32_t lim2 = block_hoare(base, d, dim, ids, lim1, count, cut, true, scr + off, sm);
+    if (threadIdx.x == 0) {
+      const uint32_t mid = split_at(count, lim1, lim2);
       const int l = (int)(child_base + 2 * i), r = l + 1;
-      nodes[l] = child_node(x.start, x.start + sp.mid, nd, x.depth + 1, x.tree);
-      nodes[r] = child_node(x.start + sp.mid, x.end, nd, x.depth + 1, x.tree);
-      nodes[nd].dim = sp.dim;
-      nodes[nd].val = sp.val;
+      nodes[l] = child_node(x.start, x.start + mid, nd, x.depth + 1, x.tree);
+      nodes[r] = child_node(x.start + mid, x.end, nd, x.depth + 1, x.tree);
+      nodes[nd].dim = dim;
+      nodes[nd].val = cut;
       nodes[nd].left = l;
       nodes[nd].right = r;
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
@@ -694,10 +798,13 @@ int init_kdt_gpu(wv_ctx *c, uint32_t T, uint32_t K, uint32_t mlevel) {
     std::vector<int> r((size_t)T * (n - 1));
     for (auto &v : r) v = c->rnd.next();
     WV_CUDA(c, cudaMemcpyAsync(rnd_d, r.data(), r.size() * 4, cudaMemcpyHostToDevice, c->stream));
-    const size_t sm = (size_t)n * 4;
-    const bool in_smem = sm <= 200 * 1024;
-    if (in_smem) WV_CUDA(c, cudaFuncSetAttribute(k_kdt_shuffle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_kdt_shuffle<<<T, 32, in_smem ? sm : 0, c->stream>>>(n, rnd_d, leaf, in_smem ? 1 : 0);
+    unsigned long long *claim = c->buf<unsigned long long>("kd_claim", total, &e);
+    uint32_t *head = c->buf<uint32_t>("kd_head", total, &e);
+    WV_CUDA(c, e);
+    WV_CUDA(c, cudaMemsetAsync(claim, 0, total * 8, c->stream));
+    WV_CUDA(c, cudaMemsetAsync(head, 0xff, total * 4, c->stream));
+    k_kdt_links<<<T, LT, 0, c->stream>>>(n, rnd_d, claim, head, scr);
+    k_kdt_place<<<nblocks(total, 256, c->sms * 8), 256, 0, c->stream>>>(n, total, rnd_d, head, scr, leaf);
     WV_CUDA(c, cudaGetLastError());
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
   }
@@ -708,26 +815,31 @@ int init_kdt_gpu(wv_ctx *c, uint32_t T, uint32_t K, uint32_t mlevel) {
   uint32_t count = T;
   std::vector<int> act(T);
   for (uint32_t t = 0; t < T; t++) act[t] = (int)t;
+  uint32_t widest = n;  // ids of the widest active node
   std::mt19937 first(1998);
   const uint32_t rv0 = (uint32_t)first();
-  WV_CUDA(c, cudaFuncSetAttribute(k_kdt_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_split));
+  const size_t smem_level = (size_t)2 * d * 4;
+  WV_CUDA(c, cudaFuncSetAttribute(k_kdt_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_level));
   WV_CUDA(c, cudaFuncSetAttribute(k_kdt_dfs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_split));
   std::vector<KNode> kids;
   while (!act.empty() && act.size() < KDT_ACTIVE_MAX) {
     const uint32_t na = (uint32_t)act.size();
     WV_CHECK(c, count + 2 * (size_t)na <= ncap, WV_ERR_LIMIT, "KD-tree node capacity");
     WV_CUDA(c, cudaMemcpyAsync(act_d, act.data(), na * 4, cudaMemcpyHostToDevice, c->stream));
-    k_kdt_level<<<nblocks(na, KW, c->sms * 8), KW * 32, smem_split, c->stream>>>(c->base.as<float>(), d, n, leaf,
-                                                                                   scr, nodes, act_d, na, count, rv0);
+    k_kdt_level<<<na, LV, smem_level, c->stream>>>(c->base.as<float>(), d, n, leaf, scr, nodes, act_d, na, count,
+                                                     rv0);
     WV_CUDA(c, cudaGetLastError());
     kids.resize(2 * (size_t)na);
     WV_CUDA(c, cudaMemcpyAsync(kids.data(), nodes + count, kids.size() * sizeof(KNode), cudaMemcpyDeviceToHost,
                                c->stream));
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
     std::vector<int> next;
-    for (uint32_t i = 0; i < na; i++) {
-      if (kids[2 * i].end - kids[2 * i].start > K) next.push_back((int)(count + 2 * i));
-      if (kids[2 * i + 1].end - kids[2 * i + 1].start > K) next.push_back((int)(count + 2 * i + 1));
+    widest = 0;
+    for (uint32_t i = 0; i < 2 * na; i++) {
+      const uint32_t size = kids[i].end - kids[i].start;
+      if (size <= K) continue;
+      next.push_back((int)(count + i));
+      widest = std::max(widest, size);
     }
     count += 2 * na;
     act.swap(next);
@@ -735,13 +847,7 @@ int init_kdt_gpu(wv_ctx *c, uint32_t T, uint32_t K, uint32_t mlevel) {
   WV_CUDA(c, cudaMemcpyAsync(ncount, &count, 4, cudaMemcpyHostToDevice, c->stream));
   if (!act.empty()) {
     const uint32_t na = (uint32_t)act.size();
-    uint32_t nmt = 0;  // splits below one active node: fewer than its ids
-    std::vector<KNode> an(na);
-    for (uint32_t i = 0; i < na; i++) {
-      WV_CUDA(c, cudaMemcpyAsync(&an[i], nodes + act[i], sizeof(KNode), cudaMemcpyDeviceToHost, c->stream));
-    }
-    WV_CUDA(c, cudaStreamSynchronize(c->stream));
-    for (auto &x : an) nmt = std::max(nmt, x.end - x.start);
+    const uint32_t nmt = widest;  // splits below one active node: fewer than its ids
     uint32_t *mt = c->buf<uint32_t>("kd_mt", nmt + 1, &e);
     const int blocks = nblocks(na, KW, c->sms * 4);
     int *stacks = c->buf<int>("kd_stack", (size_t)blocks * KW * KDT_MAX_DEPTH, &e);
