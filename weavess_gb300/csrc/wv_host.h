@@ -12,21 +12,24 @@ namespace wv {
 // glibc's rand(): the TYPE_3 additive feedback generator (r[i] = r[i-3] +
 // r[i-31] mod 2^32, output r[i] >> 1) seeded by a 16807 Lehmer sequence with
 // 310 discarded outputs.  Reproduces the stream a fresh process sees (seed 1).
+// Words are made a block at a time (three chains of adds without an index to
+// wrap): 1 ns per value against 7 with a ring index taken modulo its length,
+// which bound the centroid entry's seed draw and the overflow draws of
+// NN-Descent.
 class GlibcRand {
  public:
   explicit GlibcRand(uint32_t seed = 1) { seed_with(seed); }
   void seed_with(uint32_t seed);
-  int next() { return (int)(step() >> 1); }
+  int next() {
+    if (pos_ == END) refill();
+    return (int)(w_[pos_++] >> 1);
+  }
 
  private:
-  uint32_t step() {
-    uint32_t v = r_[(i_ + 3) % 34] + r_[(i_ + 31) % 34];
-    r_[i_] = v;
-    i_ = (i_ + 1) % 34;
-    return v;
-  }
-  uint32_t r_[34];
-  int i_ = 0;
+  static constexpr int HIST = 31, BLOCK = 495, END = HIST + BLOCK;  // (BLOCK: a multiple of 3)
+  void refill();
+  uint32_t w_[END];  // the last 31 words of the previous block, then a block
+  int pos_ = END;    // the next word to hand out
 };
 
 // The rand() source a context draws from: its own glibc-compatible stream or
