@@ -1,11 +1,13 @@
 """Real-valued rows in the reference's order, read by eight lanes at a time:
 row lengths about the 32 and 64 dimensions of a step, few and many rows at
-once, in the greedy route and its exact rerank.  Ids, counts and distance bits
-against the oracle."""
+once, in the greedy route, its exact rerank and the layered route, whose lists
+here also hold an id twice.  Ids, counts and distance bits against the
+oracle."""
 import numpy as np
 import pytest
 
 import oracle as O
+from weavess_gb300 import datasets as ds
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +45,34 @@ def test_route_matches_oracle(ctx, d, K):
     res, dc, hc, dd = ctx.search(query, 45, 10, entry="rand", return_dist=True)
     same_bits(dd, query, base[res])
     ctx.set_precision("fp32")
+
+
+@pytest.mark.parametrize("router", ["hnsw", "nsw"])
+@pytest.mark.parametrize("kind,d", [("int", 128), ("int", 48), ("int", 20), ("real", 36), ("real", 128)])
+def test_layered_route_with_repeated_ids(ctx, kind, d, router):
+    rng = np.random.default_rng(d)
+    n = 1200
+    if kind == "int":
+        base, query = ds.int_mixture(n, d, 8, seed=5, n_query=40)
+        query[::5] += 0.25  # a real-valued query on integer rows
+    else:
+        base, query = rng.normal(size=(n, d)).astype(np.float32), rng.normal(size=(40, d)).astype(np.float32)
+    for repeats in (False, True):
+        words = [3, 1]
+        for v in range(n):
+            layers = 2 if v % 16 == 3 else 1
+            words += [v, layers]
+            for lv in range(layers):
+                pool = np.arange(n) if lv == 0 else np.arange(3, n, 16)
+                row = rng.choice(pool, 36 if lv == 0 else 8, replace=False).tolist()
+                if repeats:
+                    row = row[:20] + row[5:9] + row[20:] + row[:3]
+                words += [len(row)] + row
+        words = np.array(words, np.uint32)
+        ctx.upload_base(base)
+        ctx.load_hnsw(words)
+        for L in (10, 70):
+            res, dist, dc, hc = ctx.search_hnsw(query, L, 10, router=router, return_dist=True)
+            want, wdc, whc = O.search_hnsw(base, query, words, L, router=router)
+            assert np.array_equal(res, want) and (dc, hc) == (wdc, whc)
+            same_bits(dist, query, base[res])

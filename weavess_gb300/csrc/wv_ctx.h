@@ -118,10 +118,11 @@ struct wv_ctx {
 
   unsigned *d_next() { return misc.as<unsigned>(); }
   unsigned long long *d_counters() { return reinterpret_cast<unsigned long long *>(misc.as<char>() + 8); }
-  // whether a row of the search graph / of the built graph a link searches
-  // lists an id twice within 32 slots (rows_repeat)
+  // whether a row of the search graph / of the built graph a link searches /
+  // of the layered graph lists an id twice within 32 slots (rows_repeat)
   int *d_repeats() { return reinterpret_cast<int *>(misc.as<char>() + 52); }
   int *d_link_repeats() { return reinterpret_cast<int *>(misc.as<char>() + 56); }
+  int *d_hnsw_repeats() { return reinterpret_cast<int *>(misc.as<char>() + 60); }
   int *d_status() { return reinterpret_cast<int *>(misc.as<char>() + 32); }
   void release_work() {
     for (auto &kv : work) kv.second.release();

@@ -17,9 +17,13 @@
 // CloserFirst, a min-heap) are kept as libstdc++ heaps with the same
 // comparators, so equal distances resolve exactly as they do there.  A
 // neighbour list is handled 32 entries at a time: the lanes mark the visited
-// bits and take the distances (exact reference order, a lane per row), then one lane applies
-// the queue updates in list order.  The visited set is a per-warp bitset over
-// the nodes, cleared through the list of words it touched (VisitedList::Reset
+// bits, the warp takes the distances (the reference's value), then one lane
+// applies the queue updates in list order -- of those entries only that pass
+// the result queue's bound as it stood before the chunk (it only falls).
+// Integer data is read as bytes, real-valued rows by eight lanes each (a lane
+// per row read 32 lines per load).  What bounds it: the chain of a query's
+// expansions.  5,000 queries at L = 100 over 100k x 128: 1.85 -> 1.63 ms.
+// The visited set is a per-warp bitset over the nodes, cleared through the list of words it touched (VisitedList::Reset
 // gives a fresh set for every layer and every SearchAtLayer).
 #include <algorithm>
 #include <cstdio>
@@ -28,8 +32,10 @@
 #include "stl_order.cuh"
 #include "wv_common.cuh"
 #include "wv_ctx.h"
+#include "wv_search.h"
+#include "wv_search_common.cuh"
 
-using namespace wv;
+namespace wv {
 
 namespace {
 
@@ -58,7 +64,10 @@ struct CloserLess {  // std::less<CloserFirst>: a min-heap by distance (index.h:
 
 struct HnswArgs {
   const float *base;
+  const uint8_t *base8;  // integer base (d a multiple of 16 up to 256): the rows as bytes, or null
+  const float *xnorm;    // squared row norms (integer data)
   uint32_t n, d;
+  const int *repeats;    // 0 there: no layer-0 list holds an id twice within 32 entries
   const uint32_t *l0_ids, *l0_deg;
   uint32_t w0;
   const uint32_t *up_off, *up;
@@ -85,6 +94,11 @@ struct WarpState {
   float *dist;    // 32
   HEnt *path;     // HN_PATH
   HEnt *csh;      // HN_CSH: the shared part of the candidate queue
+  bool ints;      // integer base and query, rows from the byte copy
+  bool distinct;  // no repeats in the layer-0 lists
+  uint4 qc;       // this lane's bytes of an integer query
+  float qn;       // its squared norm
+  bool nan;       // the query met a distance that is not a number
 };
 
 __host__ __device__ inline size_t hn_warp_bytes(uint32_t d, uint32_t L) {
@@ -109,16 +123,19 @@ __device__ inline WarpState hn_carve(uint8_t *p, uint32_t d, uint32_t L) {
   return w;
 }
 
-// exact-order squared L2 (Distance::compare, include/weavess/distance.h) of
-// base row `id` and the query in shared memory, by one lane: a row's 16-byte
-// pieces are read straight from global memory (each lane its own row)
-__device__ __forceinline__ float hn_dist(const float *__restrict__ base, uint32_t d, uint32_t id, const float *qv) {
-  const float4 *x = reinterpret_cast<const float4 *>(base + (size_t)id * d);
-  const float4 *q = reinterpret_cast<const float4 *>(qv);
+// squared L2 (Distance::compare, include/weavess/distance.h) of `cnt` rows
+// (ids in lanes 0..cnt-1) and the query, as the reference's order gives it
+__device__ __forceinline__ float hn_dist(const HnswArgs &a, const WarpState &s, uint32_t id, int cnt, int lane) {
+  return s.ints ? rows_dist_i8(a.base8, a.xnorm, a.d, id, cnt, s.qc, s.qn, lane)
+                : rows_dist_f32(a.base, a.d, id, cnt, s.qv, lane);
+}
+// of one row, on every lane (a query's first steps: no second copy of the above)
+__device__ __forceinline__ float hn_dist1(const HnswArgs &a, const WarpState &s, uint32_t id) {
+  const float4 *x = reinterpret_cast<const float4 *>(a.base + (size_t)id * a.d);
+  const float4 *q = reinterpret_cast<const float4 *>(s.qv);
   float acc = 0.f;
-  const uint32_t d4 = d >> 2;
-#pragma unroll 8
-  for (uint32_t g = 0; g < d4; g++) acc = __fadd_rn(acc, group4(q[g], __ldg(x + g)));
+#pragma unroll 4
+  for (uint32_t g = 0; g < a.d >> 2; g++) acc = __fadd_rn(acc, group4(q[g], __ldg(x + g)));
   return acc;
 }
 
@@ -164,15 +181,15 @@ __device__ __forceinline__ void hn_row(const HnswArgs &a, uint32_t node, uint32_
 // the fresh (not yet visited) entries of row[b0, b0 + 32) in list order into
 // s.ids / s.dist (distances in the reference's order); returns their count
 __device__ int hn_chunk(const HnswArgs &a, WarpState &s, Bits &vis, const uint32_t *row, uint32_t deg, uint32_t b0,
-                        int lane) {
+                        bool distinct, int lane) {
   const uint32_t j = b0 + lane;
   uint32_t id = j < deg ? row[j] : HN_NONE;
   if (id != HN_NONE && id >= a.n) {
     set_err(a.status, DEV_BAD_ID);
     id = HN_NONE;
   }
-  const unsigned same = __match_any_sync(FULL, id);
-  const bool leader = id != HN_NONE && (__ffs(same) - 1) == lane;
+  bool leader = id != HN_NONE;
+  if (!distinct) leader &= (__ffs(__match_any_sync(FULL, id)) - 1) == lane;  // (warp-uniform: every lane matches)
   const bool fresh = vis.test_set(leader, id, lane);
   const unsigned fm = __ballot_sync(FULL, fresh);
   const int cnt = __popc(fm);
@@ -181,8 +198,10 @@ __device__ int hn_chunk(const HnswArgs &a, WarpState &s, Bits &vis, const uint32
   if (fresh) s.ids[__popc(fm & ((1u << lane) - 1u))] = my;
   __syncwarp();
   const uint32_t cid = lane < cnt ? s.ids[lane] : 0u;
-  const float dd = lane < cnt ? hn_dist(a.base, a.d, cid, s.qv) : 0.f;
-  if (lane < cnt) s.dist[lane] = dd;
+  if (cnt) {
+    const float dd = hn_dist(a, s, cid, cnt, lane);
+    if (lane < cnt) s.dist[lane] = dd;
+  }
   __syncwarp();
   return cnt;
 }
@@ -193,7 +212,8 @@ __device__ void hn_search_layer(const HnswArgs &a, WarpState &s, Bits &vis, Spli
                                 uint32_t &rs, unsigned long long &dc, unsigned long long &hc, int lane) {
   // the entry's distance, then both queues hold it
   {
-    const float de = lane == 0 ? hn_dist(a.base, a.d, entry, s.qv) : 0.f;
+    const float de = hn_dist1(a, s, entry);
+    s.nan |= de != de;
     dc++;
     vis.clear(lane);
     vis.test_set(lane == 0, entry, lane);
@@ -226,10 +246,17 @@ __device__ void hn_search_layer(const HnswArgs &a, WarpState &s, Bits &vis, Spli
     uint32_t deg;
     hn_row(a, node, 0, row, deg);
     for (uint32_t b0 = 0; b0 < deg; b0 += 32) {
-      const int cnt = hn_chunk(a, s, vis, row, deg, b0, lane);
+      const int cnt = hn_chunk(a, s, vis, row, deg, b0, s.distinct, lane);
       dc += cnt;
+      // entries that a full result queue turns away now stay turned away (a
+      // NaN in the queue voids its order: then every entry is looked at)
+      const float di = lane < cnt ? s.dist[lane] : 0.f, top = s.res[0].d;
+      s.nan |= __any_sync(FULL, di != di);
+      unsigned todo = __ballot_sync(FULL, lane < cnt && (s.nan || rs < a.L || top > di));
+      if (!todo) continue;
       if (lane == 0) {
-        for (int t = 0; t < cnt; t++) {
+        for (; todo; todo &= todo - 1) {
+          const int t = __ffs(todo) - 1;
           const float d = s.dist[t];
           if (rs < a.L || s.res[0].d > d) {
             s.res[rs] = HEnt{d, s.ids[t]};
@@ -257,7 +284,8 @@ __device__ void hn_search_layer(const HnswArgs &a, WarpState &s, Bits &vis, Spli
   }
 }
 
-__global__ void __launch_bounds__(HN_WARPS * 32) k_hnsw(HnswArgs a) {
+// (80 registers and a few spills: 1.61 ms where 126 take 2.07 and 64 take 1.89)
+__global__ void __launch_bounds__(HN_WARPS * 32, 6) k_hnsw(HnswArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpState s = hn_carve(smem + (size_t)warp * hn_warp_bytes(a.d, a.L), a.d, a.L);
@@ -265,19 +293,31 @@ __global__ void __launch_bounds__(HN_WARPS * 32) k_hnsw(HnswArgs a) {
   Bits vis{a.bits + (size_t)slot * a.words, a.touched + (size_t)slot * a.words, 0};
   const SplitHeap cand{s.csh, a.cand + (size_t)slot * a.ccap};
   unsigned long long dc = 0, hc = 0;
+  s.distinct = *a.repeats == 0;
   for (;;) {
     uint32_t q = 0;
     if (lane == 0) q = atomicAdd(a.next_query, 1u);
     q = __shfl_sync(FULL, q, 0);
     if (q >= a.nq) break;
-    for (uint32_t k = lane; k < a.d; k += 32) s.qv[k] = a.queries[(size_t)q * a.d + k];
+    bool qint = true;
+    float qn = 0.f;
+    for (uint32_t k = lane; k < a.d; k += 32) {
+      const float v = a.queries[(size_t)q * a.d + k];
+      s.qv[k] = v;
+      qn = fmaf(v, v, qn);
+      qint &= v >= 0.f && v <= 255.f && v == rintf(v);
+    }
+    for (int o = 16; o > 0; o >>= 1) qn += __shfl_xor_sync(FULL, qn, o);
+    s.qn = qn;
+    s.nan = false;
+    s.ints = a.base8 && __all_sync(FULL, qint);
     __syncwarp();
+    s.qc = s.ints ? query_chunk_i8(s.qv, a.d, lane) : make_uint4(0u, 0u, 0u, 0u);
     uint32_t rs = 0;
     if (a.router == 0) {
       // ---- greedy descent through every layer (component_route.cpp:144-184)
       uint32_t cur = a.ep;
-      float cur_dist = lane == 0 ? hn_dist(a.base, a.d, cur, s.qv) : 0.f;
-      cur_dist = __shfl_sync(FULL, cur_dist, 0);
+      float cur_dist = hn_dist1(a, s, cur);
       dc++;
       uint32_t plen = 1;  // path entries so far (the last HN_PATH kept)
       if (lane == 0) s.path[0] = HEnt{cur_dist, cur};
@@ -292,7 +332,7 @@ __global__ void __launch_bounds__(HN_WARPS * 32) k_hnsw(HnswArgs a) {
           uint32_t deg;
           hn_row(a, cur, (uint32_t)lv, row, deg);  // the list of the node the pass started from
           for (uint32_t b0 = 0; b0 < deg; b0 += 32) {
-            const int cnt = hn_chunk(a, s, vis, row, deg, b0, lane);
+            const int cnt = hn_chunk(a, s, vis, row, deg, b0, lv == 0 && s.distinct, lane);
             dc += cnt;
             // improvements in list order, each against the running minimum
             uint32_t nc = cur, np = plen;
@@ -369,6 +409,9 @@ __global__ void __launch_bounds__(HN_WARPS * 32) k_hnsw(HnswArgs a) {
 }
 
 }  // namespace
+}  // namespace wv
+
+using namespace wv;
 
 // ================================================================ host side
 extern "C" {
@@ -439,6 +482,7 @@ int wv_load_hnsw(wv_ctx *c, const uint32_t *words, size_t count) {
   WV_CUDA(c, cudaMemcpyAsync(d_deg0, deg0.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
   WV_CUDA(c, cudaMemcpyAsync(d_upoff, up_off.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
   WV_CUDA(c, cudaMemcpyAsync(d_up, up.data(), up.size() * 4, cudaMemcpyHostToDevice, c->stream));
+  WV_CUDA(c, rows_repeat(d_l0, d_deg0, n, w0, c->d_hnsw_repeats(), c->sms, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
   c->hnsw.n = n;
   c->hnsw.w0 = w0;
@@ -484,6 +528,9 @@ int wv_search_hnsw(wv_ctx *c, const float *queries, uint32_t nq, int router, uin
   WV_CUDA(c, cudaMemsetAsync(bits, 0, slots * words * 4, c->stream));
   HnswArgs a{};
   a.base = c->base.as<float>();
+  a.base8 = c->base_int ? c->base8.as<uint8_t>() : nullptr;
+  a.xnorm = c->xnorm.as<float>();
+  a.repeats = c->d_hnsw_repeats();
   a.n = n;
   a.d = c->d;
   a.l0_ids = c->work["hn_l0"].as<uint32_t>();
