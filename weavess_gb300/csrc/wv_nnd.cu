@@ -614,6 +614,55 @@ __device__ __forceinline__ void ji_tile(const uint8_t *I, const uint8_t *J, uint
   }
 }
 
+// FP32 distances, in the reference's order, of i rows pa, pa + NW (NI of
+// them) and this lane's j rows pj, pj + 32 (NJ).  A lane's row is four
+// wavefronts of shared memory per 16 bytes, 12 operations of a pair: one pair
+// at a time the shared memory bound the join, two by two the arithmetic does.
+template <int NI, int NJ>
+__device__ __forceinline__ void jf_pairs(const float *ri, const float *rj, uint32_t fs, uint32_t d4, uint32_t pa,
+                                         uint32_t nw, uint32_t pj, uint32_t tj, uint32_t i0, uint32_t j0, uint32_t a,
+                                         float *G, uint32_t gs) {
+  bool need = false;
+  auto wanted = [&](int u, int v) {
+    const uint32_t gi = i0 + pa + u * nw, gj = j0 + pj + 32 * v;
+    return pj + 32 * v < tj && gj > (gj < a ? gi : 0u);
+  };
+#pragma unroll
+  for (int v = 0; v < NJ; v++) need |= wanted(0, v);  // (the first i row wants all the others do)
+  if (!need) return;
+  const float4 *x[NI], *y[NJ];
+#pragma unroll
+  for (int u = 0; u < NI; u++) x[u] = reinterpret_cast<const float4 *>(ri + (size_t)(pa + u * nw) * fs);
+#pragma unroll
+  for (int v = 0; v < NJ; v++) y[v] = reinterpret_cast<const float4 *>(rj + (size_t)min(pj + 32 * v, tj - 1) * fs);
+  float dist[NI][NJ];
+#pragma unroll
+  for (int u = 0; u < NI; u++)
+#pragma unroll
+    for (int v = 0; v < NJ; v++) dist[u][v] = 0.f;
+#pragma unroll 2
+  for (uint32_t k = 0; k < d4; k++) {
+    float4 xk[NI], yk[NJ];
+#pragma unroll
+    for (int u = 0; u < NI; u++) xk[u] = x[u][k];
+#pragma unroll
+    for (int v = 0; v < NJ; v++) yk[v] = y[v][k];
+#pragma unroll
+    for (int u = 0; u < NI; u++)
+#pragma unroll
+      for (int v = 0; v < NJ; v++) dist[u][v] = __fadd_rn(dist[u][v], group4(xk[u], yk[v]));
+  }
+#pragma unroll
+  for (int u = 0; u < NI; u++)
+#pragma unroll
+    for (int v = 0; v < NJ; v++) {
+      if (!wanted(u, v)) continue;
+      const uint32_t gi = i0 + pa + u * nw, gj = j0 + pj + 32 * v;
+      G[(size_t)gj * gs + gi] = dist[u][v];
+      if (gj < a) G[(size_t)gi * gs + gj] = dist[u][v];
+    }
+}
+
 // the local join of nodes [n0, n1), a node per block at a time.  I8: integer
 // rows in [0, 255] from the byte copy of the base (d a multiple of 16, d <=
 // 256); else FP32 rows, every distance folded in the reference's order.
@@ -713,17 +762,13 @@ __global__ void __launch_bounds__(I8 ? JI_THREADS : J_THREADS)
           __syncthreads();
           // warps take i rows, lanes take j rows; a pair of new rows is
           // computed once (the distance is symmetric bit for bit)
-          for (uint32_t pa = warp; pa < ti; pa += NW) {
-            const uint32_t gi = i0 + pa;
-            for (uint32_t pj0 = 0; pj0 < tj; pj0 += 32) {
-              const uint32_t pj = pj0 + lane, gj = j0 + pj;
-              if (pj >= tj || gj <= (gj < a ? gi : 0u)) continue;
-              const float4 *x = reinterpret_cast<const float4 *>(ri + (size_t)pa * fs);
-              const float4 *y = reinterpret_cast<const float4 *>(rj + (size_t)pj * fs);
-              float dist = 0.f;
-              for (uint32_t k = 0; k < d4; k++) dist = __fadd_rn(dist, group4(x[k], y[k]));
-              G[(size_t)gj * gs + gi] = dist;
-              if (gj < a) G[(size_t)gi * gs + gj] = dist;
+          for (uint32_t pa = warp; pa < ti; pa += 2 * NW) {
+            for (uint32_t pj = lane; pj - lane < tj; pj += 64) {
+              const bool i2 = pa + NW < ti, j2 = pj - lane + 32 < tj;
+              if (i2 && j2) jf_pairs<2, 2>(ri, rj, fs, d4, pa, NW, pj, tj, i0, j0, a, G, gs);
+              else if (i2) jf_pairs<2, 1>(ri, rj, fs, d4, pa, NW, pj, tj, i0, j0, a, G, gs);
+              else if (j2) jf_pairs<1, 2>(ri, rj, fs, d4, pa, NW, pj, tj, i0, j0, a, G, gs);
+              else jf_pairs<1, 1>(ri, rj, fs, d4, pa, NW, pj, tj, i0, j0, a, G, gs);
             }
           }
         }
