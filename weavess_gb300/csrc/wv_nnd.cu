@@ -487,8 +487,9 @@ __global__ void k_bucket_apply(Nnd s, const uint32_t *boff, const uint32_t *bcnt
 // a vote per 32 pairs.  The 100k x 128 build (S 10, L 40, R 100) takes
 // 31.2 ms; 33.2 ms with fragments widened on the fly and votes; its seven
 // joins had been 28.6 ms of 82 with the FP32 rows, the tcgen05 Gram tile and
-// the two atomics.  Six joins of 60k x 96 real-valued (FP32): 14.5 ms
-// against 18.6 ms.
+// the two atomics.  Six joins of 60k x 96 real-valued (FP32): 18.6 ms with
+// those atomics, 14.5 ms without, 13.4 ms with pairs taken two by two, 12.3 ms
+// with 32 new rows per tile (the other rows staged half as often).
 struct JoinOut {
   uint2 *ent;                  // {distance bits, candidate id}
   uint16_t *eq;                // the candidate's position in the node's list (new ++ old): the replay's key
@@ -500,6 +501,7 @@ struct JoinOut {
   const float *mx;             // pool maxima (-inf: empty pool)
 };
 struct JoinCfg {
+  uint32_t ti;     // FP32: rows per i tile
   uint32_t tj;     // rows per j tile
   uint32_t gcap;   // floats of G in shared memory; larger tiles take the block's slab of gscr
   float *gscr;
@@ -508,7 +510,7 @@ struct JoinCfg {
 };
 
 constexpr int J_THREADS = 256;
-constexpr int J_TI = 16;  // FP32: new rows per i tile
+constexpr int J_TI = 16, J_TI_BIG = 32;  // FP32: new rows per i tile (the larger where the tile stays below 64 KB)
 constexpr int J_TJ = 64;  // FP32: rows per j tile (new ++ old); fewer for long rows (the tile must fit shared memory)
 constexpr int JI_THREADS = 128;       // integer rows
 constexpr uint32_t JI_ROWS = 96;      // integer rows staged at once (all of a node's rows, or a 48 x 48 tile)
@@ -675,7 +677,7 @@ __global__ void __launch_bounds__(I8 ? JI_THREADS : J_THREADS)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t capt = s.capn + s.capo;
   const uint32_t stride = I8 ? ji_stride(s.d) : (((s.d + 3) & ~3u) + 4) * 4;  // bytes
-  const size_t rbytes = (size_t)(I8 ? JI_ROWS : J_TI + cf.tj) * stride;
+  const size_t rbytes = (size_t)(I8 ? JI_ROWS : cf.ti + cf.tj) * stride;
   float *Gs = reinterpret_cast<float *>(smem + rbytes);
   uint32_t *ids = cf.lscr ? cf.lscr + (size_t)blockIdx.x * (4 + NW) * capt : reinterpret_cast<uint32_t *>(Gs + cf.gcap);
   float *mx = reinterpret_cast<float *>(ids + capt);
@@ -744,9 +746,9 @@ __global__ void __launch_bounds__(I8 ? JI_THREADS : J_THREADS)
     } else {
       const uint32_t fs = stride / 4, d4 = s.d >> 2;
       float *ri = reinterpret_cast<float *>(smem);
-      float *rj = ri + (size_t)J_TI * fs;
-      for (uint32_t i0 = 0; i0 < a; i0 += J_TI) {
-        const uint32_t ti = min((uint32_t)J_TI, a - i0);
+      float *rj = ri + (size_t)cf.ti * fs;
+      for (uint32_t i0 = 0; i0 < a; i0 += cf.ti) {
+        const uint32_t ti = min(cf.ti, a - i0);
         for (uint32_t j0 = 0; j0 < tot; j0 += cf.tj) {
           const uint32_t tj = min(cf.tj, tot - j0);
           if (j0 + tj <= min(a, i0 + 1)) continue;  // both new: computed with the roles exchanged
@@ -1523,9 +1525,10 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
   // shared memory: the rows, then the tile and the node's lists as far as
   // they fit (else they live in global memory, a slab per block)
   const uint32_t fstride = ((c->d + 3) & ~3u) + 4;
+  jc.ti = (size_t)(J_TI_BIG + J_TJ) * fstride * 4 <= 64 * 1024 ? J_TI_BIG : J_TI;
   if (!join_i8)
-    while (jc.tj > 32 && (size_t)(J_TI + jc.tj) * fstride * 4 > 200 * 1024) jc.tj -= 32;
-  size_t join_smem = join_i8 ? (size_t)JI_ROWS * ji_stride(c->d) : (size_t)(J_TI + jc.tj) * fstride * 4;
+    while (jc.tj > 32 && (size_t)(jc.ti + jc.tj) * fstride * 4 > 200 * 1024) jc.tj -= 32;
+  size_t join_smem = join_i8 ? (size_t)JI_ROWS * ji_stride(c->d) : (size_t)(jc.ti + jc.tj) * fstride * 4;
   const uint32_t lwords = 4 + (join_i8 ? JI_THREADS : J_THREADS) / 32;  // words per list entry
   const size_t lists = (size_t)capt * lwords * 4;
   const bool lists_smem = join_smem + lists <= 200 * 1024;
