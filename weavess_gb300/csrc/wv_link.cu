@@ -111,8 +111,8 @@ __device__ __forceinline__ bool ssg_occludes(float pd, float rd, float djk, floa
 // ---- the prune with a block per node
 // The walk over a node's sorted pool needs its order only where distances
 // differ: the pool is sorted by (distance, id), and a node where equal
-// distances could have come out in another order is left to k_prune, which
-// sorts as std::sort does -- two picks of equal distance, a candidate
+// distances could have come out in another order is left to the EXACT form,
+// which sorts as std::sort does -- two picks of equal distance, a candidate
 // occluded by a pick of its own distance, equal distances on both sides of
 // the examination bound, or among the entries a Vamana refill takes.  Pools
 // of more than 1,024 entries are sorted a window at a time, as far as the
@@ -1449,6 +1449,27 @@ __global__ void k_ssg_repair(const float *base, uint32_t d, uint32_t n, uint32_t
   *nfront = 1;
 }
 
+// the first row whose degree is above w or that holds an id >= n (a warp a row)
+__global__ void k_conn_check(const uint32_t *ids, const uint32_t *deg, uint32_t n, uint32_t w, uint32_t *bad) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
+    const uint32_t dg = deg[v];
+    bool b = dg > w;
+    for (uint32_t j = lane; j < min(dg, w); j += 32) b |= ids[(size_t)v * w + j] >= n;
+    if (__any_sync(FULL, b) && lane == 0) atomicMin(bad, v);
+  }
+}
+
+// rows list[0..m) (a warp a row)
+__global__ void k_conn_gather(const uint32_t *ids, uint32_t w, const uint32_t *list, uint32_t m, uint32_t *out) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (r >= m) return;
+  const uint32_t *src = ids + (size_t)list[r] * w;
+  for (uint32_t j = lane; j < w; j += 32) out[(size_t)r * w + j] = src[j];
+}
+
 __global__ void k_mark_root(uint32_t *bits, uint32_t r, uint32_t *front) {
   bits[r >> 5] |= 1u << (r & 31);
   front[0] = r;
@@ -1938,22 +1959,70 @@ int conn_dfs_gpu(wv_ctx *c, uint32_t L_refine, uint32_t *added) {
   // copied) each batch is one search.
   //
   // The rows stay on the device (edges appended there, widths changed by a
-  // copy kernel); the host keeps the rows as they were, for the walk, and
-  // ep's row with its new edges, for the seeds.
+  // copy kernel).  What ep reaches does not depend on the walk's order, so it
+  // is found there, level by level; the host walks the other nodes, few as a
+  // rule, on a copy of their rows, and keeps ep's row with its new edges, for
+  // the seeds.  The 200k x 128 NSG link takes 142 ms so, 157 ms with all rows
+  // copied to the host, checked and walked there.
   const uint32_t n = c->n, ep = c->fg_ep, w0 = c->fg_w;
   uint32_t w = w0;
-  std::vector<uint32_t> deg(n), ids((size_t)n * w0);
-  WV_CUDA(c, cudaMemcpyAsync(deg.data(), c->fg_deg.p, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
-  WV_CUDA(c, cudaMemcpyAsync(ids.data(), c->fg_ids.p, (size_t)n * w0 * 4, cudaMemcpyDeviceToHost, c->stream));
-  WV_CUDA(c, cudaStreamSynchronize(c->stream));
-  *added = 0;
-  // the walk: flag times and the linked nodes
   constexpr uint32_t NONE = 0xffffffffu;
-  std::vector<uint32_t> ft(n, NONE), tgt, st;
-  for (uint32_t v = 0; v < n; v++) {
-    WV_CHECK(c, deg[v] <= w0, WV_ERR_STATE, "row %u: degree %u > width %u", v, deg[v], w0);
-    for (uint32_t j = 0; j < deg[v]; j++)
-      WV_CHECK(c, ids[(size_t)v * w0 + j] < n, WV_ERR_STATE, "row %u holds id %u >= n", v, ids[(size_t)v * w0 + j]);
+  *added = 0;
+  cudaError_t e0 = cudaSuccess;
+  const uint32_t words = (n + 31) / 32;
+  uint32_t *bits = c->buf<uint32_t>("cn_bits", words, &e0);
+  uint32_t *fa = c->buf<uint32_t>("cn_fa", n, &e0);
+  uint32_t *fb = c->buf<uint32_t>("cn_fb", n, &e0);
+  uint32_t *cnt = c->buf<uint32_t>("cn_cnt", 4, &e0);  // [0] frontier size, [1] first bad row
+  WV_CUDA(c, e0);
+  std::vector<uint32_t> deg(n);
+  uint32_t bad = NONE;
+  WV_CUDA(c, cudaMemsetAsync(cnt, 0xff, 8, c->stream));
+  k_conn_check<<<c->sms * 8, 256, 0, c->stream>>>(c->fg_ids.as<uint32_t>(), c->fg_deg.as<uint32_t>(), n, w0, cnt + 1);
+  WV_CUDA(c, cudaGetLastError());
+  WV_CUDA(c, cudaMemcpyAsync(&bad, cnt + 1, 4, cudaMemcpyDeviceToHost, c->stream));
+  WV_CUDA(c, cudaMemcpyAsync(deg.data(), c->fg_deg.p, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
+  WV_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (bad != NONE) {
+    WV_CHECK(c, deg[bad] <= w0, WV_ERR_STATE, "row %u: degree %u > width %u", bad, deg[bad], w0);
+    WV_CHECK(c, false, WV_ERR_STATE, "row %u holds an id >= n", bad);
+  }
+  std::vector<uint32_t> hbits(words), rest;
+  WV_CUDA(c, cudaMemsetAsync(bits, 0, (size_t)words * 4, c->stream));
+  k_mark_root<<<1, 1, 0, c->stream>>>(bits, ep, fa);
+  for (uint32_t nf = 1; nf;) {
+    WV_CUDA(c, cudaMemsetAsync(cnt, 0, 4, c->stream));
+    const uint32_t blocks = std::min<uint32_t>((nf + 7) / 8, (uint32_t)c->sms * 32);
+    k_bfs_level<<<blocks, 256, 0, c->stream>>>(c->fg_ids.as<uint32_t>(), c->fg_deg.as<uint32_t>(), w0, n, fa, nf, bits,
+                                               fb, cnt, c->d_status());
+    WV_CUDA(c, cudaGetLastError());
+    WV_CUDA(c, cudaMemcpyAsync(&nf, cnt, 4, cudaMemcpyDeviceToHost, c->stream));
+    WV_CUDA(c, cudaStreamSynchronize(c->stream));
+    std::swap(fa, fb);
+  }
+  WV_CUDA(c, cudaMemcpyAsync(hbits.data(), bits, (size_t)words * 4, cudaMemcpyDeviceToHost, c->stream));
+  WV_CUDA(c, cudaStreamSynchronize(c->stream));
+  for (uint32_t v = 0; v < n; v++)
+    if (!(hbits[v >> 5] >> (v & 31) & 1u)) rest.push_back(v);
+  if (rest.empty()) return WV_OK;
+  // the rows of the nodes ep does not reach
+  const uint32_t nr = (uint32_t)rest.size();
+  uint32_t *drows = c->buf<uint32_t>("cn_rows", (size_t)nr * w0, &e0);
+  WV_CUDA(c, e0);
+  std::vector<uint32_t> ids((size_t)nr * w0), at(n, NONE), ep_row(deg[ep]);
+  WV_CUDA(c, cudaMemcpyAsync(fa, rest.data(), (size_t)nr * 4, cudaMemcpyHostToDevice, c->stream));
+  k_conn_gather<<<(nr + 7) / 8, 256, 0, c->stream>>>(c->fg_ids.as<uint32_t>(), w0, fa, nr, drows);
+  WV_CUDA(c, cudaGetLastError());
+  WV_CUDA(c, cudaMemcpyAsync(ids.data(), drows, ids.size() * 4, cudaMemcpyDeviceToHost, c->stream));
+  if (deg[ep])
+    WV_CUDA(c, cudaMemcpyAsync(ep_row.data(), c->fg_ids.as<uint32_t>() + (size_t)ep * w0, (size_t)deg[ep] * 4,
+                               cudaMemcpyDeviceToHost, c->stream));
+  WV_CUDA(c, cudaStreamSynchronize(c->stream));
+  // the walk: flag times and the linked nodes
+  std::vector<uint32_t> ft(n, 0), tgt, st;
+  for (uint32_t i = 0; i < nr; i++) {
+    at[rest[i]] = i;
+    ft[rest[i]] = NONE;
   }
   auto walk = [&](uint32_t start, uint32_t t) {  // DFS (component_conn.cpp:31-57)
     st.assign(1, start);
@@ -1962,8 +2031,8 @@ int conn_dfs_gpu(wv_ctx *c, uint32_t L_refine, uint32_t *added) {
     while (!st.empty()) {
       uint32_t next = NONE;
       for (uint32_t j = 0; j < deg[tmp]; j++)
-        if (ft[ids[(size_t)tmp * w0 + j]] == NONE) {
-          next = ids[(size_t)tmp * w0 + j];
+        if (ft[ids[(size_t)at[tmp] * w0 + j]] == NONE) {
+          next = ids[(size_t)at[tmp] * w0 + j];
           break;
         }
       if (next == NONE) {
@@ -1977,16 +2046,12 @@ int conn_dfs_gpu(wv_ctx *c, uint32_t L_refine, uint32_t *added) {
       st.push_back(tmp);
     }
   };
-  walk(ep, 0);
-  for (uint32_t cur = 0;;) {  // findroot's first unflagged id only grows
-    while (cur < n && ft[cur] != NONE) cur++;
-    if (cur == n) break;
-    tgt.push_back(cur);
-    walk(cur, (uint32_t)tgt.size());
+  for (uint32_t v : rest) {  // findroot's first unflagged id only grows
+    if (ft[v] != NONE) continue;
+    tgt.push_back(v);
+    walk(v, (uint32_t)tgt.size());
   }
   const uint32_t m = (uint32_t)tgt.size();
-  if (m == 0) return WV_OK;
-  std::vector<uint32_t> ep_row(ids.begin() + (size_t)ep * w0, ids.begin() + (size_t)ep * w0 + deg[ep]);
   // re-lays the device rows out with width nw
   auto relayout = [&](uint32_t nw) -> int {
     DevBuf &ti = c->work["conn_ri"], &td = c->work["conn_rd"];
