@@ -6,11 +6,10 @@
 // threads depend on the OpenMP schedule: every split's std::mt19937 is seeded
 // 1998 ^ omp_get_thread_num(), and the trees' shuffles share rand()):
 //  * id lists: std::random_shuffle of 0..n-1 per tree on the context's rand()
-//    stream, tree by tree (n - 1 draws each, drawn on the host in order; the
-//    swaps run on the device, one thread per tree, in the inside-out form --
-//    before step i the list holds i at position i);
-//  * splits (meanSplit / selectDivision / planeSplit, :648-756): one warp per
-//    node -- the per-dimension means and variances of the first 101 ids are
+//    stream, tree by tree (n - 1 draws each, drawn on the host in order; on
+//    the device every value walks the steps that move it);
+//  * splits (meanSplit / selectDivision / planeSplit, :648-756): a block per
+//    node in the active levels, a warp below -- the per-dimension means and variances of the first 101 ids are
 //    folded in the reference's order with round-to-nearest adds and
 //    multiplies, one lane takes the top-5 variance scan, and the two Hoare
 //    partitions are done in parallel from their closed form: the k-th

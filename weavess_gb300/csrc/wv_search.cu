@@ -15,8 +15,8 @@
 //
 // Exactness (the plain FP32 form): result ids, pool order and the
 // DistCount/HopCount counters equal the reference's, because
-//  * distances are folded in the reference's order (one lane per row,
-//    wv_common.cuh), or -- when base and query are integers in [0, 255] and
+//  * distances are folded in the reference's order (a lane adds a row's sums,
+//    eight lanes read it, wv_search_common.cuh), or -- when base and query are integers in [0, 255] and
 //    d <= 256, so every partial sum is an integer below 2^24 and any order
 //    gives the same FP32 value -- summed by a coalesced warp reduction;
 //  * the seed pool is ordered as std::sort orders it: a bitonic sort on
