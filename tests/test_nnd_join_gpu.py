@@ -31,6 +31,8 @@ def data(kind):
         x = rng.normal(size=(4000, 24)).astype(np.float32)
         x[0] = 0.0
         return x
+    if kind in ("long", "longest"):  # real-valued rows whose tiles are smaller
+        return rng.normal(size=(700, 200 if kind == "long" else 1000)).astype(np.float32)
     if kind == "wide":  # integer rows of 256 dimensions
         return ds.int_mixture(1500, 256, 6, seed=3)[0]
     if kind == "odd":  # integer data without byte rows (d not a multiple of 16)
@@ -49,7 +51,8 @@ def same(ctx, g):
 @pytest.mark.parametrize("kind,S,K,L,R,cap", [
     ("ties", 10, 20, 40, 60, None), ("ties", 10, 20, 40, 60, "20000"), ("hub", 12, 20, 40, 100, None),
     ("hub_real", 12, 20, 40, 100, None), ("wide", 10, 20, 33, 40, None), ("odd", 10, 20, 40, 60, None),
-    ("narrow", 30, 60, 256, 150, None), ("narrow", 1, 1, 1, 1, None)])
+    ("narrow", 30, 60, 256, 150, None), ("narrow", 1, 1, 1, 1, None), ("long", 20, 20, 40, 60, None),
+    ("longest", 20, 20, 40, 60, None)])
 def test_join_matches_oracle(ctx, kind, S, K, L, R, cap, monkeypatch):
     if cap:
         monkeypatch.setenv("WV_NND_OFFER_CAP", cap)
