@@ -61,3 +61,37 @@ def test_inter_insert_matches_oracle(ctx, link, kind, R):
     live = np.arange(w)[None, :] < deg[:, None]
     assert np.array_equal(ids[:, :w][live], want.ids[:, :w][live])
     assert np.array_equal(dist[:, :w][live].view(np.uint32), want.dist[:, :w][live].view(np.uint32))
+
+
+@pytest.mark.parametrize("kind,R", [("hub", 60), ("hub", 61), ("real", 62)])
+@pytest.mark.parametrize("link", ["nsg", "vamana", "clean", "ssg"])
+def test_few_spare_slots_match_oracle(ctx, link, kind, R):
+    """Rows with three, two and one spare slot: some of a batch's senders are
+    copied ahead, the others where they are inserted."""
+    test_inter_insert_matches_oracle(ctx, link, kind, R)
+
+
+@pytest.mark.parametrize("link", ["nsg", "vamana"])
+def test_repeated_builds_are_identical(ctx, link):
+    """Rows beyond the L2 and many mutual edges (refused insertions): the rows
+    must not depend on the order in which the vectors' copies land."""
+    base = ds.unit_mixture(300000, 128, 300, seed=8)[0]
+    ctx.upload_base(base)
+    ctx.srand(1)
+    ctx.init_random(10)
+    ctx.nnd_refine(10, 32, 44, 4, 60)
+    ids, dist, deg, _ = ctx.get_graph()
+    first = None
+    for _ in range(3):
+        ctx.srand(2)
+        ctx.set_graph(ids, deg, dist=dist)
+        if link == "nsg":
+            ctx.nsg_refine(50, 32, 300)
+        else:
+            ctx.vamana_refine(50, 32, 1.2)
+        g = ctx.get_graph()
+        rows = (g[0], g[1].view(np.uint32), g[2])
+        if first is None:
+            first = rows
+        else:
+            assert all(np.array_equal(x, y) for x, y in zip(first, rows))

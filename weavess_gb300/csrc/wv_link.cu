@@ -46,6 +46,7 @@
 #include "wv_scan.h"
 #include "wv_search.h"
 #include "wv_segsort.h"
+#include "wv_slots.cuh"
 
 namespace wv {
 namespace {
@@ -816,7 +817,7 @@ struct IIRow {
   // entries are taken, s unless one of them occludes it (the row stays as it
   // was), the farther ones unless s occludes them.
   bool kept;
-  unsigned long long free;  // slots not in use
+  Slots slots;
 };
 
 template <bool I8>
@@ -830,7 +831,9 @@ struct II {
     return I8 ? a.base8 + (size_t)w.sid[slot] * a.d
               : reinterpret_cast<const uint8_t *>(a.base + (size_t)w.sid[slot] * a.d);
   }
-  // starts the copy of row `id` into slot f (a warp); the caller waits
+  // starts the copy of row `id` into slot f (a warp); the caller waits.  A slot
+  // given back unwaited is not taken again before a wait (wv_slots.cuh): two
+  // copies into one slot could land in either order
   __device__ void stage(uint32_t f, uint32_t id) const {
     if (lane == 0) w.sid[f] = id;
     if (!a.cs) return;
@@ -841,6 +844,9 @@ struct II {
   __device__ void landed() const {
     cp_async_wait_all();
     __syncwarp();
+  }
+  __device__ uint32_t take(IIRow &r) const {
+    return r.slots.take([&]() { landed(); });
   }
   __device__ float dist(uint32_t x, uint32_t y) const {
     return pf_dist<I8>(vec(x), vec(y), a.d, I8 ? (int)__ldg(a.xnorm + w.sid[x]) : 0,
@@ -878,7 +884,7 @@ struct II {
     if (lane > 0 && lane < (int)deg) asc &= up0 < r.d[0];
     if (lane + 32 < (int)deg) asc &= up1 < r.d[1];
     r.kept = __all_sync(FULL, asc);
-    r.free = ~0ull >> (64 - w.NS);
+    r.slots.reset(w.NS);
   }
   __device__ void store(const IIRow &r, uint32_t *ids, float *dist) const {
 #pragma unroll
@@ -892,9 +898,10 @@ struct II {
   }
   // slots and vectors for the whole row
   __device__ void give_slots(IIRow &r) const {
+    r.slots.reclaim([&]() { landed(); });
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      unsigned long long f = r.free;  // entry j takes the j-th free slot
+      unsigned long long f = r.slots.free;  // entry j takes the j-th free slot
       const uint32_t j = lane + 32 * h;
       if (j < r.rs) {
         for (uint32_t k = 0; k < j; k++) f &= f - 1;
@@ -906,7 +913,7 @@ struct II {
       const uint32_t sl = j < 32 ? __shfl_sync(FULL, r.slot[0], j) : __shfl_sync(FULL, r.slot[1], j - 32);
       stage(sl, id);
     }
-    r.free &= ~used(r);
+    r.slots.free &= ~used(r);
     r.vvalid = true;
   }
   __device__ void all_pairs(IIRow &r) const {
@@ -940,7 +947,7 @@ struct II {
     const uint32_t R = a.R, NS = w.NS, rs = r.rs;
     const bool h0 = lane < (int)rs, h1 = lane + 32 < (int)rs;
     auto give_back = [&]() {
-      if (fs != INVALID) r.free |= 1ull << fs;
+      if (fs != INVALID) r.slots.give_back(fs);
     };
     if (__any_sync(FULL, (h0 && r.i[0] == s) || (h1 && r.i[1] == s))) return give_back();
     auto column = [&](uint32_t f, float (&x)[2]) {  // distances of the row's entries to slot f
@@ -955,8 +962,7 @@ struct II {
     };
     auto slot_for = [&]() {
       if (fs == INVALID) {
-        fs = __ffsll(r.free) - 1;
-        r.free &= r.free - 1;
+        fs = take(r);
         stage(fs, s);
       }
       landed();
@@ -995,7 +1001,7 @@ struct II {
     uint32_t nres = 0;
     if (quick) {
       if (__any_sync(FULL, (h0 && r.d[0] < sd && x[0] < sd) || (h1 && r.d[1] < sd && x[1] < sd))) {
-        r.free |= 1ull << fs;
+        r.slots.free |= 1ull << fs;  // (its copy has landed)
         return;
       }
       // the survivors, in order, with s after the nearer ones
@@ -1129,7 +1135,7 @@ struct II {
     __syncwarp();
     // the slots of entries that left (and s's, if it was not taken) are free;
     // those of pending vectors stay taken
-    r.free = (r.free | old_slots | (1ull << fs)) & ~used(r);
+    r.slots.free = (r.slots.free | old_slots | (1ull << fs)) & ~used(r);
   }
 };
 
@@ -1214,8 +1220,7 @@ __global__ void __launch_bounds__(II_WARPS * 32) k_ii_forward(IIArgs a) {
         hit[k][1] = __ballot_sync(FULL, lane + 32 < dg[k] && id[k][1] == n);
         fs[k] = INVALID;
         if (k < (int)a.spare && (hit[k][0] | hit[k][1]) && (r.vvalid || r.rs == R)) {
-          fs[k] = __ffsll(r.free) - 1;
-          r.free &= r.free - 1;
+          fs[k] = t.take(r);
           t.stage(fs[k], mk[k]);
         }
       }
@@ -1280,8 +1285,7 @@ __global__ void __launch_bounds__(II_WARPS * 32) k_ii_backward(IIArgs a) {
         nxt = INVALID;
         if (cur != INVALID) t.landed();
         if (q + 1 < nb && a.spare > 0 && r.vvalid) {
-          nxt = __ffsll(r.free) - 1;
-          r.free &= r.free - 1;
+          nxt = t.take(r);
           t.stage(nxt, __shfl_sync(FULL, ml, q + 1));
         }
         t.template apply<MODE>(r, m, sd, pos, cur);
