@@ -1195,6 +1195,7 @@ __global__ void __launch_bounds__(II_WARPS * 32) k_ii_forward(IIArgs a) {
         }
         if (!__shfl_sync(FULL, ok, 0)) return;
       }
+      __syncwarp();  // orders every lane's reads of the rows after the lanes' acquires (votes and shuffles do not)
       const uint32_t have = __ffs(~__ballot_sync(FULL, up != 0)) - 1;
       for (uint32_t k = 0; k < have; k++) level = max(level, __shfl_sync(FULL, up, k));
       // their rows (read past the L1, which other warps' rows may share lines with)
