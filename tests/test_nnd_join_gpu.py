@@ -79,3 +79,18 @@ def test_stale_init_distances(ctx):
     ctx.set_graph(g0.ids, g0.deg, dist=g0.dist)
     ctx.nnd_refine(10, 20, 30, 4, 40)
     same(ctx, O.nndescent(base, g0, 10, 20, 30, 4, 40, r))
+
+
+@pytest.mark.parametrize("kind", ["narrow", "hub", "long"])
+def test_join_in_chunks_of_list_entries(ctx, kind, monkeypatch):
+    """A join whose lists exceed a launch's limit runs in chunks of nodes."""
+    monkeypatch.setenv("WV_NND_LIST_CAP", "8000")
+    base = data(kind)
+    ctx.upload_base(base)
+    ctx.srand(1)
+    ctx.init_random(10)
+    st = ctx.nnd_refine(10, 20, 40, 5, 60)
+    assert st["chunks"] > 4  # joins
+    r = O.Rand(1)
+    same(ctx, O.nndescent(base, O.init_random(base, 10, r), 10, 20, 40, 5, 60, r))
+    assert ctx.rand() == r.next()

@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "wv_common.cuh"
+#include "wv_join_plan.h"
 #include "wv_mt.cuh"
 #include "wv_nnd.h"
 #include "wv_scan.h"
@@ -516,19 +517,24 @@ constexpr int JI_THREADS = 128;       // integer rows
 constexpr uint32_t JI_ROWS = 96;      // integer rows staged at once (all of a node's rows, or a 48 x 48 tile)
 constexpr uint32_t J_GCAP = 3072;     // floats of G in shared memory
 
-// occurrences of every id in the lists of nodes [n0, n1), a warp per node,
-// and the largest tile a node needs
-__global__ void k_occ_count(Nnd s, uint32_t n0, uint32_t n1, uint32_t *occ, unsigned long long *gmax) {
+// occurrences of every id in the lists of nodes [n0, n1), a warp per node, the
+// largest tile a node needs, and the list entries of all (over 10 million nodes
+// of long lists have more than 32 bits count)
+__global__ void k_occ_count(Nnd s, uint32_t n0, uint32_t n1, uint32_t *occ, unsigned long long *gmax,
+                            unsigned long long *lists) {
   const int lane = threadIdx.x & 31;
+  unsigned long long sum = 0;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t n = n0 + w; n < n1; n += nw) {
     const uint32_t a = s.lnew[n], b = s.lold[n];
     if (a == 0) continue;
     const unsigned long long g = (unsigned long long)(a + b) * (a | 1u);
     if (lane == 0 && g > J_GCAP) atomicMax(gmax, g);
+    sum += a + b;
     for (uint32_t t = lane; t < a + b; t += 32)
       atomicAdd(&occ[t < a ? s.nnew[(size_t)n * s.capn + t] : s.nold[(size_t)n * s.capo + (t - a)]], 1u);
   }
+  if (lane == 0 && sum) atomicAdd(lists, sum);
 }
 
 // nhood::insert's first test is against the pool's current maximum, the
@@ -1572,8 +1578,15 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
     dist_ok = h != 0;
   }
 
-  // one join over nodes [n0, n1); `whole`: all nodes at once.  Returns with
-  // *need > cap (and nothing applied) when the entries did not fit.
+  // list entries per launch (WV_NND_LIST_CAP caps them further)
+  uint64_t lists_max = JOIN_LISTS_MAX;
+  if (const char *env = getenv("WV_NND_LIST_CAP"))
+    lists_max = std::min<uint64_t>(lists_max, std::max<uint64_t>(1024u, (uint64_t)atol(env)));
+
+  // one join over nodes [n0, n1); `whole`: all nodes at once.  Nothing is
+  // applied when its lists exceed the limit (fits = false) or its offers the
+  // entry buffers (hs.cursor > cap).
+  bool fits = true;
   struct {
     unsigned long long cursor;
     uint32_t redo[4];
@@ -1581,20 +1594,20 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
   auto join = [&](uint32_t n0, uint32_t n1, bool whole, const uint32_t *mclr) -> int {
     WV_CUDA(c, cudaMemsetAsync(tcnt, 0, (size_t)n * 4, c->stream));
     const int ob = (int)std::min<uint32_t>((n1 - n0 + 7) / 8, (uint32_t)c->sms * 16);
-    unsigned long long *gmax = reinterpret_cast<unsigned long long *>(small) + 4, hg = 0;
+    unsigned long long *gmax = reinterpret_cast<unsigned long long *>(small) + 4, hc[2];  // largest tile, list entries
     WV_CUDA(c, cudaMemsetAsync(small, 0, 48, c->stream));
-    k_occ_count<<<ob, 256, 0, c->stream>>>(s, n0, n1, tcnt, gmax);
+    k_occ_count<<<ob, 256, 0, c->stream>>>(s, n0, n1, tcnt, gmax, gmax + 1);
     WV_CUDA(c, exclusive_scan_u32(tcnt, toff, n, scan_tmp, c->stream));
-    uint32_t tl[2];
-    WV_CUDA(c, cudaMemcpyAsync(&tl[0], toff + n - 1, 4, cudaMemcpyDeviceToHost, c->stream));
-    WV_CUDA(c, cudaMemcpyAsync(&tl[1], tcnt + n - 1, 4, cudaMemcpyDeviceToHost, c->stream));
     WV_CUDA(c, cudaMemsetAsync(tcur, 0, (size_t)n * 4, c->stream));
-    WV_CUDA(c, cudaMemcpyAsync(&hg, gmax, 8, cudaMemcpyDeviceToHost, c->stream));
+    WV_CUDA(c, cudaMemcpyAsync(hc, gmax, 16, cudaMemcpyDeviceToHost, c->stream));
     k_pool_max<<<nb, NODE_THREADS, 0, c->stream>>>(s, pmax);
     WV_CUDA(c, cudaGetLastError());
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
+    unsigned long long hg = hc[0];
+    fits = hc[1] <= lists_max;
+    if (!fits) return WV_OK;
     cudaError_t e2 = cudaSuccess;  // (of the buffers sized below)
-    jo.desc = c->buf<uint4>("of_d", (size_t)tl[0] + tl[1] + 1, &e2);
+    jo.desc = c->buf<uint4>("of_d", (size_t)hc[1] + 1, &e2);
     WV_CUDA(c, e2);
     uint32_t grid = std::min(jgrid, n1 - n0);
     if (jc.gcap == 0) hg = std::max<unsigned long long>(hg, J_GCAP);
@@ -1656,6 +1669,10 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
       while (!chunked && !done) {
         int rc = join(0, n, true, mclr);
         if (rc) return rc;
+        if (!fits) {
+          chunked = true;
+          break;
+        }
         if (hs.cursor <= cap) {
           done = true;
           S.offers += hs.cursor;
@@ -1678,21 +1695,15 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
         WV_CUDA(c, cudaStreamSynchronize(c->stream));
         uint32_t n0 = 0;
         while (n0 < n) {
-          // chunk: the most nodes whose offer upper bound fits `cap`
-          uint64_t acc = 0;
-          uint32_t n1 = n0;
-          while (n1 < n) {
-            const uint64_t a = h_lnew[n1], b = h_lold[n1];
-            const uint64_t ub = a * (a - (a > 0)) + 2 * a * b;  // 2 offers per pair
-            if (n1 > n0 && acc + ub > cap) break;
-            acc += ub;
-            n1++;
-          }
-          WV_CHECK(c, acc <= cap, WV_ERR_LIMIT, "node %u alone may produce %llu offers (> %llu)", n0,
-                   (unsigned long long)acc, (unsigned long long)cap);
+          const JoinChunk ch = join_chunk(h_lnew.data(), h_lold.data(), n0, n, JoinLimits{cap, lists_max});
+          const uint32_t n1 = ch.end;
+          WV_CHECK(c, ch.offers <= cap, WV_ERR_LIMIT, "node %u alone may produce %llu offers (> %llu)", n0,
+                   (unsigned long long)ch.offers, (unsigned long long)cap);
+          WV_CHECK(c, ch.lists <= lists_max, WV_ERR_LIMIT, "node %u alone lists %llu ids (> %llu)", n0,
+                   (unsigned long long)ch.lists, (unsigned long long)lists_max);
           int rc = join(n0, n1, false, nullptr);
           if (rc) return rc;
-          WV_CHECK(c, hs.cursor <= cap, WV_ERR_STATE, "a join chunk produced more offers than its bound");
+          WV_CHECK(c, fits && hs.cursor <= cap, WV_ERR_STATE, "a join chunk is larger than its bound");
           S.offers += hs.cursor;
           S.chunks++;
           rc = take_pairs(true);
