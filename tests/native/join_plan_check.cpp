@@ -52,6 +52,13 @@ int main() {
   uint32_t wrapped = 0;
   for (uint32_t i = 0; i < n; i++) wrapped += a[i] + b[i];
   if (wrapped == (uint64_t)n * 1010) return printf("the case does not wrap\n"), 1;
+  // the descriptors' memory: half of what is free or theirs, not less than
+  // they hold or a million, not more than 32 bits count
+  const uint64_t G = 1ull << 30;
+  if (join_lists_room(100 * G, 0, 16) * 16 > 50 * G || join_lists_room(100 * G, 0, 16) * 16 < 49 * G ||
+      join_lists_room(2 * G, 6 * G, 16) * 16 != 6 * G || join_lists_room(10 * G, 2 * G, 16) * 16 != 6 * G ||
+      join_lists_room(0, 0, 16) != 1u << 20 || join_lists_room(4096 * G, 0, 16) != JOIN_LISTS_MAX)
+    return printf("room for lists\n"), 1;
   printf("OK %ld\n", total + c);
   return 0;
 }

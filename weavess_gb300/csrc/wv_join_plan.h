@@ -12,6 +12,14 @@ struct JoinLimits {
 };
 constexpr uint64_t JOIN_LISTS_MAX = 0xffffffffull;
 
+// list entries whose descriptors (desc_bytes each) may be held: half of what is
+// free or held by them already (the rest of a join needs memory too), and not
+// below a million
+inline uint64_t join_lists_room(uint64_t free_bytes, uint64_t held_bytes, uint64_t desc_bytes) {
+  const uint64_t half = (free_bytes + held_bytes) / 2 / desc_bytes;
+  return std::min(JOIN_LISTS_MAX, std::max({half, held_bytes / desc_bytes, (uint64_t)1 << 20}));
+}
+
 struct JoinChunk {
   uint32_t end;            // nodes [n0, end)
   uint64_t offers, lists;  // at most so many offers; list entries

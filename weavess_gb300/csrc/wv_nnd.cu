@@ -1578,10 +1578,21 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
     dist_ok = h != 0;
   }
 
-  // list entries per launch (WV_NND_LIST_CAP caps them further)
-  uint64_t lists_max = JOIN_LISTS_MAX;
+  // list entries per launch: what their descriptors may take of the device's
+  // memory beside the entry buffers, asked where they have to grow
+  // (WV_NND_LIST_CAP caps them further)
+  uint64_t lists_cap = JOIN_LISTS_MAX, lists_max = 0;
   if (const char *env = getenv("WV_NND_LIST_CAP"))
-    lists_max = std::min<uint64_t>(lists_max, std::max<uint64_t>(1024u, (uint64_t)atol(env)));
+    lists_cap = std::min<uint64_t>(lists_cap, std::max<uint64_t>(1024u, (uint64_t)atol(env)));
+  auto lists_room = [&](uint64_t want) -> int {
+    const uint64_t held = c->work["of_d"].bytes;
+    lists_max = std::min<uint64_t>(lists_cap, held / sizeof(uint4));
+    if (want < lists_max) return WV_OK;
+    size_t free_b = 0, total_b = 0;
+    WV_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    lists_max = std::min(lists_cap, join_lists_room(free_b, held, sizeof(uint4)));
+    return WV_OK;
+  };
 
   // one join over nodes [n0, n1); `whole`: all nodes at once.  Nothing is
   // applied when its lists exceed the limit (fits = false) or its offers the
@@ -1604,10 +1615,14 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
     WV_CUDA(c, cudaGetLastError());
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
     unsigned long long hg = hc[0];
-    fits = hc[1] <= lists_max;
-    if (!fits) return WV_OK;
+    if (whole) {
+      const int rl = lists_room(hc[1]);
+      if (rl) return rl;
+      fits = hc[1] <= lists_max;
+      if (!fits) return WV_OK;
+    }
     cudaError_t e2 = cudaSuccess;  // (of the buffers sized below)
-    jo.desc = c->buf<uint4>("of_d", (size_t)hc[1] + 1, &e2);
+    jo.desc = c->buf<uint4>("of_d", (size_t)hc[1], &e2);
     WV_CUDA(c, e2);
     uint32_t grid = std::min(jgrid, n1 - n0);
     if (jc.gcap == 0) hg = std::max<unsigned long long>(hg, J_GCAP);
@@ -1695,15 +1710,17 @@ int nndescent_gpu(wv_ctx *c, const NndParams &p, NndStats *st) {
         WV_CUDA(c, cudaStreamSynchronize(c->stream));
         uint32_t n0 = 0;
         while (n0 < n) {
+          int rc = lists_room(JOIN_LISTS_MAX);
+          if (rc) return rc;
           const JoinChunk ch = join_chunk(h_lnew.data(), h_lold.data(), n0, n, JoinLimits{cap, lists_max});
           const uint32_t n1 = ch.end;
           WV_CHECK(c, ch.offers <= cap, WV_ERR_LIMIT, "node %u alone may produce %llu offers (> %llu)", n0,
                    (unsigned long long)ch.offers, (unsigned long long)cap);
           WV_CHECK(c, ch.lists <= lists_max, WV_ERR_LIMIT, "node %u alone lists %llu ids (> %llu)", n0,
                    (unsigned long long)ch.lists, (unsigned long long)lists_max);
-          int rc = join(n0, n1, false, nullptr);
+          rc = join(n0, n1, false, nullptr);
           if (rc) return rc;
-          WV_CHECK(c, fits && hs.cursor <= cap, WV_ERR_STATE, "a join chunk is larger than its bound");
+          WV_CHECK(c, hs.cursor <= cap, WV_ERR_STATE, "a join chunk produced more offers than its bound");
           S.offers += hs.cursor;
           S.chunks++;
           rc = take_pairs(true);
