@@ -47,3 +47,32 @@ def test_integer_rows_match_oracle(ctx, d):
             assert np.all(np.abs(dd - e) <= (d + 2) * 2.0**-24 * (e + 2 * 255.0**2 * d))
         ctx.set_expansion(0)
     ctx.set_precision("fp32")
+
+
+def test_upload_without_room_for_the_byte_copy():
+    """A device whose memory holds the base but not its byte copy: the upload
+    succeeds and the searches read the FP32 rows, with the same results."""
+    torch = pytest.importorskip("torch")
+    from weavess_gb300 import Context
+    rng = np.random.default_rng(9)
+    n, d = 2_000_000, 128
+    base = rng.integers(0, 256, (n, d), dtype=np.uint8).astype(np.float32)
+    query = rng.integers(0, 256, (40, d)).astype(np.float32)
+    rows = rng.integers(0, n, (n, 6), dtype=np.uint32)
+    out = []
+    for tight in (True, False):
+        ctx = Context(0)
+        hold = None
+        if tight:  # room for the rows, their norms and 96 MB; the byte copy takes 256
+            free, _ = torch.cuda.mem_get_info()
+            hold = torch.empty(free - (n * d * 4 + n * 4 + (96 << 20)), dtype=torch.uint8, device="cuda")
+        ctx.upload_base(base)
+        del hold
+        torch.cuda.empty_cache()
+        ctx.upload_graph(rows, np.full(n, 6, np.uint32))
+        ctx.srand(1)
+        out.append(ctx.search(query, 40, 10, entry="rand", return_dist=True))
+        ctx.close()
+    (i0, dc0, hc0, d0), (i1, dc1, hc1, d1) = out
+    assert np.array_equal(i0, i1) and (dc0, hc0) == (dc1, hc1)
+    assert np.array_equal(d0.view(np.uint32), d1.view(np.uint32))

@@ -306,19 +306,24 @@ int wv_upload_base(wv_ctx *c, const float *base, uint32_t n, uint32_t d) {
   WV_CUDA(c, cudaMemcpyAsync(&hok, ok, 4, cudaMemcpyDeviceToHost, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
   c->base_int = hok == 1;
+  bool bytes = false;
   if (c->base_int) {
     // the distance kernels use |q|^2 + |x|^2 - 2 q.x on integer data (exact)
     WV_CUDA(c, c->xnorm.ensure((size_t)n * 4));
     k_row_norms<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float>(), n, d, c->xnorm.as<float>());
     WV_CUDA(c, cudaGetLastError());
-    if (d % 16 == 0 && d <= 256) {
-      WV_CUDA(c, c->base8.ensure((size_t)n * d));
+    bytes = d % 16 == 0 && d <= 256;
+    if (bytes && c->base8.ensure((size_t)n * d) != cudaSuccess) {  // no room: the kernels read the FP32 rows
+      cudaGetLastError();
+      bytes = false;
+    }
+    if (bytes) {
       k_pack8<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float4>(), (size_t)n * d / 4, c->base8.as<uint32_t>());
       WV_CUDA(c, cudaGetLastError());
     }
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
   }
-  if (!(c->base_int && d % 16 == 0 && d <= 256)) c->base8.release();
+  if (!bytes) c->base8.release();
   return WV_OK;
 }
 

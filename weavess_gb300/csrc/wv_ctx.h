@@ -55,8 +55,9 @@ struct wv_ctx {
   uint32_t n = 0, d = 0;
   bool base_int = false;  // every value an integer in [0, 255]
   wv::DevBuf xnorm;       // squared norm of every base row (when base_int: exact)
-  // the rows as bytes (when base_int, d a multiple of 16 up to 256; released
-  // otherwise): exact, a quarter of the FP32 rows' traffic
+  // the rows as bytes (when base_int, d a multiple of 16 up to 256 and the
+  // device has room; released otherwise): exact, a quarter of the FP32 rows'
+  // traffic
   wv::DevBuf base8;
   // low-precision copy of the base for candidate distances
   int storage = 0;
