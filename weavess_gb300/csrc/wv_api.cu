@@ -118,7 +118,7 @@ SearchArgs wv::search_args(wv_ctx *c, const float *d_q, uint32_t nq, const uint3
   a.status = c->d_status();
   a.int_exact = c->base_int;
   a.xnorm = c->xnorm.as<float>();
-  a.base8 = c->base_int ? c->base8.as<uint8_t>() : nullptr;
+  a.base8 = c->base_int && c->d <= SEARCH_I8_D ? c->base8.as<uint8_t>() : nullptr;
   a.storage = c->storage;
   a.qbase = c->qbase.p;
   a.qscale = c->qscale.as<float>();

@@ -64,7 +64,7 @@ struct CloserLess {  // std::less<CloserFirst>: a min-heap by distance (index.h:
 
 struct HnswArgs {
   const float *base;
-  const uint8_t *base8;  // integer base (d a multiple of 16 up to 256): the rows as bytes, or null
+  const uint8_t *base8;  // integer base (d a multiple of 16 up to SEARCH_I8_D): the rows as bytes, or null
   const float *xnorm;    // squared row norms (integer data)
   uint32_t n, d;
   const int *repeats;    // 0 there: no layer-0 list holds an id twice within 32 entries
@@ -528,7 +528,7 @@ int wv_search_hnsw(wv_ctx *c, const float *queries, uint32_t nq, int router, uin
   WV_CUDA(c, cudaMemsetAsync(bits, 0, slots * words * 4, c->stream));
   HnswArgs a{};
   a.base = c->base.as<float>();
-  a.base8 = c->base_int ? c->base8.as<uint8_t>() : nullptr;
+  a.base8 = c->base_int && c->d <= SEARCH_I8_D ? c->base8.as<uint8_t>() : nullptr;
   a.xnorm = c->xnorm.as<float>();
   a.repeats = c->d_hnsw_repeats();
   a.n = n;

@@ -1533,7 +1533,7 @@ int run_build_search(wv_ctx *c, const float *d_queries, uint32_t nq, const uint3
   a.vlimit = vlimit;
   a.int_exact = c->base_int;
   a.xnorm = c->xnorm.as<float>();
-  a.base8 = c->base_int ? c->base8.as<uint8_t>() : nullptr;
+  a.base8 = c->base_int && c->d <= SEARCH_I8_D ? c->base8.as<uint8_t>() : nullptr;
   int nb = (int)std::min<size_t>((size_t)blocks, ((size_t)nq + search_warps_per_block() - 1) / search_warps_per_block());
   WV_CUDA(c, launch_search_exact(a, std::max(nb, 1), c->stream));
   return WV_OK;

@@ -414,7 +414,7 @@ __device__ __forceinline__ float batch_dist(const float *__restrict__ base, uint
 }
 
 // distances of `cnt` (<= 32) integer rows -- ids in lanes 0..cnt-1 of `my` --
-// from the byte copy of the base (d a multiple of 16 up to 256) to an integer
+// from the byte copy of the base (d a multiple of 16 up to SEARCH_I8_D) to an integer
 // query (qc: this lane's 16 bytes of it, query_chunk_i8): |q|^2 + |x|^2 - 2 q.x in 32-bit integers, below 2^24, so
 // the FP32 value of the reference's sum.  G lanes read a row in 16-byte
 // chunks, 32 / G rows per pass, G passes for 32 rows with their loads issued
@@ -458,10 +458,10 @@ __device__ __forceinline__ uint32_t rows_dot_i8(const uint8_t *__restrict__ base
   return __shfl_sync(FULL, dot[0], (lane % RPP) * G + lane / RPP);
 }
 
-// the same with the lanes per row taken at run time (other d), a pass at a time
+// the same with the lanes per row taken at run time (d <= 64), a pass at a time
 __device__ __forceinline__ uint32_t rows_dot_i8_any(const uint8_t *__restrict__ base8, uint32_t d, uint32_t my, int cnt,
                                                     uint4 qc, int lane) {
-  const int ch = (int)(d / 16), G = ch > 8 ? 16 : ch > 4 ? 8 : ch > 2 ? 4 : 2, rpp = 32 / G;
+  const int ch = (int)(d / 16), G = ch > 2 ? 4 : 2, rpp = 32 / G;
   const int sub = lane & (G - 1), grp = lane / G;
   uint32_t out = 0;
 #pragma unroll 4
@@ -481,14 +481,14 @@ __device__ __forceinline__ uint32_t rows_dot_i8_any(const uint8_t *__restrict__ 
 __device__ __forceinline__ float rows_dist_i8(const uint8_t *__restrict__ base8, const float *__restrict__ xnorm,
                                               uint32_t d, uint32_t my, int cnt, uint4 qc, float qn, int lane) {
   const int xn = lane < cnt ? (int)__ldg(xnorm + my) : 0;
-  const uint32_t dot = d > 64 && d <= 128 ? rows_dot_i8<8>(base8, d, my, cnt, qc, lane)
-                                          : rows_dot_i8_any(base8, d, my, cnt, qc, lane);
+  const uint32_t dot = d > 64 ? rows_dot_i8<8>(base8, d, my, cnt, qc, lane)
+                              : rows_dot_i8_any(base8, d, my, cnt, qc, lane);
   return (float)((int)qn + xn - 2 * (int)dot);
 }
 
 // the 16 bytes of an integer query (qv: d FP32 values) this lane multiplies
 __device__ __forceinline__ uint4 query_chunk_i8(const float *qv, uint32_t d, int lane) {
-  const uint32_t ch = d / 16, G = ch > 8 ? 16 : ch > 4 ? 8 : ch > 2 ? 4 : 2, sub = lane & (G - 1);
+  const uint32_t ch = d / 16, G = ch > 4 ? 8 : ch > 2 ? 4 : 2, sub = lane & (G - 1);
   uint32_t w[4] = {0u, 0u, 0u, 0u};
   if (sub < ch) {
 #pragma unroll
