@@ -160,11 +160,12 @@ __device__ void sort_seeds(WarpSmem &s, int L, uint32_t hwords, uint32_t *gscrat
 }
 
 
+template <bool LP>
 __device__ __forceinline__ float cand_dist(const SearchArgs &a, bool ints, uint32_t my, int cnt, const float *qv,
                                            uint4 qc, int lane, float qn) {
   // bytes of integer data: the exact value, as FP32 and bf16 rows give it
   if (ints && a.base8 && a.storage != 2) return rows_dist_i8(a.base8, a.xnorm, a.d, my, cnt, qc, qn, lane);
-  if (a.storage != 0)
+  if (LP)
     // the norm form unless integer data at d > 128 (where only the
     // difference form stays exact)
     return lowp_rows_dist(LowpRows{a.qbase, a.qscale, (ints && a.d > 128) ? nullptr : a.qnorm, a.storage, a.d}, my,
@@ -195,7 +196,12 @@ __device__ __forceinline__ float shifted_seed_dist(const float *__restrict__ bas
 //   marked visited, and every visited (id, dist) -- the seeds in drawn order,
 //   then each newly visited id in visit order -- is appended to the query's
 //   visit list (vis, vcap apart, vlimit entries kept, count in vcnt).
-template <bool BUILD>
+// LP: candidates from the low-precision copy, an exact rerank at the end.
+//   One kernel for both kinds of rows was slower with either (its registers go
+//   to whichever path needs the most): 10,000 queries at L = 100 over 60k unit
+//   vectors of d = 96 take 1.74 ms with fp8 candidates and took 2.20 ms, with
+//   FP32 rows 1.70 ms and 1.84 ms.
+template <bool BUILD, bool LP>
 __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -258,7 +264,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         id = 0;
       }
       const float dist = (!BUILD && a.seed_shift) ? (lane < cnt ? shifted_seed_dist(a.base, a.d, id, s.qv) : 0.f)
-                                                 : cand_dist(a, ints, id, cnt, s.qv, qc, lane, qn);
+                                                 : cand_dist<LP>(a, ints, id, cnt, s.qv, qc, lane, qn);
       if (lane < cnt) {
         drawn[b + lane] = DI{dist, id};
         if (BUILD && nvis + lane < a.vlimit) vis_out[nvis + lane] = DI{dist, id};
@@ -345,7 +351,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         const int cnt = (int)min(32u, nfresh - b);
         const uint32_t raw = lane < cnt ? s.si[b + lane] : 0u;
         const uint32_t my = raw & ID_MASK;
-        const float dist = cand_dist(a, ints, my, cnt, s.qv, qc, lane, qn);
+        const float dist = cand_dist<LP>(a, ints, my, cnt, s.qv, qc, lane, qn);
         if (BUILD) {
           if (lane < cnt && nvis + lane < a.vlimit) vis_out[nvis + lane] = DI{dist, my};
           nvis += cnt;
@@ -480,7 +486,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
       k = first_flag(pi, next, L, lane);
     }
     // ---- exact FP32 rerank of the final pool (low-precision storage) ----
-    if (!BUILD && a.storage != 0 && a.rerank > 0) {
+    if (LP && a.rerank > 0) {
       const int R = min((int)a.rerank, L);
       float *xd = reinterpret_cast<float *>(s.hash);  // the visited set is done with
       uint32_t *xi = s.hash + R;
@@ -489,7 +495,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         const uint32_t id = lane < cnt ? (pi[b + lane] & ID_MASK) : 0u;
         const float ex = ints && a.base8 ? rows_dist_i8(a.base8, a.xnorm, a.d, id, cnt, qc, qn, lane)
                          : ints          ? batch_dist<true>(a.base, a.d, id, cnt, s.qv, lane, qn, a.d <= 128 ? a.xnorm : nullptr)
-                                         : batch_dist<false>(a.base, a.d, id, cnt, s.qv, lane);
+                                         : lane_rows_f32(a.base, a.d, id, cnt, s.qv, lane);
         if (lane < cnt) {
           xd[b + lane] = ex;
           xi[b + lane] = id;
@@ -529,12 +535,12 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   }
 }
 
-template <bool B>
+template <bool B, bool LP>
 int max_blocks(int W, size_t smem) {
-  if (cudaFuncSetAttribute(k_search<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_search<B, LP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return -1;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<B>, W * 32, smem) != cudaSuccess) return -1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<B, LP>, W * 32, smem) != cudaSuccess) return -1;
   return per_sm;
 }
 
@@ -562,8 +568,8 @@ int search_grid(uint32_t d, uint32_t Lmax, uint32_t cap, int device, SearchShape
   const size_t smem = search_block_smem(d, Lmax, cap, sh);
   if (smem > 227 * 1024) return 0;
   // (the build variant runs in the default shape only)
-  int per_sm = max_blocks<false>(sh.wpb, smem);
-  if (sh.wpb == WARPS) per_sm = std::min(per_sm, max_blocks<true>(sh.wpb, smem));
+  int per_sm = std::min(max_blocks<false, false>(sh.wpb, smem), max_blocks<false, true>(sh.wpb, smem));
+  if (sh.wpb == WARPS) per_sm = std::min(per_sm, max_blocks<true, false>(sh.wpb, smem));
   if (per_sm <= 0) {
     cudaGetLastError();
     return 0;
@@ -662,8 +668,9 @@ cudaError_t launch_search(const SearchArgs &a, SearchShape sh, int blocks, cudaS
   b.wide_hash = sh.wide ? 1 : 0;
   const size_t smem = search_block_smem(a.d, a.Lmax, a.cap, sh);
   if (a.vis && sh.wpb != WARPS) return cudaErrorInvalidValue;
-  if (a.vis) k_search<true><<<blocks, sh.wpb * 32, smem, stream>>>(b);
-  else k_search<false><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  if (a.vis) k_search<true, false><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  else if (a.storage != 0) k_search<false, true><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  else k_search<false, false><<<blocks, sh.wpb * 32, smem, stream>>>(b);
   return cudaGetLastError();
 }
 cudaError_t launch_search_exact(const SearchArgs &a, int blocks, cudaStream_t stream) {

@@ -10,8 +10,9 @@ namespace wv {
 
 // The searches read byte rows up to this dimension (8 chunks of 16 bytes a
 // row).  Beyond it the FP32 rows, a warp over each, are faster: 10,000 queries
-// at L = 150 over 100k integer rows of d = 256 take 3.33 ms and took 4.87 ms
-// with byte rows (d = 144: 3.40 and 5.31); at d = 128 it is 3.07 against 2.69.
+// at L = 150 over 100k integer rows of d = 256 take 3.23 ms and took 4.87 ms
+// with byte rows (d = 144: 3.30 and 5.31); at d = 128 byte rows take 2.62 ms,
+// FP32 rows took 3.07.
 constexpr uint32_t SEARCH_I8_D = 128;
 
 struct SearchArgs {
