@@ -76,3 +76,9 @@ def test_layered_route_with_repeated_ids(ctx, kind, d, router):
             want, wdc, whc = O.search_hnsw(base, query, words, L, router=router)
             assert np.array_equal(res, want) and (dc, hc) == (wdc, whc)
             same_bits(dist, query, base[res])
+
+
+@pytest.mark.parametrize("d", [8, 12, 16, 20])
+def test_short_rows_match_oracle(ctx, d):
+    """Rows about the length up to which a lane reads a whole row."""
+    test_route_matches_oracle(ctx, d, 24)

@@ -160,12 +160,16 @@ __device__ void sort_seeds(WarpSmem &s, int L, uint32_t hwords, uint32_t *gscrat
 }
 
 
-template <bool LP>
+// the rows a kernel's candidate distances are read from
+enum Rows { ROWS_F32, ROWS_LOWP, ROWS_SHORT };
+
+template <Rows RW>
 __device__ __forceinline__ float cand_dist(const SearchArgs &a, bool ints, uint32_t my, int cnt, const float *qv,
                                            uint4 qc, int lane, float qn) {
+  if (RW == ROWS_SHORT && !ints) return lane_rows_f32(a.base, a.d, my, cnt, qv, lane);
   // bytes of integer data: the exact value, as FP32 and bf16 rows give it
   if (ints && a.base8 && a.storage != 2) return rows_dist_i8(a.base8, a.xnorm, a.d, my, cnt, qc, qn, lane);
-  if (LP)
+  if (RW == ROWS_LOWP)
     // the norm form unless integer data at d > 128 (where only the
     // difference form stays exact)
     return lowp_rows_dist(LowpRows{a.qbase, a.qscale, (ints && a.d > 128) ? nullptr : a.qnorm, a.storage, a.d}, my,
@@ -196,12 +200,17 @@ __device__ __forceinline__ float shifted_seed_dist(const float *__restrict__ bas
 //   marked visited, and every visited (id, dist) -- the seeds in drawn order,
 //   then each newly visited id in visit order -- is appended to the query's
 //   visit list (vis, vcap apart, vlimit entries kept, count in vcnt).
-// LP: candidates from the low-precision copy, an exact rerank at the end.
-//   One kernel for both kinds of rows was slower with either (its registers go
-//   to whichever path needs the most): 10,000 queries at L = 100 over 60k unit
-//   vectors of d = 96 take 1.74 ms with fp8 candidates and took 2.20 ms, with
-//   FP32 rows 1.70 ms and 1.84 ms.
-template <bool BUILD, bool LP>
+// RW: ROWS_F32; ROWS_LOWP, candidates from the low-precision copy and an exact
+//   rerank at the end; ROWS_SHORT, FP32 rows of up to SHORT_D dimensions, a
+//   lane each (of eight lanes to a row most would have nothing to read).
+//   One kernel for all was slower with each (its registers go to whichever
+//   path needs the most).  10,000 queries at L = 100 over 60k unit vectors,
+//   now and in one kernel: d = 96, fp8 candidates 1.74 ms (2.20), FP32 rows
+//   1.70 (1.84); d = 4: 1.11 (1.35), 1.26 with eight lanes a row in a kernel
+//   of its own; d = 8: 1.23 and 1.39 so; at d = 12 eight lanes take 1.45 ms, a
+//   lane each took 1.49.
+constexpr uint32_t SHORT_D = 8;
+template <bool BUILD, Rows RW>
 __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -264,7 +273,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         id = 0;
       }
       const float dist = (!BUILD && a.seed_shift) ? (lane < cnt ? shifted_seed_dist(a.base, a.d, id, s.qv) : 0.f)
-                                                 : cand_dist<LP>(a, ints, id, cnt, s.qv, qc, lane, qn);
+                                                 : cand_dist<RW>(a, ints, id, cnt, s.qv, qc, lane, qn);
       if (lane < cnt) {
         drawn[b + lane] = DI{dist, id};
         if (BUILD && nvis + lane < a.vlimit) vis_out[nvis + lane] = DI{dist, id};
@@ -351,7 +360,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
         const int cnt = (int)min(32u, nfresh - b);
         const uint32_t raw = lane < cnt ? s.si[b + lane] : 0u;
         const uint32_t my = raw & ID_MASK;
-        const float dist = cand_dist<LP>(a, ints, my, cnt, s.qv, qc, lane, qn);
+        const float dist = cand_dist<RW>(a, ints, my, cnt, s.qv, qc, lane, qn);
         if (BUILD) {
           if (lane < cnt && nvis + lane < a.vlimit) vis_out[nvis + lane] = DI{dist, my};
           nvis += cnt;
@@ -486,7 +495,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
       k = first_flag(pi, next, L, lane);
     }
     // ---- exact FP32 rerank of the final pool (low-precision storage) ----
-    if (LP && a.rerank > 0) {
+    if (RW == ROWS_LOWP && a.rerank > 0) {
       const int R = min((int)a.rerank, L);
       float *xd = reinterpret_cast<float *>(s.hash);  // the visited set is done with
       uint32_t *xi = s.hash + R;
@@ -535,12 +544,12 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   }
 }
 
-template <bool B, bool LP>
+template <bool B, Rows RW>
 int max_blocks(int W, size_t smem) {
-  if (cudaFuncSetAttribute(k_search<B, LP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_search<B, RW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return -1;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<B, LP>, W * 32, smem) != cudaSuccess) return -1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<B, RW>, W * 32, smem) != cudaSuccess) return -1;
   return per_sm;
 }
 
@@ -568,8 +577,9 @@ int search_grid(uint32_t d, uint32_t Lmax, uint32_t cap, int device, SearchShape
   const size_t smem = search_block_smem(d, Lmax, cap, sh);
   if (smem > 227 * 1024) return 0;
   // (the build variant runs in the default shape only)
-  int per_sm = std::min(max_blocks<false, false>(sh.wpb, smem), max_blocks<false, true>(sh.wpb, smem));
-  if (sh.wpb == WARPS) per_sm = std::min(per_sm, max_blocks<true, false>(sh.wpb, smem));
+  int per_sm = std::min({max_blocks<false, ROWS_F32>(sh.wpb, smem), max_blocks<false, ROWS_LOWP>(sh.wpb, smem),
+                         max_blocks<false, ROWS_SHORT>(sh.wpb, smem)});
+  if (sh.wpb == WARPS) per_sm = std::min(per_sm, max_blocks<true, ROWS_F32>(sh.wpb, smem));
   if (per_sm <= 0) {
     cudaGetLastError();
     return 0;
@@ -668,9 +678,10 @@ cudaError_t launch_search(const SearchArgs &a, SearchShape sh, int blocks, cudaS
   b.wide_hash = sh.wide ? 1 : 0;
   const size_t smem = search_block_smem(a.d, a.Lmax, a.cap, sh);
   if (a.vis && sh.wpb != WARPS) return cudaErrorInvalidValue;
-  if (a.vis) k_search<true, false><<<blocks, sh.wpb * 32, smem, stream>>>(b);
-  else if (a.storage != 0) k_search<false, true><<<blocks, sh.wpb * 32, smem, stream>>>(b);
-  else k_search<false, false><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  if (a.vis) k_search<true, ROWS_F32><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  else if (a.storage != 0) k_search<false, ROWS_LOWP><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  else if (a.d <= SHORT_D) k_search<false, ROWS_SHORT><<<blocks, sh.wpb * 32, smem, stream>>>(b);
+  else k_search<false, ROWS_F32><<<blocks, sh.wpb * 32, smem, stream>>>(b);
   return cudaGetLastError();
 }
 cudaError_t launch_search_exact(const SearchArgs &a, int blocks, cudaStream_t stream) {
