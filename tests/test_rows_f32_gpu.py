@@ -82,3 +82,33 @@ def test_layered_route_with_repeated_ids(ctx, kind, d, router):
 def test_short_rows_match_oracle(ctx, d):
     """Rows about the length up to which a lane reads a whole row."""
     test_route_matches_oracle(ctx, d, 24)
+
+
+@pytest.mark.parametrize("kind,d", [("int", 64), ("int", 80), ("int", 128), ("int", 144), ("int", 256),
+                                    ("real", 188), ("real", 192)])
+def test_layered_route_every_way_of_reading_rows(ctx, kind, d):
+    """Byte rows (integer rows of 65 to 128 dimensions, integer and real-valued
+    queries in one batch), a lane per row, eight lanes per row."""
+    rng = np.random.default_rng(d)
+    n = 1200
+    if kind == "int":
+        base, query = ds.int_mixture(n, d, 8, seed=5, n_query=40)
+    else:
+        base, query = rng.normal(size=(n, d)).astype(np.float32), rng.normal(size=(40, d)).astype(np.float32)
+    words = [3, 1]
+    for v in range(n):
+        upper = v % 16 == 3
+        words += [v, 1 + upper, 36] + rng.choice(n, 36, replace=False).tolist()
+        if upper:
+            words += [8] + rng.choice(np.arange(3, n, 16), 8, replace=False).tolist()
+    words = np.array(words, np.uint32)
+    ctx.upload_base(base)
+    ctx.load_hnsw(words)
+    for real_at in (None, 1, 0):
+        q = query.copy()
+        if real_at is not None:
+            q[real_at::5] += 0.25
+        res, dist, dc, hc = ctx.search_hnsw(q, 40, 10, return_dist=True)
+        want, wdc, whc = O.search_hnsw(base, q, words, 40, router="hnsw")
+        assert np.array_equal(res, want) and (dc, hc) == (wdc, whc)
+        same_bits(dist, q, base[res])

@@ -20,12 +20,12 @@
 // bits, the warp takes the distances (the reference's value), then one lane
 // applies the queue updates in list order -- of those entries only that pass
 // the result queue's bound as it stood before the chunk (it only falls).
-// Integer data is read as bytes, real-valued rows by eight lanes each (a lane
-// per row read 32 lines per load).  What bounds it: the chain of a query's
-// expansions.  5,000 queries at L = 100 over 100k x 128: 1.85 -> 1.63 ms.
+// What bounds it: the chain of a query's expansions, and the queries resident at
+// once.  How the rows are read decides both, so each way has its kernel (HnRows).
 // The visited set is a per-warp bitset over the nodes, cleared through the list of words it touched (VisitedList::Reset
 // gives a fresh set for every layer and every SearchAtLayer).
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <vector>
 
@@ -64,7 +64,7 @@ struct CloserLess {  // std::less<CloserFirst>: a min-heap by distance (index.h:
 
 struct HnswArgs {
   const float *base;
-  const uint8_t *base8;  // integer base (d a multiple of 16 up to SEARCH_I8_D): the rows as bytes, or null
+  const uint8_t *base8;  // (HN_WARP) integer base, d from 65 to SEARCH_I8_D: the rows as bytes, or null
   const float *xnorm;    // squared row norms (integer data)
   uint32_t n, d;
   const int *repeats;    // 0 there: no layer-0 list holds an id twice within 32 entries
@@ -123,9 +123,28 @@ __device__ inline WarpState hn_carve(uint8_t *p, uint32_t d, uint32_t L) {
   return w;
 }
 
+// How a kernel reads the rows.  HN_LANE: a lane per FP32 row, 56 registers, 36
+// queries on an SM.  HN_WARP: the bytes of integer rows of 65 to 128 dimensions
+// (eight 16-byte chunks) for an integer query, eight lanes per FP32 row
+// otherwise; 80 registers, 24 queries: one query's chain is shorter, which is
+// worth the residency for byte rows and from 192 dimensions on.  Milliseconds
+// over 50k rows, HN_LANE / HN_WARP (bytes) / HN_WARP (FP32):
+//   d = 32, 5,000 queries, L = 50: 0.68 / 0.81 / 0.82
+//   d = 96, 5,000 queries, L = 50: 0.84 / 0.85 / 0.95; 1 query: 0.38 / 0.35 / 0.36
+//   d = 128, 5,000 queries, L = 200: 2.86 / 2.55 / 2.78; 1 query: 0.42 / 0.36 / 0.39
+//   d = 144, 5,000 queries, L = 50: 0.95 / - / 1.08; 100 queries: 0.49 / - / 0.46
+//   d = 192, 5,000 queries, L = 50: 1.12 / - / 1.10; 100 queries: 0.53 / - / 0.48
+//   d = 256, 5,000 queries, L = 50: 1.65 / - / 1.23; 100 queries: 0.58 / - / 0.50
+// (A kernel with the eight lanes alone, without the byte path, was compiled to
+// something half as fast.)
+enum HnRows { HN_LANE, HN_WARP };
+constexpr uint32_t HN_WARP_D = 192;
+
 // squared L2 (Distance::compare, include/weavess/distance.h) of `cnt` rows
 // (ids in lanes 0..cnt-1) and the query, as the reference's order gives it
+template <HnRows RW>
 __device__ __forceinline__ float hn_dist(const HnswArgs &a, const WarpState &s, uint32_t id, int cnt, int lane) {
+  if (RW == HN_LANE) return lane_rows_f32(a.base, a.d, id, cnt, s.qv, lane);
   return s.ints ? rows_dist_i8(a.base8, a.xnorm, a.d, id, cnt, s.qc, s.qn, lane)
                 : rows_dist_f32(a.base, a.d, id, cnt, s.qv, lane);
 }
@@ -180,6 +199,7 @@ __device__ __forceinline__ void hn_row(const HnswArgs &a, uint32_t node, uint32_
 
 // the fresh (not yet visited) entries of row[b0, b0 + 32) in list order into
 // s.ids / s.dist (distances in the reference's order); returns their count
+template <HnRows RW>
 __device__ int hn_chunk(const HnswArgs &a, WarpState &s, Bits &vis, const uint32_t *row, uint32_t deg, uint32_t b0,
                         bool distinct, int lane) {
   const uint32_t j = b0 + lane;
@@ -199,7 +219,7 @@ __device__ int hn_chunk(const HnswArgs &a, WarpState &s, Bits &vis, const uint32
   __syncwarp();
   const uint32_t cid = lane < cnt ? s.ids[lane] : 0u;
   if (cnt) {
-    const float dd = hn_dist(a, s, cid, cnt, lane);
+    const float dd = hn_dist<RW>(a, s, cid, cnt, lane);
     if (lane < cnt) s.dist[lane] = dd;
   }
   __syncwarp();
@@ -208,6 +228,7 @@ __device__ int hn_chunk(const HnswArgs &a, WarpState &s, Bits &vis, const uint32
 
 // SearchAtLayer (component_route.cpp:85-131 / 214-260) from `entry`,
 // pushing into the result queue (size rs, lane 0's copy is authoritative)
+template <HnRows RW>
 __device__ void hn_search_layer(const HnswArgs &a, WarpState &s, Bits &vis, SplitHeap cand, uint32_t entry,
                                 uint32_t &rs, unsigned long long &dc, unsigned long long &hc, int lane) {
   // the entry's distance, then both queues hold it
@@ -246,7 +267,7 @@ __device__ void hn_search_layer(const HnswArgs &a, WarpState &s, Bits &vis, Spli
     uint32_t deg;
     hn_row(a, node, 0, row, deg);
     for (uint32_t b0 = 0; b0 < deg; b0 += 32) {
-      const int cnt = hn_chunk(a, s, vis, row, deg, b0, s.distinct, lane);
+      const int cnt = hn_chunk<RW>(a, s, vis, row, deg, b0, s.distinct, lane);
       dc += cnt;
       // entries that a full result queue turns away now stay turned away (a
       // NaN in the queue voids its order: then every entry is looked at)
@@ -284,8 +305,10 @@ __device__ void hn_search_layer(const HnswArgs &a, WarpState &s, Bits &vis, Spli
   }
 }
 
-// (80 registers and a few spills: 1.61 ms where 126 take 2.07 and 64 take 1.89)
-__global__ void __launch_bounds__(HN_WARPS * 32, 6) k_hnsw(HnswArgs a) {
+// (HN_WARP: 80 registers and a few spills take 0.85 ms, 72 take 0.87: 50k x 96,
+// 5,000 queries, L = 50)
+template <HnRows RW>
+__global__ void __launch_bounds__(HN_WARPS * 32, RW == HN_LANE ? 9 : 6) k_hnsw(HnswArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpState s = hn_carve(smem + (size_t)warp * hn_warp_bytes(a.d, a.L), a.d, a.L);
@@ -310,7 +333,7 @@ __global__ void __launch_bounds__(HN_WARPS * 32, 6) k_hnsw(HnswArgs a) {
     for (int o = 16; o > 0; o >>= 1) qn += __shfl_xor_sync(FULL, qn, o);
     s.qn = qn;
     s.nan = false;
-    s.ints = a.base8 && __all_sync(FULL, qint);
+    s.ints = RW == HN_WARP && a.base8 && __all_sync(FULL, qint);
     __syncwarp();
     s.qc = s.ints ? query_chunk_i8(s.qv, a.d, lane) : make_uint4(0u, 0u, 0u, 0u);
     uint32_t rs = 0;
@@ -332,7 +355,7 @@ __global__ void __launch_bounds__(HN_WARPS * 32, 6) k_hnsw(HnswArgs a) {
           uint32_t deg;
           hn_row(a, cur, (uint32_t)lv, row, deg);  // the list of the node the pass started from
           for (uint32_t b0 = 0; b0 < deg; b0 += 32) {
-            const int cnt = hn_chunk(a, s, vis, row, deg, b0, lv == 0 && s.distinct, lane);
+            const int cnt = hn_chunk<RW>(a, s, vis, row, deg, b0, lv == 0 && s.distinct, lane);
             dc += cnt;
             // improvements in list order, each against the running minimum
             uint32_t nc = cur, np = plen;
@@ -370,10 +393,10 @@ __global__ void __launch_bounds__(HN_WARPS * 32, 6) k_hnsw(HnswArgs a) {
             entry = s.path[(plen - 1) % HN_PATH].id;
           }
         }
-        hn_search_layer(a, s, vis, cand, entry, rs, dc, hc, lane);
+        hn_search_layer<RW>(a, s, vis, cand, entry, rs, dc, hc, lane);
       }
     } else {
-      hn_search_layer(a, s, vis, cand, 0u, rs, dc, hc, lane);  // ROUTER_NSW: node 0
+      hn_search_layer<RW>(a, s, vis, cand, 0u, rs, dc, hc, lane);  // ROUTER_NSW: node 0
     }
     // ---- the K nearest through the CloserFirst queue (component_route.cpp:197-210)
     if (lane == 0) {
@@ -515,9 +538,15 @@ int wv_search_hnsw(wv_ctx *c, const float *queries, uint32_t nq, int router, uin
   WV_CUDA(c, cudaMemcpyAsync(c->q_buf.p, queries, (size_t)nq * c->d * 4, cudaMemcpyHostToDevice, c->stream));
   const size_t smem = (size_t)HN_WARPS * hn_warp_bytes(c->d, L);
   WV_CHECK(c, smem <= 227 * 1024, WV_ERR_LIMIT, "d=%u L=%u need %zu bytes of shared memory per block", c->d, L, smem);
-  WV_CUDA(c, cudaFuncSetAttribute(k_hnsw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // integer queries come with integer rows as a rule: the first one stands for
+  // the batch (every kernel takes any query)
+  bool bytes = c->base_int && c->base8.p && c->d > 64 && c->d <= SEARCH_I8_D;
+  for (uint32_t k = 0; bytes && k < c->d; k++)
+    bytes = queries[k] >= 0.f && queries[k] <= 255.f && queries[k] == std::rint(queries[k]);
+  const auto kern = bytes || c->d >= HN_WARP_D ? k_hnsw<HN_WARP> : k_hnsw<HN_LANE>;
+  WV_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  WV_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hnsw, HN_WARPS * 32, smem));
+  WV_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, HN_WARPS * 32, smem));
   WV_CHECK(c, per_sm > 0, WV_ERR_LIMIT, "the HNSW kernel does not fit an SM with d=%u L=%u", c->d, L);
   const uint32_t blocks = std::min<uint32_t>((uint32_t)c->sms * per_sm, (nq + HN_WARPS - 1) / HN_WARPS);
   const size_t slots = (size_t)blocks * HN_WARPS, words = (n + 31) / 32;
@@ -528,7 +557,7 @@ int wv_search_hnsw(wv_ctx *c, const float *queries, uint32_t nq, int router, uin
   WV_CUDA(c, cudaMemsetAsync(bits, 0, slots * words * 4, c->stream));
   HnswArgs a{};
   a.base = c->base.as<float>();
-  a.base8 = c->base_int && c->d <= SEARCH_I8_D ? c->base8.as<uint8_t>() : nullptr;
+  a.base8 = bytes ? c->base8.as<uint8_t>() : nullptr;
   a.xnorm = c->xnorm.as<float>();
   a.repeats = c->d_hnsw_repeats();
   a.n = n;
@@ -561,7 +590,7 @@ int wv_search_hnsw(wv_ctx *c, const float *queries, uint32_t nq, int router, uin
     WV_CUDA(c, e);
     WV_CUDA(c, cudaMemsetAsync(c->misc.p, 0, 32, c->stream));
     WV_CUDA(c, cudaMemsetAsync(c->d_status(), 0, 4, c->stream));
-    k_hnsw<<<blocks, HN_WARPS * 32, smem, c->stream>>>(a);
+    kern<<<blocks, HN_WARPS * 32, smem, c->stream>>>(a);
     WV_CUDA(c, cudaGetLastError());
     int st = 0;
     WV_CUDA(c, cudaMemcpyAsync(&st, c->d_status(), 4, cudaMemcpyDeviceToHost, c->stream));
