@@ -87,6 +87,8 @@ struct Stage {
         const int gr = r0 + 8 * ((warp % WG) * 4 + (lane >> 3));
         if (gk < K && gr + 8 <= R) {
           v[i] = __ldg(reinterpret_cast<const uint4 *>(X + (long long)gk * s_k + gr));
+        } else if (gk >= K || gr >= R) {  // (a batch of a few rows is mostly these)
+          v[i] = make_uint4(0, 0, 0, 0);
         } else {
           uint16_t t[8];
 #pragma unroll
@@ -97,6 +99,8 @@ struct Stage {
         const int e = tid + 128 * i, gr = r0 + e / (TK / 8), gk = k0 + (e % (TK / 8)) * 8;
         if (mode == 0 && gr < R && gk + 8 <= K) {
           v[i] = __ldg(reinterpret_cast<const uint4 *>(X + (long long)gr * s_row + gk));
+        } else if (gk >= K || gr >= R) {
+          v[i] = make_uint4(0, 0, 0, 0);
         } else {
           uint16_t t[8];
 #pragma unroll
