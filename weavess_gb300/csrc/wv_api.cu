@@ -52,11 +52,21 @@ __global__ void k_row_norms(const float *x, uint32_t n, uint32_t d, float *out) 
   }
 }
 
-// integer rows as bytes, four values per thread
-__global__ void k_pack8(const float4 *x, size_t count4, uint32_t *out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count4; i += (size_t)gridDim.x * blockDim.x) {
-    const float4 v = x[i];
-    out[i] = (uint32_t)v.x | (uint32_t)v.y << 8 | (uint32_t)v.z << 16 | (uint32_t)v.w << 24;
+// the same and the integer rows as bytes, from one read of them (d a multiple
+// of 4): G lanes (a power of two) per row
+__global__ void k_row_norms_pack8(const float4 *x, uint32_t n, uint32_t d4, uint32_t G, float *norm, uint32_t *out) {
+  const uint32_t sub = threadIdx.x & (G - 1);
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / G, nw = (gridDim.x * blockDim.x) / G;
+  for (uint32_t r0 = 0; r0 < n; r0 += nw) {  // (every lane of a warp takes every turn)
+    const uint32_t r = r0 + w;
+    float a = 0.f;
+    for (uint32_t k = sub; r < n && k < d4; k += G) {
+      const float4 v = x[(size_t)r * d4 + k];
+      a = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, a))));
+      out[(size_t)r * d4 + k] = (uint32_t)v.x | (uint32_t)v.y << 8 | (uint32_t)v.z << 16 | (uint32_t)v.w << 24;
+    }
+    for (uint32_t o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(FULL, a, o);
+    if (sub == 0 && r < n) norm[r] = a;
   }
 }
 
@@ -310,17 +320,19 @@ int wv_upload_base(wv_ctx *c, const float *base, uint32_t n, uint32_t d) {
   if (c->base_int) {
     // the distance kernels use |q|^2 + |x|^2 - 2 q.x on integer data (exact)
     WV_CUDA(c, c->xnorm.ensure((size_t)n * 4));
-    k_row_norms<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float>(), n, d, c->xnorm.as<float>());
-    WV_CUDA(c, cudaGetLastError());
     bytes = d % 16 == 0 && d <= 256;
     if (bytes && c->base8.ensure((size_t)n * d) != cudaSuccess) {  // no room: the kernels read the FP32 rows
       cudaGetLastError();
       bytes = false;
     }
-    if (bytes) {
-      k_pack8<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float4>(), (size_t)n * d / 4, c->base8.as<uint32_t>());
-      WV_CUDA(c, cudaGetLastError());
-    }
+    uint32_t G = 4;  // lanes per row
+    while (G < 32 && G < d / 4) G *= 2;
+    if (bytes)
+      k_row_norms_pack8<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float4>(), n, d / 4, G,
+                                                           c->xnorm.as<float>(), c->base8.as<uint32_t>());
+    else
+      k_row_norms<<<c->sms * 8, 256, 0, c->stream>>>(c->base.as<float>(), n, d, c->xnorm.as<float>());
+    WV_CUDA(c, cudaGetLastError());
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
   }
   if (!bytes) c->base8.release();
