@@ -34,3 +34,24 @@ def test_rows_with_repeated_ids(w):
         res, _, _ = ctx.search(query, 40, 10, entry="rand")
         assert all(len(set(r)) == 10 for r in res.tolist())
         ctx.set_expansion(0)
+
+
+@pytest.mark.parametrize("row,first,second", [(0, 0, 31), (777, 3, 4), (1499, 30, 31), (600, 33, 49), (5, 1, 40)])
+def test_one_row_with_a_repeated_id(row, first, second):
+    """A single row of 1,500 lists an id twice: its results must show that the
+    second one was passed over."""
+    from weavess_gb300 import Context
+    ctx = Context(0)
+    rng = np.random.default_rng(row)
+    n, w = 1500, 50
+    base = rng.integers(0, 256, (n, 32)).astype(np.float32)
+    ids = np.stack([rng.choice(n, w, replace=False) for _ in range(n)]).astype(np.uint32)
+    ids[row, second] = ids[row, first]
+    query = base[np.r_[row, rng.integers(0, n, 60)]]  # the row itself is reached
+    ctx.upload_base(base)
+    g = O.Graph(ids, np.zeros(ids.shape, np.float32), np.full(n, w, np.uint32), 0)
+    ctx.upload_graph(ids, g.deg, 0)
+    ctx.srand(4)
+    res, dc, hc = ctx.search(query, 40, 10, entry="rand")
+    want, wdc, whc = O.search(base, query, g, 40, O.Rand(4))
+    assert np.array_equal(res, want) and (dc, hc) == (wdc, whc)
