@@ -303,7 +303,7 @@ __device__ void beam_share(const SearchArgs &a, const BeamSmem &s, uint32_t kind
       uint32_t *xi = s.hash + R;
       const uint32_t id = lane < cnt ? (s.pi[c + lane] & ID_MASK) : 0u;
       const float ex = ints ? batch_dist<true>(a.base, a.d, id, cnt, s.qv, lane, qn, a.d <= 128 ? a.xnorm : nullptr)
-                            : batch_dist<false>(a.base, a.d, id, cnt, s.qv, lane);
+                            : lane_rows_f32(a.base, a.d, id, cnt, s.qv, lane);
       if (lane < cnt) {
         xd[c + lane] = ex;
         xi[c + lane] = id;
