@@ -105,7 +105,7 @@ SearchArgs wv::search_args(wv_ctx *c, const float *d_q, uint32_t nq, const uint3
   a.gids = c->gids.as<uint32_t>();
   a.gdeg = c->gdeg.as<uint32_t>();
   a.gw = c->gw;
-  a.repeats = c->d_repeats();
+  a.distinct = c->distinct;
   a.queries = d_q;
   a.nq = nq;
   a.nq_dev = nq_dev;
@@ -346,12 +346,16 @@ int wv_upload_graph(wv_ctx *c, const uint32_t *ids, const uint32_t *deg, uint32_
   WV_CHECK(c, ep < n, WV_ERR_ARG, "entry point %u >= n=%u", ep, n);
   for (uint32_t i = 0; i < n; i++) WV_CHECK(c, deg[i] <= width, WV_ERR_ARG, "row %u has degree %u > width %u", i, deg[i], width);
   WV_CUDA(c, cudaSetDevice(c->device));
+  c->distinct = false;
   WV_CUDA(c, c->gids.ensure((size_t)n * width * 4));
   WV_CUDA(c, c->gdeg.ensure((size_t)n * 4));
   WV_CUDA(c, cudaMemcpyAsync(c->gids.p, ids, (size_t)n * width * 4, cudaMemcpyHostToDevice, c->stream));
   WV_CUDA(c, cudaMemcpyAsync(c->gdeg.p, deg, (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
-  WV_CUDA(c, rows_repeat(c->gids.as<uint32_t>(), c->gdeg.as<uint32_t>(), n, width, c->d_repeats(), c->sms, c->stream));
+  int repeats = 1;
+  WV_CUDA(c, rows_repeat(c->gids.as<uint32_t>(), c->gdeg.as<uint32_t>(), n, width, c->d_repeats(), &repeats, c->sms,
+                         c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
+  c->distinct = !repeats;
   c->generation++;
   c->gn = n;
   c->gw = width;

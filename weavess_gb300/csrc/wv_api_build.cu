@@ -65,16 +65,19 @@ int wv_load_built_graph(wv_ctx *c) {
   WV_CHECK(c, c->fg_w <= SEARCH_MAX_WIDTH, WV_ERR_LIMIT, "graph width %u above %u", c->fg_w, SEARCH_MAX_WIDTH);
   WV_CUDA(c, cudaSetDevice(c->device));
   const size_t n = c->fg_n, w = c->fg_w;
+  c->distinct = false;
   WV_CUDA(c, c->gids.ensure(n * w * 4));
   WV_CUDA(c, c->gdeg.ensure(n * 4));
   WV_CUDA(c, cudaMemcpyAsync(c->gids.p, c->fg_ids.p, n * w * 4, cudaMemcpyDeviceToDevice, c->stream));
   WV_CUDA(c, cudaMemcpyAsync(c->gdeg.p, c->fg_deg.p, n * 4, cudaMemcpyDeviceToDevice, c->stream));
+  int repeats = 1;
   WV_CUDA(c, wv::rows_repeat(c->gids.as<uint32_t>(), c->gdeg.as<uint32_t>(), (uint32_t)n, (uint32_t)w, c->d_repeats(),
-                             c->sms, c->stream));
+                             &repeats, c->sms, c->stream));
   const uint32_t ep = c->fg_has_ep ? c->fg_ep : 0;
   uint32_t dep = 0;
   WV_CUDA(c, cudaMemcpyAsync(&dep, c->fg_deg.as<uint32_t>() + ep, 4, cudaMemcpyDeviceToHost, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
+  c->distinct = !repeats;
   c->ep_row.resize(dep);
   if (dep)
     WV_CUDA(c, cudaMemcpy(c->ep_row.data(), c->fg_ids.as<uint32_t>() + (size_t)ep * w, dep * 4,

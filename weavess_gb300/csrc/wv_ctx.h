@@ -75,6 +75,7 @@ struct wv_ctx {
   uint32_t gn = 0, gw = 0, ep = 0;
   std::vector<uint32_t> ep_row;  // host copy of the entry point's row
   std::vector<uint32_t> eps;     // SSG roots (eps_) of the search graph
+  bool distinct = false;         // no row lists an id twice within 32 slots (rows_repeat)
 
   // search scratch
   wv::DevBuf visited, touched;
@@ -95,6 +96,7 @@ struct wv_ctx {
   // in named work buffers; n = 0 while none is loaded
   struct {
     uint32_t n = 0, w0 = 0, wu = 0, ep = 0, max_level = 0, ep_layers = 0;
+    bool distinct = false;  // as above, of the layer-0 lists
   } hnsw;
 
   // KD-trees of the last INIT_KDT on this base (wv_kdt.cu), for the KD-tree
@@ -119,11 +121,7 @@ struct wv_ctx {
 
   unsigned *d_next() { return misc.as<unsigned>(); }
   unsigned long long *d_counters() { return reinterpret_cast<unsigned long long *>(misc.as<char>() + 8); }
-  // whether a row of the search graph / of the built graph a link searches /
-  // of the layered graph lists an id twice within 32 slots (rows_repeat)
-  int *d_repeats() { return reinterpret_cast<int *>(misc.as<char>() + 52); }
-  int *d_link_repeats() { return reinterpret_cast<int *>(misc.as<char>() + 56); }
-  int *d_hnsw_repeats() { return reinterpret_cast<int *>(misc.as<char>() + 60); }
+  int *d_repeats() { return reinterpret_cast<int *>(misc.as<char>() + 52); }  // rows_repeat's flag
   int *d_status() { return reinterpret_cast<int *>(misc.as<char>() + 32); }
   void release_work() {
     for (auto &kv : work) kv.second.release();

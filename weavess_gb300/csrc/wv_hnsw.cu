@@ -67,7 +67,7 @@ struct HnswArgs {
   const uint8_t *base8;  // (HN_WARP) integer base, d from 65 to SEARCH_I8_D: the rows as bytes, or null
   const float *xnorm;    // squared row norms (integer data)
   uint32_t n, d;
-  const int *repeats;    // 0 there: no layer-0 list holds an id twice within 32 entries
+  int distinct;          // no layer-0 list holds an id twice within 32 entries
   const uint32_t *l0_ids, *l0_deg;
   uint32_t w0;
   const uint32_t *up_off, *up;
@@ -95,7 +95,6 @@ struct WarpState {
   HEnt *path;     // HN_PATH
   HEnt *csh;      // HN_CSH: the shared part of the candidate queue
   bool ints;      // integer base and query, rows from the byte copy
-  bool distinct;  // no repeats in the layer-0 lists
   uint4 qc;       // this lane's bytes of an integer query
   float qn;       // its squared norm
   bool nan;       // the query met a distance that is not a number
@@ -267,7 +266,7 @@ __device__ void hn_search_layer(const HnswArgs &a, WarpState &s, Bits &vis, Spli
     uint32_t deg;
     hn_row(a, node, 0, row, deg);
     for (uint32_t b0 = 0; b0 < deg; b0 += 32) {
-      const int cnt = hn_chunk<RW>(a, s, vis, row, deg, b0, s.distinct, lane);
+      const int cnt = hn_chunk<RW>(a, s, vis, row, deg, b0, a.distinct, lane);
       dc += cnt;
       // entries that a full result queue turns away now stay turned away (a
       // NaN in the queue voids its order: then every entry is looked at)
@@ -316,7 +315,6 @@ __global__ void __launch_bounds__(HN_WARPS * 32, RW == HN_LANE ? 9 : 6) k_hnsw(H
   Bits vis{a.bits + (size_t)slot * a.words, a.touched + (size_t)slot * a.words, 0};
   const SplitHeap cand{s.csh, a.cand + (size_t)slot * a.ccap};
   unsigned long long dc = 0, hc = 0;
-  s.distinct = *a.repeats == 0;
   for (;;) {
     uint32_t q = 0;
     if (lane == 0) q = atomicAdd(a.next_query, 1u);
@@ -355,7 +353,7 @@ __global__ void __launch_bounds__(HN_WARPS * 32, RW == HN_LANE ? 9 : 6) k_hnsw(H
           uint32_t deg;
           hn_row(a, cur, (uint32_t)lv, row, deg);  // the list of the node the pass started from
           for (uint32_t b0 = 0; b0 < deg; b0 += 32) {
-            const int cnt = hn_chunk<RW>(a, s, vis, row, deg, b0, lv == 0 && s.distinct, lane);
+            const int cnt = hn_chunk<RW>(a, s, vis, row, deg, b0, lv == 0 && a.distinct, lane);
             dc += cnt;
             // improvements in list order, each against the running minimum
             uint32_t nc = cur, np = plen;
@@ -505,8 +503,10 @@ int wv_load_hnsw(wv_ctx *c, const uint32_t *words, size_t count) {
   WV_CUDA(c, cudaMemcpyAsync(d_deg0, deg0.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
   WV_CUDA(c, cudaMemcpyAsync(d_upoff, up_off.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
   WV_CUDA(c, cudaMemcpyAsync(d_up, up.data(), up.size() * 4, cudaMemcpyHostToDevice, c->stream));
-  WV_CUDA(c, rows_repeat(d_l0, d_deg0, n, w0, c->d_hnsw_repeats(), c->sms, c->stream));
+  int repeats = 1;
+  WV_CUDA(c, rows_repeat(d_l0, d_deg0, n, w0, c->d_repeats(), &repeats, c->sms, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
+  c->hnsw.distinct = !repeats;
   c->hnsw.n = n;
   c->hnsw.w0 = w0;
   c->hnsw.wu = wu;
@@ -559,7 +559,7 @@ int wv_search_hnsw(wv_ctx *c, const float *queries, uint32_t nq, int router, uin
   a.base = c->base.as<float>();
   a.base8 = bytes ? c->base8.as<uint8_t>() : nullptr;
   a.xnorm = c->xnorm.as<float>();
-  a.repeats = c->d_hnsw_repeats();
+  a.distinct = c->hnsw.distinct;
   a.n = n;
   a.d = c->d;
   a.l0_ids = c->work["hn_l0"].as<uint32_t>();

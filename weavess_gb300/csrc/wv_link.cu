@@ -1487,7 +1487,7 @@ namespace {
 
 int run_build_search(wv_ctx *c, const float *d_queries, uint32_t nq, const uint32_t *d_seeds, uint32_t seed_stride,
                      uint32_t L, const uint32_t *gids, const uint32_t *gdeg, uint32_t gw, DI *vis, uint32_t *vcnt,
-                     uint32_t vcap, uint32_t *out_ids, uint32_t K, const int *repeats, uint32_t vlimit = 0) {
+                     uint32_t vcap, uint32_t *out_ids, uint32_t K, bool distinct, uint32_t vlimit = 0) {
   if (vlimit == 0) vlimit = vcap;
   const uint32_t cap = gw + 32;
   int blocks = search_grid(c->d, L, cap, c->device);
@@ -1511,7 +1511,7 @@ int run_build_search(wv_ctx *c, const float *d_queries, uint32_t nq, const uint3
   a.gids = gids;
   a.gdeg = gdeg;
   a.gw = gw;
-  a.repeats = repeats;
+  a.distinct = distinct;
   a.queries = d_queries;
   a.nq = nq;
   a.seeds = d_seeds;
@@ -1603,6 +1603,9 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   cudaEventRecord(e0, c->stream);
   // host copies of what the host-side draws need
   std::vector<uint32_t> hdeg(n);
+  int repeats = 1;
+  WV_CUDA(c, rows_repeat(c->fg_ids.as<uint32_t>(), c->fg_deg.as<uint32_t>(), n, gw, c->d_repeats(), &repeats, c->sms,
+                         c->stream));
   WV_CUDA(c, cudaMemcpyAsync(hdeg.data(), c->fg_deg.p, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));
   auto host_row = [&](uint32_t v, std::vector<uint32_t> &out) -> int {
@@ -1615,7 +1618,6 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
   uint32_t *seed1 = c->buf<uint32_t>("seed1", p.L, &e);
   uint32_t *one = c->buf<uint32_t>("one", 4, &e);
   WV_CUDA(c, e);
-  WV_CUDA(c, rows_repeat(c->fg_ids.as<uint32_t>(), c->fg_deg.as<uint32_t>(), n, gw, c->d_link_repeats(), c->sms, c->stream));
   // ---- entry point (ComponentRefineEntryCentroid::EntryInner); SSG has none
   // (its RefineInner leaves the entry step out) and draws no rand() here
   uint32_t ep = 0;
@@ -1634,7 +1636,7 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
     DI *v1 = c->buf<DI>("vis1", (size_t)n + p.entry_L + 64, &e);
     WV_CUDA(c, e);
     rc = run_build_search(c, center, 1, seed1, p.entry_L, p.entry_L, c->fg_ids.as<uint32_t>(),
-                          c->fg_deg.as<uint32_t>(), gw, v1, one + 1, n + p.entry_L + 64, one, 1, c->d_link_repeats());
+                          c->fg_deg.as<uint32_t>(), gw, v1, one + 1, n + p.entry_L + 64, one, 1, !repeats);
     if (rc) return rc;
     WV_CUDA(c, cudaMemcpyAsync(&ep, one, 4, cudaMemcpyDeviceToHost, c->stream));
     WV_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1681,7 +1683,7 @@ int link_gpu(wv_ctx *c, const LinkParams &p, LinkStats *st) {
       int rc = ssg ? run_prop2(c, n0, cnt, p.L, vis, vcnt, vcap)
                    : run_build_search(c, c->base.as<float>() + (size_t)n0 * c->d, cnt, dseeds,
                                       shared_seeds ? 0 : p.L, p.L, c->fg_ids.as<uint32_t>(),
-                                      c->fg_deg.as<uint32_t>(), gw, vis, vcnt, vcap, nullptr, 1, c->d_link_repeats(),
+                                      c->fg_deg.as<uint32_t>(), gw, vis, vcnt, vcap, nullptr, 1, !repeats,
                                       vcap - ((vamana && !p.clean) ? 0 : gw));
       if (rc) return rc;
       int st0 = 0;
@@ -2135,7 +2137,7 @@ int conn_dfs_gpu(wv_ctx *c, uint32_t L_refine, uint32_t *added) {
       vis = c->buf<DI>("conn_vis", (size_t)B * vcap, &e);
       WV_CUDA(c, e);
       rc = run_build_search(c, dq, B, dseed, L_refine, L_refine, c->fg_ids.as<uint32_t>(), c->fg_deg.as<uint32_t>(),
-                            w, vis, dvc, vcap, dout, 1, nullptr);
+                            w, vis, dvc, vcap, dout, 1, false);
       if (rc) return rc;
       int st0 = 0;
       WV_CUDA(c, cudaMemcpyAsync(&st0, c->d_status(), 4, cudaMemcpyDeviceToHost, c->stream));

@@ -225,7 +225,6 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
   vis.touched = a.touched + (size_t)slot * a.words;
   unsigned long long dcount = 0, hcount = 0;
   const unsigned lt = (1u << lane) - 1u;
-  const bool distinct = a.repeats && *a.repeats == 0;
   float *pd = s.pd;
   uint32_t *pi = s.pi;
 
@@ -339,7 +338,7 @@ __global__ void __maxnreg__(128) k_search(SearchArgs a) {
           id = INVALID;
         }
         // a repeated id inside this chunk: only its first position visits it
-        const bool leader = distinct || (__ffs(__match_any_sync(FULL, id)) - 1) == lane;
+        const bool leader = a.distinct || (__ffs(__match_any_sync(FULL, id)) - 1) == lane;
         bool was_seed;
         const bool fresh = vis.test_and_set(id != INVALID && leader, id, lane, was_seed);
         const unsigned fm = __ballot_sync(FULL, fresh);
@@ -630,12 +629,13 @@ static __global__ void __launch_bounds__(RR_WARPS * 32)
       }
   }
 }
-cudaError_t rows_repeat(const uint32_t *ids, const uint32_t *deg, uint32_t n, uint32_t w, int *flag, int sms,
-                        cudaStream_t stream) {
+cudaError_t rows_repeat(const uint32_t *ids, const uint32_t *deg, uint32_t n, uint32_t w, int *flag, int *host,
+                        int sms, cudaStream_t stream) {
   const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), stream);
   if (e != cudaSuccess) return e;
   k_rows_repeat<<<sms * 8, RR_WARPS * 32, 0, stream>>>(ids, deg, n, w, flag);
-  return cudaGetLastError();
+  const cudaError_t x = cudaGetLastError();
+  return x != cudaSuccess ? x : cudaMemcpyAsync(host, flag, sizeof(int), cudaMemcpyDeviceToHost, stream);
 }
 
 // the dispatch order of a launch with per-query beams: a counting sort of

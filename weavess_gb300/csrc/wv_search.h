@@ -21,7 +21,7 @@ struct SearchArgs {
   const uint32_t *gids;  // graph rows, width gw
   const uint32_t *gdeg;
   uint32_t gw;
-  const int *repeats;  // 0 there: no row lists an id twice within 32 slots (rows_repeat); null: unknown
+  int distinct;  // no row lists an id twice within an aligned run of 32 slots (rows_repeat); 0: unknown
   const uint8_t *base8;  // integer base (d a multiple of 16 up to SEARCH_I8_D): the rows as bytes, or null
   const float *queries;  // nq x d
   uint32_t nq;
@@ -71,7 +71,7 @@ struct SearchArgs {
   const float *qnorm;  // squared norms of the low-precision rows
   uint32_t rerank;
   // 0: the exact traversal (k_search, the reference's expansion order);
-  // E >= 1: the throughput form (k_beam, wv_beam.cu), E pool entries
+  // E >= 1: the throughput form (k_beam, wv_beam.cuh), E pool entries
   // expanded per step, tensor-core row distances where the layout allows
   uint32_t parents;
   // the throughput form: warps per query (1, 2 or 4; set by launch_beam
@@ -113,15 +113,16 @@ int search_grid(uint32_t d, uint32_t Lmax, uint32_t cap, int device, SearchShape
 int search_grid(uint32_t d, uint32_t Lmax, uint32_t cap, int device);
 cudaError_t launch_search(const SearchArgs &a, SearchShape sh, int blocks, cudaStream_t stream);
 
-// *flag (device) = whether a row of the graph lists an id twice within an
-// aligned run of 32 slots: then the searches look for the first of equal
-// neighbours (a match over the warp, 380 cycles of a row's 1,900 of visited
-// tests), else they need not: 1,000 queries over 100k x 128 0.686 -> 0.678 ms,
-// 20,000 of mixed beams over 30k x 960 15.06 -> 14.92 ms
-cudaError_t rows_repeat(const uint32_t *ids, const uint32_t *deg, uint32_t n, uint32_t w, int *flag, int sms,
-                        cudaStream_t stream);
+// *host (valid once the stream is waited for; flag: a device word) = whether a
+// row of the graph lists an id twice within an aligned run of 32 slots: then
+// the searches look for the first of equal neighbours (a match over the warp,
+// 380 cycles of a row's 1,900 of visited tests), else they need not: 10,000
+// queries at L = 100 over a KNN graph of 100k x 128 1.63 -> 1.56 ms.  The kernels
+// have it as an argument or a variant (k_beam).
+cudaError_t rows_repeat(const uint32_t *ids, const uint32_t *deg, uint32_t n, uint32_t w, int *flag, int *host,
+                        int sms, cudaStream_t stream);
 
-// the throughput form (wv_beam.cu): candidate entries per warp for graph
+// the throughput form (wv_beam.cuh): candidate entries per warp for graph
 // width gw and E parents per step, the persistent grid of a shape, and the
 // launch (launch_search dispatches to it when a.parents > 0 and the search
 // is a route search without shifted seeds)

@@ -1,5 +1,5 @@
 // Pieces shared by the beam-search kernels (wv_search.cu: the exact
-// traversal; wv_beam.cu: the throughput form): the per-warp shared-memory
+// traversal; wv_beam.cuh: the throughput form): the per-warp shared-memory
 // sizes, pool scans, the visited set and the FP32 row distances.
 #pragma once
 #include <cstdint>
@@ -438,7 +438,7 @@ __device__ __forceinline__ float batch_dist(const float *__restrict__ base, uint
 // rows' bytes and one latency instead of four: 10,000 queries at L = 200 over
 // 300k x 128 6.50 -> 5.06 ms, 1,000 at L = 100 over 100k 0.79 -> 0.70 ms, the
 // candidate searches of a 200k NSG link 46 -> 35 ms.  The throughput form
-// (wv_beam.cu) keeps its tensor-core rows: its 10,000 learned queries took
+// (wv_beam.cuh) keeps its tensor-core rows: its 10,000 learned queries took
 // 2.03 ms with those and 2.38 ms with these.
 template <int G>
 __device__ __forceinline__ uint32_t rows_dot_i8(const uint8_t *__restrict__ base8, uint32_t d, uint32_t my, int cnt,
