@@ -345,8 +345,8 @@ __device__ __forceinline__ float rows_dist_f32(const float *__restrict__ base, u
 
 // distances of `cnt` rows (ids in lanes 0..cnt-1 of `my`) to the query.
 // INTS: warp-cooperative coalesced rows (any summation order is exact);
-// else in the reference's order.
-template <bool INTS>
+// else in the reference's order (LANES: a lane per row).
+template <bool INTS, bool LANES = false>
 __device__ __forceinline__ float batch_dist(const float *__restrict__ base, uint32_t d, uint32_t my, int cnt,
                                             const float *qv, int lane, float qn = 0.f,
                                             const float *__restrict__ xnorm = nullptr) {
@@ -420,6 +420,13 @@ __device__ __forceinline__ float batch_dist(const float *__restrict__ base, uint
       const int g = (lane - c0) & 7;
       const float t = __shfl_sync(FULL, y, ((g >> 2) << 4) | (((g >> 1) & 1) << 3) | ((g & 1) << 2));
       if (lane >= c0 && lane < c0 + G) out = dot ? qn + xn - 2.f * t : t;
+    }
+  } else if (LANES) {
+    if (lane < cnt) {
+      const float4 *row = reinterpret_cast<const float4 *>(base + (size_t)my * d);
+      const float4 *q4 = reinterpret_cast<const float4 *>(qv);
+#pragma unroll 8
+      for (uint32_t g = 0; g < d4; g++) out = __fadd_rn(out, group4(__ldg(row + g), q4[g]));
     }
   } else {
     out = rows_dist_f32(base, d, my, cnt, qv, lane);
