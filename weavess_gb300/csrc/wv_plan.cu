@@ -124,7 +124,7 @@ int enqueue(wv_plan *p) {
     const uint32_t Ls = rand_mode ? p->p.L_max : p->plain_L;
     WV_CUDA(c, cudaMemcpyAsync(p->sv.p, p->h_sv, (size_t)nqm * 4, cudaMemcpyHostToDevice, c->stream));
     WV_CUDA(c, seeds_rand_launch(p->sv.as<uint32_t>(), nqm, nq_dev, rand_mode ? p->d_L : nullptr, Ls, Ls, c->n,
-                                 p->seeds.as<uint32_t>(), Ls, c->d_status(), c->stream));
+                                 p->seeds.as<uint32_t>(), Ls, c->d_status(), c->sms, c->stream));
   }
   if (p->p.mode == WV_PLAN_LEARNED)
     return learn_enqueue(c, p->pfx.c_str(), p->d_q, nqm, nq_dev, p->p.K_max, p->d_K, p->d_out, p->d_dist,

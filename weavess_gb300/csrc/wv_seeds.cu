@@ -206,11 +206,11 @@ size_t seeds_rand_smem(uint32_t Lmax) { return (size_t)SEED_WARPS * (624 + pow2_
 
 cudaError_t seeds_rand_launch(const uint32_t *d_sv, uint32_t nq, const uint32_t *d_nq, const uint32_t *d_L,
                               uint32_t L, uint32_t Lmax, uint32_t N, uint32_t *d_out, uint32_t stride, int *d_status,
-                              cudaStream_t s) {
+                              int sms, cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
   if (Lmax <= 512) {
-    // enough blocks for the device first, then up to a warp of queries each
-    const uint32_t QB = std::min<uint32_t>(SB_QUERIES, (nq + 2 * 152 - 1) / (2 * 152));
+    // two blocks per SM first, then up to a warp of queries each
+    const uint32_t fill = 2 * (uint32_t)sms, QB = std::min<uint32_t>(SB_QUERIES, (nq + fill - 1) / fill);
     const size_t smem = (size_t)624 * (QB | 1u) * 4;
     auto go = [&](auto k) -> cudaError_t {
       const cudaError_t x = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -240,7 +240,7 @@ int draw_seeds_rand_device(wv_ctx *c, uint32_t nq, const uint32_t *d_L, uint32_t
   WV_CUDA(c, e);
   WV_CUDA(c, cudaMemcpyAsync(d_sv, sv.data(), (size_t)nq * 4, cudaMemcpyHostToDevice, c->stream));
   WV_CUDA(c, cudaStreamSynchronize(c->stream));  // sv is consumed before it goes out of scope
-  WV_CUDA(c, seeds_rand_launch(d_sv, nq, nullptr, d_L, L, Lmax, c->n, d_out, stride, c->d_status(), c->stream));
+  WV_CUDA(c, seeds_rand_launch(d_sv, nq, nullptr, d_L, L, Lmax, c->n, d_out, stride, c->d_status(), c->sms, c->stream));
   return WV_OK;
 }
 

@@ -18,7 +18,7 @@ size_t seeds_rand_smem(uint32_t Lmax);
 // DEV_OVERFLOW in *d_status and skips the query)
 cudaError_t seeds_rand_launch(const uint32_t *d_sv, uint32_t nq, const uint32_t *d_nq, const uint32_t *d_L,
                               uint32_t L, uint32_t Lmax, uint32_t N, uint32_t *d_out, uint32_t stride, int *d_status,
-                              cudaStream_t s);
+                              int sms, cudaStream_t s);
 // draws the nq rand() values from the context's stream (query order), copies
 // them to the device and launches the seed kernel on the context's stream
 int draw_seeds_rand_device(wv_ctx *c, uint32_t nq, const uint32_t *d_L, uint32_t L, uint32_t Lmax, uint32_t *d_out,
