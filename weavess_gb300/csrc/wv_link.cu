@@ -9,9 +9,9 @@
 // (component_candidate.cpp:10-109), ComponentPruneVAMANA / ComponentPruneNSG /
 // ComponentPruneSSG (component_prune.cpp:20-122, 245-300) and
 // ComponentRefineEntryCentroid (component_entry.cpp:9-92).
-// ComponentConnNSGDFS walks on the host (the depth-first walk fixes which
-// nodes get linked), with its greedy searches batched on the GPU and taken
-// in repair order; ComponentConnSSGDFS (component_conn.cpp:
+// ComponentConnNSGDFS finds what the entry reaches on the GPU, walks the other
+// nodes on the host (the depth-first walk fixes which nodes get linked) and
+// batches its greedy searches on the GPU, taken in repair order; ComponentConnSSGDFS (component_conn.cpp:
 // 169-225) walks on the GPU (frontier kernels) with the repairs on the device.
 //
 // Plain form, bit-exact with the single-threaded reference:

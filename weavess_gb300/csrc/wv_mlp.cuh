@@ -25,7 +25,7 @@ struct GemmArgs {
 
 // mma.sync (m16n8k16) form
 cudaError_t gemm_bf16(const GemmArgs &g, cudaStream_t s);
-// tcgen05 form (wv_umma.cu): 128 x 128 tiles, accumulator in tensor memory;
+// tcgen05 form (wv_umma.cu): 128 x 64 tiles, accumulator in tensor memory;
 // a bounded wait that gives up sets DEV_TIMEOUT in *status
 cudaError_t gemm_bf16_umma(const GemmArgs &g, int *status, cudaStream_t s);
 
