@@ -1154,8 +1154,8 @@ __device__ __forceinline__ uint32_t ii_acquire(const uint32_t *p) {
 // the other waits look at).  Bound by the longest chains (a hub's re-prunes,
 // one after the other).  A launch per dependency level, with a barrier after
 // each level's slowest node, took 62 ms on the 200k x 128 NSG link and 79 ms
-// on two 20k x 96 Vamana passes; this takes 10.2 ms and 12.5 ms (the backward
-// launches 8.3 -> 4.6 and 7.5 -> 5.0 ms).
+// on two 20k x 96 Vamana passes; this takes 10.4 ms and 12.7 ms (the backward
+// launches 8.3 -> 4.7 and 7.5 -> 4.9 ms).
 template <int MODE, bool I8>
 __global__ void __launch_bounds__(II_WARPS * 32) k_ii_forward(IIArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1969,8 +1969,8 @@ int conn_dfs_gpu(wv_ctx *c, uint32_t L_refine, uint32_t *added) {
   // copy kernel).  What ep reaches does not depend on the walk's order, so it
   // is found there, level by level; the host walks the other nodes, few as a
   // rule, on a copy of their rows, and keeps ep's row with its new edges, for
-  // the seeds.  The 200k x 128 NSG link takes 142 ms so, 157 ms with all rows
-  // copied to the host, checked and walked there.
+  // the seeds.  With all rows copied to the host, checked and walked there the
+  // 200k x 128 NSG link (104 ms) took 15 ms more.
   const uint32_t n = c->n, ep = c->fg_ep, w0 = c->fg_w;
   uint32_t w = w0;
   constexpr uint32_t NONE = 0xffffffffu;

@@ -486,9 +486,9 @@ __global__ void k_bucket_apply(Nnd s, const uint32_t *boff, const uint32_t *bcnt
 // (not at every fragment, a third of the tile's instructions) and read by
 // ldmatrix; the offers are counted and written by a lane per target, without
 // a vote per 32 pairs.  The 100k x 128 build (S 10, L 40, R 100) takes
-// 31.2 ms; 33.2 ms with fragments widened on the fly and votes; its seven
-// joins had been 28.6 ms of 82 with the FP32 rows, the tcgen05 Gram tile and
-// the two atomics.  Six joins of 60k x 96 real-valued (FP32): 18.6 ms with
+// 29.2 ms, its seven joins 9.9 ms of them; fragments widened on the fly and
+// votes cost 2 ms more, and the joins had been 28.6 ms of 82 with the FP32
+// rows, the tcgen05 Gram tile and the two atomics.  Six joins of 60k x 96 real-valued (FP32): 18.6 ms with
 // those atomics, 14.5 ms without, 13.4 ms with pairs taken two by two, 12.3 ms
 // with 32 new rows per tile (the other rows staged half as often).
 struct JoinOut {

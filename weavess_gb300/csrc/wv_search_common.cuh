@@ -265,8 +265,8 @@ struct Visited {
 // dimensions are exchanged over the eight lanes (a transpose), so that lane
 // (oct, sub) adds row 4 sub + oct's in order.  A lane reading a row of its
 // own touches 32 lines per load, and the L1's line rate bound the searches:
-// the Vamana pipeline on 20k x 96 unit vectors 71.8 -> 65.4 ms (its candidate
-// searches 32.6 -> 26.0 ms).  Up to 16 rows take two steps of 32 dimensions at
+// the candidate searches of the Vamana pipeline on 20k x 96 unit vectors
+// 32.6 -> 25.0 ms.  Up to 16 rows take two steps of 32 dimensions at
 // once instead of 32 rows one, the same loads in flight.
 template <int R, int C>
 __device__ __forceinline__ float rows_f32(const float4 *__restrict__ base, uint32_t d4, uint32_t my, int cnt,
@@ -443,8 +443,8 @@ __device__ __forceinline__ float batch_dist(const float *__restrict__ base, uint
 // over its G lanes by a transpose (G - 1 shuffles in all).  d = 128: 32 rows
 // in one round of 8 loads per lane and 8 shuffles, a quarter of the FP32
 // rows' bytes and one latency instead of four: 10,000 queries at L = 200 over
-// 300k x 128 6.50 -> 5.06 ms, 1,000 at L = 100 over 100k 0.79 -> 0.70 ms, the
-// candidate searches of a 200k NSG link 46 -> 35 ms.  The throughput form
+// 300k x 128 6.45 -> 4.96 ms, 1,000 at L = 100 over 100k 0.77 -> 0.66 ms, the
+// candidate searches of a 200k NSG link 46 -> 33.5 ms.  The throughput form
 // (wv_beam.cuh) keeps its tensor-core rows: its 10,000 learned queries took
 // 2.03 ms with those and 2.38 ms with these.
 template <int G>
